@@ -174,7 +174,7 @@ __device__ __forceinline__ bool bpair(BPair &P, int nz, int nzh, int nxh, const 
 }
 
 // The forward column stage as four kernels, in this order (each reads only what the previous
-// ones have finished): scalar; omega_y; v (with the mean modes); u, w and the y-physical
+// ones have finished): scalar; omega_y (with the mean modes); v; u, w and the y-physical
 // outputs of the velocity.  Splitting keeps each kernel's registers and code small; the price
 // is one extra read of v and omega_y.
 
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::fwd) k_bcol_scl(ColF
     bdct_store<K, C>(d1, fa, fb, tw, (C *)A.yp + 7 * fstride + yoff);
 }
 
-// normal vorticity (main_dns.f90:411-422, 479-484, 500-502, 520-526): phirhs, Robin solve, zero
-// on the mean column, norm, store; y-physical omega_y
+// normal vorticity (main_dns.f90:411-422, 479-502, 520-526): phirhs, Robin solve, norm, store;
+// y-physical omega_y; uzero for the mean modes in place of the (0,0) pair
 template <int K, typename C>
 __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::omy) k_bcol_omy(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                             const C *__restrict__ tw) {
@@ -227,21 +227,55 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::omy) k_bcol_omy(ColF
     const double g1 = A.re / (A.dt * A.th);
     const double2 zero = make_double2(0.0, 0.0);
     BCol<K> om;
-    bload_s<K>(om, A.omy + P.off, wsm);
-    bphirhs_g<K>(om, A.gn + P.off, A.gnm1 + P.off, wsm, A.re, 1.0, A.dt, A.th, P.w2, A.dyde, FULL);
-    const TauTab to = tab_at(T, TB_OMY, P.tcol, NYP);
-    bsolve_robin<K>(om, to, zero, zero, P.w2 + g1, A.c0, rj, FULL);
-    if (P.mean) {
+    if (P.kx == 0 && P.q == 0) {
+        // The (0,0) and Nyquist columns of omega_y are zero after the step, so this pair skips their solve and
+        // its two half-warps take the mean modes side by side (uzero; half 0: u0, half 1: w0).  One after
+        // the other behind v's solves in k_bcol_v they were the longest chain of a small grid's step: that
+        // kernel took 27 us at 32 x 33 x 32, the column stage 44 (now 10 and 37) and 68 at 64 x 65 x 64 (58).
+        const double th = A.th;
+        const int lane = threadIdx.x & 31, h = lane >> 4, t = lane & 15;
+        double *U = h == 0 ? A.u0 : A.w0;
+        const double *H = h == 0 ? A.h1n : A.h3n, *HL = h == 0 ? A.h1nm1 : A.h3nm1;
+        BCol<K> uc, dd1, dd2;
+#pragma unroll
+        for (int m = 0; m <= K; ++m) uc.v[m] = make_double2(U[bidx<K>(m)], 0.0);
+        // wrk1 = -re u0/(dt th) - re (3 h1 - h1l)/(2 th); u0 <- wrk1 - (1-th) u0''/th (solvers.f90:1127-1143)
+        bcderiv<K>(dd1, uc, A.dyde, FULL);
+        bcderiv<K>(dd2, dd1, A.dyde, FULL);
+#pragma unroll
+        for (int m = 0; m <= K; ++m) {
+            const int i = bidx<K>(m);
+            const double w1 = -A.re * uc.v[m].x / (A.dt * th) - A.re * (3.0 * H[i] - HL[i]) / (2.0 * th);
+            const double r = (th > 0.99) ? w1 : w1 - (1.0 - th) * dd2.v[m].x / th;
+            uc.v[m] = make_double2(r, 0.0);
+        }
+        const TauTab tm0 = tab_at(T, TB_U0, 0, NYP), tm1 = tab_at(T, TB_W0, 0, NYP);
+        const double gt = h == 0 ? A.gtu : A.gtw, gb = h == 0 ? A.gbu : A.gbw;
+        bsolve_robin<K>(uc, h == 0 ? tm0 : tm1, make_double2(gt, 0.0), make_double2(gb, 0.0), g1, A.c0, rj, FULL);
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < K; ++m) U[t * K + m] = uc.v[m].x;
+        if (t == 15) U[NY] = uc.v[K].x;
+        __syncwarp();
+        for (int i = lane; i < NYP; i += 32) {
+            A.h1nm1[i] = A.h1n[i];
+            A.h3nm1[i] = A.h3n[i];
+        }
 #pragma unroll
         for (int m = 0; m <= K; ++m) om.v[m] = zero;
+    } else {
+        bload_s<K>(om, A.omy + P.off, wsm);
+        bphirhs_g<K>(om, A.gn + P.off, A.gnm1 + P.off, wsm, A.re, 1.0, A.dt, A.th, P.w2, A.dyde, FULL);
+        const TauTab to = tab_at(T, TB_OMY, P.tcol, NYP);
+        bsolve_robin<K>(om, to, zero, zero, P.w2 + g1, A.c0, rj, FULL);
+        bnorm<K>(om, P.kx, P.j, A.nzh);
     }
-    bnorm<K>(om, P.kx, P.j, A.nzh);
     bstore_s<K>(A.omy + P.off, om, wsm);
     bdct_store<K, C>(om, fa, fb, tw, (C *)A.yp + 3 * fstride + yoff);
 }
 
 // wall-normal velocity (main_dns.f90:363-407, 426-466, 489-502, 520): phi, phirhs, Helmholtz and
-// Poisson solves, influence-matrix correction, uzero for the mean modes, norm, store; y-physical v
+// Poisson solves, influence-matrix correction, norm, store; y-physical v
 template <int K, typename C>
 __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::v) k_bcol_v(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                           const C *__restrict__ tw) {
@@ -309,44 +343,6 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::v) k_bcol_v(ColFwdAr
         for (int m = 0; m <= K; ++m) {
             const double2 b = cmul(c2, gfa.v[m]);
             v.v[m] = make_double2(v.v[m].x + b.x, v.v[m].y + b.y);
-        }
-    }
-    // mean modes: uzero for u0 and w0 on the (0,0) column's half-warp
-    if (P.kx == 0 && P.q == 0) {
-        if (h == 0) {
-            constexpr unsigned HM = 0x0000ffffu;
-            const double th = A.th;
-            const int t = lane & 15;
-            for (int which = 0; which < 2; ++which) {
-                double *U = which == 0 ? A.u0 : A.w0;
-                const double *H = which == 0 ? A.h1n : A.h3n, *HL = which == 0 ? A.h1nm1 : A.h3nm1;
-                BCol<K> uc, dd1, dd2;
-#pragma unroll
-                for (int m = 0; m <= K; ++m) uc.v[m] = make_double2(U[bidx<K>(m)], 0.0);
-                // wrk1 = -re u0/(dt th) - re (3 h1 - h1l)/(2 th); u0 <- wrk1 - (1-th) u0''/th (solvers.f90:1127-1143)
-                bcderiv<K>(dd1, uc, A.dyde, HM);
-                bcderiv<K>(dd2, dd1, A.dyde, HM);
-#pragma unroll
-                for (int m = 0; m <= K; ++m) {
-                    const int i = bidx<K>(m);
-                    const double w1 = -A.re * uc.v[m].x / (A.dt * th) - A.re * (3.0 * H[i] - HL[i]) / (2.0 * th);
-                    const double r = (th > 0.99) ? w1 : w1 - (1.0 - th) * dd2.v[m].x / th;
-                    uc.v[m] = make_double2(r, 0.0);
-                }
-                const TauTab tm = tab_at(T, which == 0 ? TB_U0 : TB_W0, 0, NYP);
-                const double gt = which == 0 ? A.gtu : A.gtw, gb = which == 0 ? A.gbu : A.gbw;
-                bsolve_robin<K>(uc, tm, make_double2(gt, 0.0), make_double2(gb, 0.0), g1, A.c0, rj, HM);
-                __syncwarp(HM);
-#pragma unroll
-                for (int m = 0; m < K; ++m) U[t * K + m] = uc.v[m].x;
-                if (t == 15) U[NY] = uc.v[K].x;
-                __syncwarp(HM);
-            }
-        }
-        __syncwarp();
-        for (int i = lane; i < NYP; i += 32) {
-            A.h1nm1[i] = A.h1n[i];
-            A.h3nm1[i] = A.h3n[i];
         }
     }
     bnorm<K>(v, P.kx, P.j, A.nzh);
@@ -609,11 +605,11 @@ int kmm_colblk_fwd(kmm_ctx *ctx, const ColFwdArgs &A, const FusedTabs &T, const 
         RET(kmm_smem_attr(ctx, (const void *)k_bcol_omy<KK, CC>, smem));                              \
         k_bcol_omy<KK, CC><<<nblk, CB_WARPS * 32, smem, s_omy>>>(A, T, rj, twc);                       \
         CKL();                                                                                        \
+        RET(kmm_flowrate_apply(ctx, s_omy));   /* u0 comes from this kernel's mean pair */              \
         CK(cudaEventRecord(ctx->cjoin_ev[1], s_omy));                                                 \
         RET(kmm_smem_attr(ctx, (const void *)k_bcol_v<KK, CC>, smem));                                \
         k_bcol_v<KK, CC><<<nblk, CB_WARPS * 32, smem, ctx->stream>>>(A, T, rj, twc);                   \
         CKL();                                                                                        \
-        RET(kmm_flowrate_apply(ctx, ctx->stream));                                                    \
         if (A.scalar) CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[0], 0));                      \
         CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[1], 0));                                    \
         RET(kmm_smem_attr(ctx, (const void *)k_bcol_uw<KK, CC>, smem));                               \

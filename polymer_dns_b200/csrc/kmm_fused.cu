@@ -443,112 +443,109 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         const TauTab ts = tab_at(T, TB_SCL, col, nyp);
         col_solve_robin<E>(s, ts, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + T.g[TB_SCL], nyp, A.c0);
     }
-    // ---- wall-normal velocity: phi, phirhs, Helmholtz + Poisson (main_dns.f90:363-407)
-    Col<E> v, d1, d2;
-    col_load<E>(v, A.v + off, nyp);
-    col_cderiv<E>(d1, v, nyp, A.dyde);
-    col_cderiv<E>(d2, d1, nyp, A.dyde);
-#pragma unroll
-    for (int e = 0; e < E; ++e) v.v[e] = make_double2(d2.v[e].x - w2 * v.v[e].x, d2.v[e].y - w2 * v.v[e].y);
-    {
-        Col<E> f1, f0;
-        col_load<E>(f1, A.fn + off, nyp);
-        col_load<E>(f0, A.fnm1 + off, nyp);
-        col_phirhs<E>(v, f1, f0, A.re, 1.0, A.dt, A.th, w2, nyp, A.dyde);
-    }
-    {
-        const TauTab tp = tab_at(T, TB_PHI, col, nyp);
-        col_solve_dirichlet<E>(v, tp, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0);
-        const TauTab tv = tab_at(T, TB_V, col, nyp);
-        col_solve_dirichlet<E>(v, tv, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2, nyp, A.c0);
-    }
-    // ---- normal vorticity phirhs (main_dns.f90:411-422)
-    Col<E> om;
-    col_load<E>(om, A.omy + off, nyp);
-    {
-        Col<E> g1c, g0c;
-        col_load<E>(g1c, A.gn + off, nyp);
-        col_load<E>(g0c, A.gnm1 + off, nyp);
-        col_phirhs<E>(om, g1c, g0c, A.re, 1.0, A.dt, A.th, w2, nyp, A.dyde);
-    }
-    // ---- influence matrix (main_dns.f90:426-466)
-    {
-        double2 wb, wt, tmp;
-        if (A.nb == 1 && A.nt == 1) {
-            col_wall1<E>(v, nyp, A.dyde, wb, wt);
-        } else {
-            Col<E> dv;
-            col_cderiv<E>(dv, v, nyp, A.dyde);
-            double2 b2, t2;
-            col_wall1<E>(dv, nyp, A.dyde, b2, t2);
-            col_wall1<E>(v, nyp, A.dyde, wb, wt);
-            if (A.nb == 2) wb = b2;
-            if (A.nt == 2) wt = t2;
-            (void)tmp;
-        }
-        const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[col]), cmul(wt, A.dnv2b[col])), A.denom[col]);
-        const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[col]), cmul(wb, A.dnv1t[col])), A.denom[col]);
-        Col<E> gfa;
-        col_load<E>(gfa, A.gf1 + off, nyp);
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const double2 a = cmul(c1, gfa.v[e]);
-            v.v[e] = make_double2(v.v[e].x + a.x, v.v[e].y + a.y);
-        }
-        col_load<E>(gfa, A.gf2 + off, nyp);
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const double2 b = cmul(c2, gfa.v[e]);
-            v.v[e] = make_double2(v.v[e].x + b.x, v.v[e].y + b.y);
-        }
-    }
-    // ---- normal vorticity Robin solve (main_dns.f90:479-484)
-    {
-        const TauTab to = tab_at(T, TB_OMY, col, nyp);
-        col_solve_robin<E>(om, to, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0);
-    }
-    // ---- mean modes (main_dns.f90:489-502): uzero for u0 and w0 with the warp Robin solver
-    if (mean) {
+    Col<E> v, d1, d2, om;
+    if (kx == 0 && q == 0) {
+        // ---- mean modes (main_dns.f90:489-502): uzero for u0 (warp 0) and w0 (warp 1).  v and omega_y
+        // are zero on the block's two columns, (0,0) and the Nyquist kz, so it skips their solves
         const double th = A.th;
-        for (int which = 0; which < 2; ++which) {
-            double *U = which == 0 ? A.u0 : A.w0;
-            const double *H = which == 0 ? A.h1n : A.h3n, *HL = which == 0 ? A.h1nm1 : A.h3nm1;
-            Col<E> uc, dd1, dd2;
+        double *U = warp == 0 ? A.u0 : A.w0;
+        const double *H = warp == 0 ? A.h1n : A.h3n, *HL = warp == 0 ? A.h1nm1 : A.h3nm1;
+        Col<E> uc, dd1, dd2;
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int i = lane + 32 * e;
-                uc.v[e] = make_double2(i < nyp ? U[i] : 0.0, 0.0);
+        for (int e = 0; e < E; ++e) {
+            const int i = lane + 32 * e;
+            uc.v[e] = make_double2(i < nyp ? U[i] : 0.0, 0.0);
+        }
+        // wrk1 = -re u0/(dt th) - re (3 h1 - h1l)/(2 th); u0 <- wrk1 - (1-th) u0''/th (solvers.f90:1127-1143)
+        col_cderiv<E>(dd1, uc, nyp, A.dyde);
+        col_cderiv<E>(dd2, dd1, nyp, A.dyde);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int i = lane + 32 * e;
+            double r = 0.0;
+            if (i < nyp) {
+                const double w1 = -A.re * uc.v[e].x / (A.dt * th) - A.re * (3.0 * H[i] - HL[i]) / (2.0 * th);
+                r = (th > 0.99) ? w1 : w1 - (1.0 - th) * dd2.v[e].x / th;
             }
-            // wrk1 = -re u0/(dt th) - re (3 h1 - h1l)/(2 th); u0 <- wrk1 - (1-th) u0''/th (solvers.f90:1127-1143)
-            col_cderiv<E>(dd1, uc, nyp, A.dyde);
-            col_cderiv<E>(dd2, dd1, nyp, A.dyde);
+            uc.v[e] = make_double2(r, 0.0);
+        }
+        const TauTab tm = tab_at(T, warp == 0 ? TB_U0 : TB_W0, 0, nyp);
+        const double gt = warp == 0 ? A.gtu : A.gtw, gb = warp == 0 ? A.gbu : A.gbw;
+        col_solve_robin<E>(uc, tm, make_double2(gt, 0.0), make_double2(gb, 0.0), g1, nyp, A.c0);
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int i = lane + 32 * e;
-                double r = 0.0;
-                if (i < nyp) {
-                    const double w1 = -A.re * uc.v[e].x / (A.dt * th) - A.re * (3.0 * H[i] - HL[i]) / (2.0 * th);
-                    r = (th > 0.99) ? w1 : w1 - (1.0 - th) * dd2.v[e].x / th;
-                }
-                uc.v[e] = make_double2(r, 0.0);
-            }
-            const TauTab tm = tab_at(T, which == 0 ? TB_U0 : TB_W0, 0, nyp);
-            const double gt = which == 0 ? A.gtu : A.gtw, gb = which == 0 ? A.gbu : A.gbw;
-            col_solve_robin<E>(uc, tm, make_double2(gt, 0.0), make_double2(gb, 0.0), g1, nyp, A.c0);
-            __syncwarp();
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int i = lane + 32 * e;
-                if (i < nyp) U[i] = uc.v[e].x;
+        for (int e = 0; e < E; ++e) {
+            const int i = lane + 32 * e;
+            if (i < nyp) {
+                U[i] = uc.v[e].x;
+                (warp == 0 ? A.h1nm1 : A.h3nm1)[i] = H[i];
             }
         }
-        __syncwarp();
-        for (int i = lane; i < nyp; i += 32) {
-            A.h1nm1[i] = A.h1n[i];
-            A.h3nm1[i] = A.h3n[i];
-        }
 #pragma unroll
-        for (int e = 0; e < E; ++e) om.v[e] = make_double2(0.0, 0.0);
+        for (int e = 0; e < E; ++e) v.v[e] = om.v[e] = make_double2(0.0, 0.0);
+        __syncthreads();   // warp 0 reads w0 below
+    } else {
+        // ---- wall-normal velocity: phi, phirhs, Helmholtz + Poisson (main_dns.f90:363-407)
+        col_load<E>(v, A.v + off, nyp);
+        col_cderiv<E>(d1, v, nyp, A.dyde);
+        col_cderiv<E>(d2, d1, nyp, A.dyde);
+#pragma unroll
+        for (int e = 0; e < E; ++e) v.v[e] = make_double2(d2.v[e].x - w2 * v.v[e].x, d2.v[e].y - w2 * v.v[e].y);
+        {
+            Col<E> f1, f0;
+            col_load<E>(f1, A.fn + off, nyp);
+            col_load<E>(f0, A.fnm1 + off, nyp);
+            col_phirhs<E>(v, f1, f0, A.re, 1.0, A.dt, A.th, w2, nyp, A.dyde);
+        }
+        {
+            const TauTab tp = tab_at(T, TB_PHI, col, nyp);
+            col_solve_dirichlet<E>(v, tp, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0);
+            const TauTab tv = tab_at(T, TB_V, col, nyp);
+            col_solve_dirichlet<E>(v, tv, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2, nyp, A.c0);
+        }
+        // ---- normal vorticity phirhs (main_dns.f90:411-422)
+        col_load<E>(om, A.omy + off, nyp);
+        {
+            Col<E> g1c, g0c;
+            col_load<E>(g1c, A.gn + off, nyp);
+            col_load<E>(g0c, A.gnm1 + off, nyp);
+            col_phirhs<E>(om, g1c, g0c, A.re, 1.0, A.dt, A.th, w2, nyp, A.dyde);
+        }
+        // ---- influence matrix (main_dns.f90:426-466)
+        {
+            double2 wb, wt, tmp;
+            if (A.nb == 1 && A.nt == 1) {
+                col_wall1<E>(v, nyp, A.dyde, wb, wt);
+            } else {
+                Col<E> dv;
+                col_cderiv<E>(dv, v, nyp, A.dyde);
+                double2 b2, t2;
+                col_wall1<E>(dv, nyp, A.dyde, b2, t2);
+                col_wall1<E>(v, nyp, A.dyde, wb, wt);
+                if (A.nb == 2) wb = b2;
+                if (A.nt == 2) wt = t2;
+                (void)tmp;
+            }
+            const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[col]), cmul(wt, A.dnv2b[col])), A.denom[col]);
+            const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[col]), cmul(wb, A.dnv1t[col])), A.denom[col]);
+            Col<E> gfa;
+            col_load<E>(gfa, A.gf1 + off, nyp);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const double2 a = cmul(c1, gfa.v[e]);
+                v.v[e] = make_double2(v.v[e].x + a.x, v.v[e].y + a.y);
+            }
+            col_load<E>(gfa, A.gf2 + off, nyp);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const double2 b = cmul(c2, gfa.v[e]);
+                v.v[e] = make_double2(v.v[e].x + b.x, v.v[e].y + b.y);
+            }
+        }
+        // ---- normal vorticity Robin solve (main_dns.f90:479-484)
+        {
+            const TauTab to = tab_at(T, TB_OMY, col, nyp);
+            col_solve_robin<E>(om, to, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0);
+        }
     }
     // ---- norm(v), norm(omy); veloc (main_dns.f90:520-526, solvers.f90:1576-1659)
     col_norm<E>(v, xbuf, kx, j, A.nzh);
