@@ -881,7 +881,7 @@ __global__ void k_frate_g(double *G, const double *ua, const double *ub, int nyp
 }
 
 __global__ void k_flowrate(double *__restrict__ u0, const double *__restrict__ W, const double *__restrict__ G, int nyp,
-                           double target, double *__restrict__ delta) {
+                           double target, double *__restrict__ delta, volatile double *pin) {
     const int lane = threadIdx.x & 31;
     double q = 0.0, wg = 0.0;
     for (int i = lane; i < nyp; i += 32) {
@@ -895,7 +895,10 @@ __global__ void k_flowrate(double *__restrict__ u0, const double *__restrict__ W
     }
     const double d = (target - q) / wg;
     for (int i = lane; i < nyp; i += 32) u0[i] += d * G[i];
-    if (lane == 0) *delta = d;
+    if (lane == 0) {
+        *delta = d;
+        *pin = d;   // the page-locked slot kmm_get_stats reads
+    }
 }
 
 int kmm_flowrate_setup(kmm_ctx *ctx) {
@@ -945,9 +948,8 @@ int kmm_flowrate_apply(kmm_ctx *ctx, cudaStream_t st) {
     }
     const int nyp = ctx->nyp;
     double *W = ctx->d_frate, *G = W + nyp, *delta = W + 2 * nyp;
-    k_flowrate<<<1, 32, 0, st>>>(REAL(ctx, KMM_U0), W, G, nyp, ctx->p.flow_rate, delta);
+    k_flowrate<<<1, 32, 0, st>>>(REAL(ctx, KMM_U0), W, G, nyp, ctx->p.flow_rate, delta, kmm_h_pin_delta(ctx));
     CKL();
-    CK(cudaMemcpyAsync(kmm_h_pin_delta(ctx), delta, sizeof(double), cudaMemcpyDeviceToHost, st));
     return KMM_OK;
 }
 

@@ -302,6 +302,8 @@ extern "C" int kmm_ctx_create(const kmm_params *p, int device, kmm_ctx **out) {
     CK(cudaMalloc(&c->d_scratch, sizeof(double) * 9 * KMM_MAX_NYP));
     CK(cudaMallocHost(&c->h_pin, sizeof(double) * KMM_H_PIN_DOUBLES));
     memset(c->h_pin, 0, sizeof(double) * KMM_H_PIN_DOUBLES);
+    CK(cudaMallocHost(&c->rep, sizeof(KmmReport)));
+    memset((void *)c->rep, 0, sizeof(KmmReport));
     CK(cudaMemset(c->d_status, 0, sizeof(int)));
     for (int w = 0; w < 6; ++w) {
         CK(cudaMalloc(&c->wrk[w], sizeof(double2) * c->nspec));
@@ -340,6 +342,7 @@ extern "C" int kmm_ctx_destroy(kmm_ctx *ctx) {
     kmm_ztma_release(ctx);
     kmm_tau_release(ctx);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
+    if (ctx->rep) cudaFreeHost((void *)ctx->rep);
     if (ctx->po) cudaFree(ctx->po);
     if (ctx->drag) cudaFree(ctx->drag);
     if (ctx->d_frate) cudaFree(ctx->d_frate);

@@ -19,6 +19,8 @@
 // recurrences (eqsolve, pntsolve).
 #include <math.h>
 
+#include <atomic>
+
 #include "kmm_fft.cuh"
 #include "kmm_fused.cuh"
 
@@ -221,6 +223,8 @@ static int build_tables(kmm_ctx *ctx) {
     CK(cudaMalloc(&F->q, sizeof(double2) * nq * 10));
     CK(cudaMalloc(&F->r, sizeof(double2) * nq * 4));
     CK(cudaMalloc(&F->yo, sizeof(double2) * ncp * 4));
+    CK(cudaMalloc(&F->acc, sizeof(double) * (2 * (size_t)ctx->nyp + 1)));
+    CK(cudaMemsetAsync(F->acc, 0, sizeof(double) * (2 * (size_t)ctx->nyp + 1), ctx->stream));
     return KMM_OK;
 }
 
@@ -310,7 +314,7 @@ void kmm_fused_release(kmm_ctx *ctx) {
         cudaFree(F->tabs.tf[c]);
         cudaFree(F->btabs.td[c]); cudaFree(F->btabs.te[c]); cudaFree(F->btabs.tb1[c]); cudaFree(F->btabs.tb2[c]);
     }
-    cudaFree(F->yp); cudaFree(F->q); cudaFree(F->r); cudaFree(F->yo); cudaFree(F->rj); cudaFree(F->brj);
+    cudaFree(F->yp); cudaFree(F->q); cudaFree(F->r); cudaFree(F->yo); cudaFree(F->acc); cudaFree(F->rj); cudaFree(F->brj);
     cudaFree(F->twf_y2); cudaFree(F->twf_mz); cudaFree(F->twf_mx);
     free(F);
     ctx->fused = NULL;
@@ -974,6 +978,54 @@ bool kmm_fused_applicable(const kmm_ctx *ctx) {
 
 int kmm_tracers_enqueue(kmm_ctx *ctx, cudaStream_t st);
 
+// The step's CFL maximum, |u| maximum and status to the host's report, the accumulators zeroed for the
+// next step.  One small kernel behind the x stage and the tracers, beside the z forward and back stages:
+// it takes the place of three memsets and three copies (each a node of the step's graph), and a host
+// loop over steps can launch the next step while the present one's last kernels run.
+__global__ void __launch_bounds__(128) k_report(double *acc, int nyp, KmmReport *out) {
+    __shared__ double sc[4], su[4];
+    __shared__ int sn[4];
+    const int warp = threadIdx.x >> 5;
+    double c = 0.0, u = 0.0;
+    int nan = 0;
+    for (int i = threadIdx.x; i < nyp; i += 128) {
+        const double ci = acc[i], ui = acc[nyp + i];
+        if (ci != ci) nan = 1;
+        else c = fmax(c, ci);
+        if (ui > u) u = ui;
+        acc[i] = 0.0;
+        acc[nyp + i] = 0.0;
+    }
+    for (int off = 16; off; off >>= 1) {
+        c = fmax(c, __shfl_xor_sync(0xffffffffu, c, off));
+        u = fmax(u, __shfl_xor_sync(0xffffffffu, u, off));
+    }
+    nan = __any_sync(0xffffffffu, nan);
+    if ((threadIdx.x & 31) == 0) {
+        sc[warp] = c;
+        su[warp] = u;
+        sn[warp] = nan;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 4; ++w) {
+            c = fmax(c, sc[w]);
+            u = fmax(u, su[w]);
+            nan |= sn[w];
+        }
+        int *status = reinterpret_cast<int *>(acc + 2 * nyp);
+        volatile KmmReport *o = out;
+        o->cfl = nan ? __longlong_as_double(0x7ff8000000000000ll) : c;
+        o->umax = u;
+        o->status = *status;
+        *status = 0;
+        __threadfence_system();
+        o->flag = 1;
+    }
+}
+
+void kmm_report_arm(kmm_ctx *ctx) { ctx->rep->flag = 0; }
+
 int kmm_fused_step(kmm_ctx *ctx) {
     RET(kmm_fused_enqueue(ctx));
     return kmm_fused_finish(ctx);
@@ -1064,9 +1116,13 @@ void kmm_fused_replayed(kmm_ctx *ctx, int parity) {
 int kmm_fused_enqueue(kmm_ctx *ctx) {
     // graphs only after the step that initialises the tracers (it == irstrt) and the tau tables
     const bool graphable = ctx->use_graph && !ctx->timing_on && ctx->fused != NULL && ctx->it >= ctx->p.irstrt;
-    if (!graphable) return kmm_fused_launch(ctx);
+    if (!graphable) {
+        kmm_report_arm(ctx);
+        return kmm_fused_launch(ctx);
+    }
     if (!ctx->graph_ready) RET(capture_graphs(ctx));
     const int parity = ctx->f[KMM_FN] == ctx->g_fn0 ? 0 : 1;
+    kmm_report_arm(ctx);
     CK(cudaGraphLaunch(ctx->gexec[parity], ctx->stream));
     ctx->launches += ctx->gkernels[parity];
     swap_history(ctx);
@@ -1074,12 +1130,29 @@ int kmm_fused_enqueue(kmm_ctx *ctx) {
     return KMM_OK;
 }
 
+static int fused_launch(kmm_ctx *ctx);
+
 int kmm_fused_launch(kmm_ctx *ctx) {
+    RET(build_tables(ctx));
+    // the step's kernels accumulate into the fused path's own words, which its report leaves zero (the
+    // routine entry points keep theirs and their memsets)
+    double *const cfl = ctx->d_cfl, *const um = ctx->d_umax;
+    int *const status = ctx->d_status;
+    ctx->d_cfl = ctx->fused->acc;
+    ctx->d_umax = ctx->d_cfl + ctx->nyp;
+    ctx->d_status = (int *)(ctx->d_umax + ctx->nyp);
+    const int st = fused_launch(ctx);
+    ctx->d_cfl = cfl;
+    ctx->d_umax = um;
+    ctx->d_status = status;
+    return st;
+}
+
+static int fused_launch(kmm_ctx *ctx) {
     const int nyp = ctx->nyp, nz = ctx->nz, nxh = ctx->nxh, mz = ctx->mz;
     const size_t ncols = (size_t)nz * nxh;
     const int scalar = ctx->p.scalar_on ? 1 : 0;
     const int nbase = scalar ? 8 : 6, nq = scalar ? 9 : 6, nout = scalar ? 4 : 3;
-    RET(build_tables(ctx));
     KmmFused *FU = ctx->fused;
     double2 *g_yp = FU->yp, *g_q = FU->q, *g_r = FU->r, *g_yo = FU->yo;
     (void)nbase;
@@ -1153,9 +1226,6 @@ int kmm_fused_launch(kmm_ctx *ctx) {
     if (scalar) { ctx->f[KMM_SCNM1] = sn_old; ctx->f[KMM_SCN] = snm1_old; }
 
     // z inverse transforms
-    CK(cudaMemsetAsync(ctx->d_cfl, 0, sizeof(double) * nyp, ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_umax, 0, sizeof(double) * nyp, ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
     const size_t smz = sizeof(double2) * ((size_t)ZT_WARPS * 2 * mz + (size_t)ZT_Y * mz * ZT_KX);
     const size_t smzf = sizeof(double2) * ((size_t)ZT_WARPS * 2 * mz + (size_t)ZT_KX * nz * ZT_Y);
     const dim3 gz((nxh + ZT_KX - 1) / ZT_KX, (nyp + ZT_Y - 1) / ZT_Y);
@@ -1207,12 +1277,14 @@ int kmm_fused_launch(kmm_ctx *ctx) {
     kmm_toc(ctx, KMM_STAGE_XPHYS);
     // tracers (solvers.f90:3463-3476) on the side stream: they read only the particles and the
     // 3/2-grid u, v, w just written, so they overlap the z-forward and back stages (kept in line
-    // while the stages are being timed)
-    const bool tracers_forked = ctx->p.npart > 0 && !ctx->timing_on;
-    if (tracers_forked) {
+    // while the stages are being timed), and with them the step's report
+    const bool forked = !ctx->timing_on;
+    if (forked) {
         CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
         CK(cudaStreamWaitEvent(ctx->side, ctx->fork_ev, 0));
         RET(kmm_tracers_enqueue(ctx, ctx->side));
+        k_report<<<1, 128, 0, ctx->side>>>(FU->acc, nyp, ctx->rep);
+        CKL();
     }
     // z forward transforms
     kmm_tic(ctx);
@@ -1284,41 +1356,70 @@ int kmm_fused_launch(kmm_ctx *ctx) {
     CKL();
     }
     kmm_toc(ctx, KMM_STAGE_POST);
-    if (tracers_forked) {
+    if (forked) {
         CK(cudaEventRecord(ctx->join_ev, ctx->side));
         CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
     } else {
         RET(kmm_tracers_enqueue(ctx, ctx->stream));
+        k_report<<<1, 128, 0, ctx->stream>>>(FU->acc, nyp, ctx->rep);
+        CKL();
     }
-    // the CFL maxima and the tracer status go to pinned host memory for kmm_fused_finish
-    // (solvers.f90:3497-3514)
-    double *h_cfl = ctx->h_pin, *h_um = ctx->h_pin + KMM_MAX_NYP;
-    CK(cudaMemcpyAsync(h_cfl, ctx->d_cfl, sizeof(double) * nyp, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(h_um, ctx->d_umax, sizeof(double) * nyp, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(kmm_h_pin_status(ctx), ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     return KMM_OK;
 }
 
-int kmm_fused_finish(kmm_ctx *ctx) {
-    const int nyp = ctx->nyp;
-    CK(cudaStreamSynchronize(ctx->stream));
-    const double *h_cfl = ctx->h_pin, *h_um = ctx->h_pin + KMM_MAX_NYP;
+// the status of an enqueued step from its report (solvers.f90:3497-3514)
+static int report_status(kmm_ctx *ctx) {
+    const KmmReport *R = ctx->rep;
     int st = KMM_OK;
-    if (ctx->p.npart > 0 && *kmm_h_pin_status(ctx)) {
+    if (R->late || R->status == KMM_ERR_TIMEOUT) {
+        ctx->rep->late = 0;
+        kmm_set_error(ctx, "a device-side wait ran out");
+        st = KMM_ERR_TIMEOUT;
+    } else if (ctx->p.npart > 0 && R->status) {
         kmm_set_error(ctx, "particle interpolation cell index out of range (part_track.f90:580-590)");
         st = KMM_ERR_INTERP;
     }
-    double cflmax = 0.0, umax = 0.0;
-    bool nan = false;
-    for (int i = 0; i < nyp; ++i) {
-        if (h_cfl[i] != h_cfl[i]) nan = true;
-        else if (h_cfl[i] > cflmax) cflmax = h_cfl[i];
-        if (h_um[i] > umax) umax = h_um[i];
-    }
-    ctx->stats.cflmax = nan ? NAN : cflmax;
-    ctx->stats.umax = umax;
+    const bool nan = R->cfl != R->cfl;
+    ctx->stats.cflmax = R->cfl;
+    ctx->stats.umax = R->umax;
     if (st == KMM_OK && nan) st = KMM_ERR_NAN;
-    if (st == KMM_OK && cflmax > 1.0) st = KMM_ERR_CFL;
+    if (st == KMM_OK && R->cfl > 1.0) st = KMM_ERR_CFL;
     ctx->stats.status = st;
+    return st;
+}
+
+int kmm_fused_finish(kmm_ctx *ctx) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    return report_status(ctx);
+}
+
+int kmm_fused_report(kmm_ctx *ctx) {
+    // the report is the last store of a kernel already enqueued; the stream is asked now and then, so
+    // that a launch or device error ends the wait
+    for (unsigned k = 1; !ctx->rep->flag; ++k) {
+        if ((k & 0xfff) == 0) {
+            const cudaError_t e = cudaStreamQuery(ctx->stream);
+            if (e != cudaErrorNotReady) {
+                CK(e);
+                CK(cudaStreamSynchronize(ctx->stream));
+                if (!ctx->rep->flag) {
+                    kmm_set_error(ctx, "the step ended without its report");
+                    return KMM_ERR_CUDA;
+                }
+            }
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return report_status(ctx);
+}
+
+int kmm_fused_drain(kmm_ctx *ctx, int st) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->rep->late) {
+        ctx->rep->late = 0;
+        kmm_set_error(ctx, "a device-side wait ran out");
+        ctx->stats.status = KMM_ERR_TIMEOUT;
+        if (st == KMM_OK) st = KMM_ERR_TIMEOUT;
+    }
     return st;
 }

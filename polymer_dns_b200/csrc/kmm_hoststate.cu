@@ -210,10 +210,11 @@ extern "C" int kmm_run_host(kmm_ctx *ctx, int n) {
     CK(cudaStreamWaitEvent(S->h2d, S->entry_ev, 0));
     RET(enqueue_uploads(ctx, S, false));
     int st = KMM_OK;
+    bool pending = false;
     for (int s = 0; s < n; ++s) {
         st = enqueue_early_downloads(ctx, S);
         if (st) break;
-        st = kmm_step(ctx);
+        st = kmm_step_reported(ctx, &pending);   // the copies follow the step on its stream
         if (st == KMM_ERR_CUDA || st == KMM_ERR_NOMEM || st == KMM_ERR_ARG) break;
         // the host arrays receive this step's result even when the step reports a stop status
         const int dst = enqueue_downloads(ctx, S);
@@ -232,5 +233,5 @@ extern "C" int kmm_run_host(kmm_ctx *ctx, int n) {
             st = KMM_ERR_CUDA;
         }
     }
-    return st;
+    return pending ? kmm_fused_drain(ctx, st) : st;
 }

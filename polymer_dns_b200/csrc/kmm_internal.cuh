@@ -40,6 +40,15 @@ struct DevPlan {
     const double2 *tw;
 };
 
+// what a fused step reports to the host (page-locked, written by k_report before the step's last
+// kernels): max CFL number (NaN if any is), max |u|, the device status word
+struct KmmReport {
+    double cfl, umax;
+    int status;
+    volatile int late;   // a status raised after the report (the z forward transform's bounded waits)
+    volatile int flag;   // set last
+};
+
 struct kmm_ctx {
     kmm_params p;
     int device;
@@ -78,6 +87,7 @@ struct kmm_ctx {
     double *d_pumax;             // inertial particles: part_track's running max relative speed (umax1)
     double *d_umax;              // scratch for |u| max (per plane)
     double *d_scratch;           // 9*KMM_MAX_NYP doubles for the (0,0)-mode solver
+    KmmReport *rep;              // the fused step's report (pinned host)
     double *h_pin;               // pinned host: cfl[KMM_MAX_NYP], umax[KMM_MAX_NYP], status (step read-backs)
     double *scsource;            // the KMM_SCSOURCE field's storage (scl_flag = 2, 4, 5)
     // targeted sources (scl_flag = 4, 5): -Q on the 3/2 grid, the candidate list and its count,
@@ -134,10 +144,17 @@ struct kmm_ctx {
 void kmm_hoststate_release(kmm_ctx *ctx);
 void kmm_fused_release(kmm_ctx *ctx);
 int kmm_fused_step(kmm_ctx *ctx);
-// the fused step in two halves: enqueue every kernel and the read-back of CFL / status, then wait
-// and evaluate (kmm_fused_step = launch + finish; the ensemble launches all members first)
+// the fused step in two halves: enqueue every kernel, then wait and evaluate the CFL number and the
+// status (kmm_fused_step = launch + finish; the ensemble launches all members first).
+// kmm_fused_report is the finish that does not wait for the step's last kernels; the caller must end
+// with kmm_fused_drain, which does and returns a status raised after the report.
 int kmm_fused_launch(kmm_ctx *ctx);
 int kmm_fused_finish(kmm_ctx *ctx);
+int kmm_fused_report(kmm_ctx *ctx);
+int kmm_fused_drain(kmm_ctx *ctx, int st);
+// kmm_step that returns after a fused step's report; *pending is set when kmm_fused_drain is due
+int kmm_step_reported(kmm_ctx *ctx, bool *pending);
+void kmm_report_arm(kmm_ctx *ctx);   // before a step is enqueued
 int kmm_fused_graph_for_step(kmm_ctx *ctx, int *parity);
 unsigned long long kmm_graph_generation();   // a process-wide counter: every capture / release gets a new value
 void kmm_ensemble_forget(kmm_ctx *ctx);      // drop the cached ensemble graphs that hold ctx

@@ -16,8 +16,8 @@
 // kinds of tile are swizzled by the length of their rows.
 //
 // Every wait on an mbarrier is bounded (KMM_OPT_WAIT_LIMIT_MS, default 2 s of %globaltimer); a wait
-// that runs out records KMM_ERR_TIMEOUT in the step's status word and the CTA finishes without the
-// data.
+// that runs out records KMM_ERR_TIMEOUT in the step's status word (the forward transform, which runs
+// beside or after the step's report, in the host's late word) and the CTA finishes without the data.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
 template <int MZ, typename C, int KX, int YT, int MINB>
 __global__ void __launch_bounds__(KX * YT * 32, MINB)
     k_zf_tma(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout,
-             const C *__restrict__ tw, int nper, double scale, int *status) {
+             const C *__restrict__ tw, int nper, double scale, volatile int *status) {
     typedef typename kct::Real<C>::T T;
     constexpr int NZ = 2 * MZ / 3, NZH = NZ / 2, W = KX * YT, TIN = MZ * W, TOUT = NZ * W;
     extern __shared__ unsigned char zsm_raw[];
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
             for (int o = 0; o < nper; ++o)
                 if (((issued >> o) & 1u) && !((ready >> o) & 1u)) mbar_wait(&bar[o], 0);
     }
-    if (!ok && lane == 0) atomicMax(status, KMM_ERR_TIMEOUT);
+    if (!ok && lane == 0) *status = KMM_ERR_TIMEOUT;
 }
 
 // ---------------------------------------------------------------------------
@@ -434,7 +434,7 @@ static int zf_launch(kmm_ctx *ctx, const C *r, C *yo, int nout, const C *tw) {
     const dim3 grid((ctx->nxh + KX - 1) / KX, (ctx->nyp + YT - 1) / YT, nout / nper);
     RET(kmm_smem_attr(ctx, (const void *)k_zf_tma<MZ, C, KX, YT, MINB>, smem));
     k_zf_tma<MZ, C, KX, YT, MINB><<<grid, W * 32, smem, ctx->stream>>>(M->fwd.in, M->fwd.out, tw, nper,
-                                                                       (double)ctx->mx * (double)ctx->mz, ctx->d_status);
+                                                                       (double)ctx->mx * (double)ctx->mz, &ctx->rep->late);
     return KMM_OK;   // the caller checks the launch and counts it
 }
 
