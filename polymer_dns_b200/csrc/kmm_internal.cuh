@@ -277,12 +277,7 @@ __host__ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
     return make_double2((a.x * b.x + a.y * b.y) / den, (a.y * b.x - a.x * b.y) / den);
 }
 
-// ---------------------------------------------------------------------------
-// shared-memory Stockham FFT over a batch of sequences.
-//   a, b: two smem buffers; sequence s occupies [s*ld, s*ld + n).
-//   sign -1: exp(-2 pi i jk/n) (FFTW_FORWARD), +1: exp(+...) (FFTW_BACKWARD).
-//   All threads of the block must call it; returns the buffer holding the result.
-// ---------------------------------------------------------------------------
+// X_q = sum_r v_r exp(sign 2 pi i r q / R) in place, R = 2, 3, 4, 5 (a compile-time constant where inlined)
 __device__ __forceinline__ void radix_dft(int R, double2 *v, int sign) {
     if (R == 2) {
         double2 a0 = v[0], a1 = v[1];
@@ -326,48 +321,6 @@ __device__ __forceinline__ void radix_dft(int R, double2 *v, int sign) {
     }
 }
 
-__device__ __forceinline__ double2 *fft_smem(const DevPlan &P, double2 *a, double2 *b, int nseq, int ld, int sign) {
-    const int n = P.n;
-    double2 *src = a, *dst = b;
-    int Ns = 1;
-    for (int f = 0; f < P.nf; ++f) {
-        const int R = P.fac[f];
-        const int nR = n / R;
-        const int tstep = n / (Ns * R);
-        const int total = nseq * nR;
-        for (int t = threadIdx.x; t < total; t += blockDim.x) {
-            const int s = t / nR, j = t - s * nR;
-            const int k = j % Ns;
-            const double2 *sp = src + (size_t)s * ld;
-            double2 *dp = dst + (size_t)s * ld;
-            double2 v[5];
-#pragma unroll
-            for (int r = 0; r < 5; ++r) {
-                if (r < R) {
-                    double2 x = sp[j + r * nR];
-                    if (r && k) {
-                        double2 w = __ldg(&P.tw[(r * k * tstep) % n]);
-                        if (sign > 0) w.y = -w.y;
-                        x = cmul(x, w);
-                    }
-                    v[r] = x;
-                }
-            }
-            radix_dft(R, v, sign);
-            const int idxD = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int q = 0; q < 5; ++q)
-                if (q < R) dp[idxD + q * Ns] = v[q];
-        }
-        __syncthreads();
-        double2 *tmp = src;
-        src = dst;
-        dst = tmp;
-        Ns *= R;
-    }
-    return src;
-}
-
 // radix-8 DFT (two radix-4 halves + the W8 twiddles), same sign convention as radix_dft
 __device__ __forceinline__ void radix8_dft(double2 *v, int sign) {
     double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
@@ -388,41 +341,95 @@ __device__ __forceinline__ void radix8_dft(double2 *v, int sign) {
     v[7] = csub(e[3], t3);
 }
 
+// q = j / d by a multiplication, exact for j < 65536: m = div_magic(d)
+__device__ __forceinline__ unsigned div_magic(int d) { return 0xffffffffu / (unsigned)d + 1u; }   // 0 for d = 1
+__device__ __forceinline__ int div_by(int j, unsigned m) { return m ? (int)__umulhi((unsigned)j, m) : j; }
+
+// one radix-R butterfly j of a Stockham stage of stride Ns over n values: reads src[j + r n/R], writes
+// dst[(j - k) R + k + q Ns], k = j mod Ns; the twiddle index r k n/(Ns R) is below n
+template <int R>
+__device__ __forceinline__ void rt_butterfly(const double2 *__restrict__ src, double2 *__restrict__ dst, int j, int nR,
+                                             int Ns, unsigned mNs, int tstep, const double2 *__restrict__ tw,
+                                             int sign) {
+    const int jq = div_by(j, mNs), k = j - jq * Ns;
+    double2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        double2 x = src[j + r * nR];
+        if (r && k) {
+            double2 w = __ldg(&tw[r * k * tstep]);
+            if (sign > 0) w.y = -w.y;
+            x = cmul(x, w);
+        }
+        v[r] = x;
+    }
+    if constexpr (R == 8) radix8_dft(v, sign);
+    else radix_dft(R, v, sign);
+    const int o = jq * Ns * R + k;
+#pragma unroll
+    for (int q = 0; q < R; ++q) dst[o + q * Ns] = v[q];
+}
+
 // ---------------------------------------------------------------------------
-// warp-private Stockham FFT: one sequence of length P.n in the warp's own shared buffers a, b;
-// only __syncwarp between stages.  Radices 8, 4, 2, 3, 5 (plan from kmm_plan_r8).
+// shared-memory Stockham FFT over a batch of sequences.
+//   a, b: two smem buffers; sequence s occupies [s*ld, s*ld + n).
+//   sign -1: exp(-2 pi i jk/n) (FFTW_FORWARD), +1: exp(+...) (FFTW_BACKWARD).
+//   All threads of the block must call it; returns the buffer holding the result.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 *fft_warp(const DevPlan &P, double2 *a, double2 *b, int sign) {
-    const int n = P.n;
-    const int lane = threadIdx.x & 31;
+// One stage at a time with the radix a compile-time constant and the divisions by the stage's strides
+// replaced by multiplications: the index arithmetic, not the butterflies, was most of these transforms'
+// instructions.
+template <int R>
+__device__ __forceinline__ void fft_smem_stage(const double2 *src, double2 *dst, const double2 *tw, int n, int Ns,
+                                               int nseq, int ld, int sign) {
+    const int nR = n / R, tstep = nR / Ns, total = nseq * nR;
+    const unsigned mR = div_magic(nR), mNs = div_magic(Ns);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        const int s = div_by(t, mR), j = t - s * nR;
+        rt_butterfly<R>(src + s * ld, dst + s * ld, j, nR, Ns, mNs, tstep, tw, sign);
+    }
+}
+
+__device__ __forceinline__ double2 *fft_smem(const DevPlan &P, double2 *a, double2 *b, int nseq, int ld, int sign) {
     double2 *src = a, *dst = b;
     int Ns = 1;
     for (int f = 0; f < P.nf; ++f) {
         const int R = P.fac[f];
-        const int nR = n / R;
-        const int tstep = n / (Ns * R);
-        for (int j = lane; j < nR; j += 32) {
-            const int k = j % Ns;
-            double2 v[8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                if (r < R) {
-                    double2 x = src[j + r * nR];
-                    if (r && k) {
-                        double2 w = __ldg(&P.tw[(r * k * tstep) % n]);
-                        if (sign > 0) w.y = -w.y;
-                        x = cmul(x, w);
-                    }
-                    v[r] = x;
-                }
-            }
-            if (R == 8) radix8_dft(v, sign);
-            else radix_dft(R, v, sign);
-            const int idxD = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (q < R) dst[idxD + q * Ns] = v[q];
-        }
+        if (R == 4) fft_smem_stage<4>(src, dst, P.tw, P.n, Ns, nseq, ld, sign);
+        else if (R == 2) fft_smem_stage<2>(src, dst, P.tw, P.n, Ns, nseq, ld, sign);
+        else if (R == 3) fft_smem_stage<3>(src, dst, P.tw, P.n, Ns, nseq, ld, sign);
+        else fft_smem_stage<5>(src, dst, P.tw, P.n, Ns, nseq, ld, sign);
+        __syncthreads();
+        double2 *tmp = src;
+        src = dst;
+        dst = tmp;
+        Ns *= R;
+    }
+    return src;
+}
+
+// ---------------------------------------------------------------------------
+// warp-private Stockham FFT: one sequence of length P.n in the warp's own shared buffers a, b;
+// only __syncwarp between stages.  Radices 8, 4, 2, 3, 5 (plan from kmm_plan_r8).
+// ---------------------------------------------------------------------------
+template <int R>
+__device__ __forceinline__ void fft_warp_stage(const double2 *src, double2 *dst, const double2 *tw, int n, int Ns,
+                                               int sign) {
+    const int nR = n / R, tstep = nR / Ns;
+    const unsigned mNs = div_magic(Ns);
+    for (int j = threadIdx.x & 31; j < nR; j += 32) rt_butterfly<R>(src, dst, j, nR, Ns, mNs, tstep, tw, sign);
+}
+
+__device__ __forceinline__ double2 *fft_warp(const DevPlan &P, double2 *a, double2 *b, int sign) {
+    double2 *src = a, *dst = b;
+    int Ns = 1;
+    for (int f = 0; f < P.nf; ++f) {
+        const int R = P.fac[f];
+        if (R == 8) fft_warp_stage<8>(src, dst, P.tw, P.n, Ns, sign);
+        else if (R == 4) fft_warp_stage<4>(src, dst, P.tw, P.n, Ns, sign);
+        else if (R == 2) fft_warp_stage<2>(src, dst, P.tw, P.n, Ns, sign);
+        else if (R == 3) fft_warp_stage<3>(src, dst, P.tw, P.n, Ns, sign);
+        else fft_warp_stage<5>(src, dst, P.tw, P.n, Ns, sign);
         __syncwarp();
         double2 *tmp = src;
         src = dst;
