@@ -575,9 +575,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::bwd) k_bcol_bwd(ColB
 // K = ny / 16 where blocked kernels are compiled: the fused column kernels for ny = 32 .. 128 (K <=
 // 8), the routine path's solver also for ny = 256
 static int colblk_k(const kmm_ctx *ctx) {
-    const int ny = ctx->ny;
-    if (ny != 32 && ny != 64 && ny != 96 && ny != 128 && ny != 256) return 0;
-    return ny / 16;
+    return kmm_blocked_ny(ctx->ny) ? ctx->ny / 16 : 0;
 }
 
 int kmm_colblk_fwd(kmm_ctx *ctx, const ColFwdArgs &A, const FusedTabs &T, const double *rj, const void *tw,
@@ -678,7 +676,8 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CB_MINB) k_bsolve(SolveList ul,
 int kmm_colblk_solve_many(kmm_ctx *ctx, double2 *const *u, int nf, double g, int robin, double at, double bt,
                           double ab, double bb, const double2 *gt, const double2 *gb) {
     const int K = colblk_k(ctx);
-    if (!K || !ctx->use_colblk) return KMM_ERR_UNSUPPORTED;
+    if (!K) return kmm_warpcol_solve_many(ctx, u, nf, g, robin, at, bt, ab, bb, gt, gb);
+    if (!ctx->use_colblk) return KMM_ERR_UNSUPPORTED;
     const double *tb[5], *rj = NULL;
     const int st = kmm_tau_tabset(ctx, g, robin, at, bt, ab, bb, tb, &rj);
     if (st != KMM_OK) return st;
@@ -789,7 +788,8 @@ __global__ void __launch_bounds__(CB_WARPS * 32, K > 8 ? 2 : CB_MINB)
 int kmm_colblk_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec) {
     const int K = colblk_k(ctx);
-    if (!K || !ctx->use_colblk) return KMM_ERR_UNSUPPORTED;
+    if (!K) return kmm_warpcol_phirhs_solve(ctx, x, fn, fnm1, nf, var, phi, nsolve, spec);
+    if (!ctx->use_colblk) return KMM_ERR_UNSUPPORTED;
     if (nf < 1 || nf > KMM_SOLVE_BATCH || nsolve < 1 || nsolve > 2) return KMM_ERR_ARG;
     PhiSolveCfg S[2];
     const double *rj = NULL;

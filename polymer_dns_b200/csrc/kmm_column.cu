@@ -31,8 +31,15 @@ __device__ __forceinline__ void tile_store(double2 *__restrict__ g, const double
 // ---------------------------------------------------------------------------
 // cderiv(f,df), derivatives.f90:258-314: two independent parity chains per column
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(TPB) k_cderiv(const double2 *__restrict__ f, double2 *__restrict__ df, int ncols,
-                                                int nyp, double dyde) {
+// up to KMM_CDERIV_BATCH independent (input, output) pairs per launch, blockIdx.y picking the pair
+struct CderivList {
+    const double2 *f[KMM_CDERIV_BATCH];
+    double2 *df[KMM_CDERIV_BATCH];
+};
+
+__global__ void __launch_bounds__(TPB) k_cderiv(CderivList list, int ncols, int nyp, double dyde) {
+    const double2 *f = list.f[blockIdx.y];
+    double2 *df = list.df[blockIdx.y];
     extern __shared__ double2 sm[];
     double2 *sf = sm, *sd = sm + (size_t)TILE * nyp;
     const int col0 = blockIdx.x * TILE;
@@ -76,12 +83,6 @@ __global__ void __launch_bounds__(TPB) k_cderiv(const double2 *__restrict__ f, d
 // 8 columns (one contiguous run in global memory) pass through shared memory with coalesced loads
 // and stores; coefficient i sits at i + i / K there, so a lane's K values start K + 1 slots after
 // its neighbour's and the 16 lanes' accesses spread over the banks.
-// up to KMM_CDERIV_BATCH independent (input, output) pairs per launch, blockIdx.y picking the pair
-struct CderivList {
-    const double2 *f[KMM_CDERIV_BATCH];
-    double2 *df[KMM_CDERIV_BATCH];
-};
-
 template <int K>
 __global__ void __launch_bounds__(128) k_cderiv_hw(CderivList list, int ncols, double dyde) {
     constexpr int NY = 16 * K, NYP = NY + 1, SK = K + 1, CS = 16 * SK + 1;
@@ -167,16 +168,18 @@ __global__ void __launch_bounds__(128) k_cderiv_hw(CderivList list, int ncols, d
 int kmm_internal_cderiv_many(kmm_ctx *ctx, const double2 *const *f, double2 *const *df, int n) {
     const int ncols = ctx->nz * ctx->nxh;
     const int ny = ctx->nyp - 1;
-    if (ctx->use_colblk && ny % 16 == 0 && ny >= 32 && (ny <= 128 || ny == 256)) {
-        const int nblk = (ncols + 7) / 8;
-        for (int p0 = 0; p0 < n; p0 += KMM_CDERIV_BATCH) {
-            const int nb = n - p0 < KMM_CDERIV_BATCH ? n - p0 : KMM_CDERIV_BATCH;
-            CderivList list;
-            for (int m = 0; m < nb; ++m) {
-                list.f[m] = f[p0 + m];
-                list.df[m] = df[p0 + m];
-            }
-            const dim3 grid(nblk, nb);
+    const bool hw = ctx->use_colblk && ny % 16 == 0 && ny >= 32 && (ny <= 128 || ny == 256);
+    const size_t sm = tile_smem(ctx->nyp, 2);
+    if (!hw) RET(kmm_smem_attr(ctx, (const void *)k_cderiv, sm));
+    for (int p0 = 0; p0 < n; p0 += KMM_CDERIV_BATCH) {
+        const int nb = n - p0 < KMM_CDERIV_BATCH ? n - p0 : KMM_CDERIV_BATCH;
+        CderivList list;
+        for (int m = 0; m < nb; ++m) {
+            list.f[m] = f[p0 + m];
+            list.df[m] = df[p0 + m];
+        }
+        if (hw) {
+            const dim3 grid((ncols + 7) / 8, nb);
             switch (ny / 16) {
             case 2: k_cderiv_hw<2><<<grid, 128, 0, ctx->stream>>>(list, ncols, ctx->dyde); break;
             case 3: k_cderiv_hw<3><<<grid, 128, 0, ctx->stream>>>(list, ncols, ctx->dyde); break;
@@ -187,14 +190,9 @@ int kmm_internal_cderiv_many(kmm_ctx *ctx, const double2 *const *f, double2 *con
             case 8: k_cderiv_hw<8><<<grid, 128, 0, ctx->stream>>>(list, ncols, ctx->dyde); break;
             case 16: k_cderiv_hw<16><<<grid, 128, 0, ctx->stream>>>(list, ncols, ctx->dyde); break;
             }
-            CKL();
+        } else {
+            k_cderiv<<<dim3((ncols + TILE - 1) / TILE, nb), TPB, sm, ctx->stream>>>(list, ncols, ctx->nyp, ctx->dyde);
         }
-        return KMM_OK;
-    }
-    const size_t sm = tile_smem(ctx->nyp, 2);
-    RET(kmm_smem_attr(ctx, (const void *)k_cderiv, sm));
-    for (int m = 0; m < n; ++m) {
-        k_cderiv<<<(ncols + TILE - 1) / TILE, TPB, sm, ctx->stream>>>(f[m], df[m], ncols, ctx->nyp, ctx->dyde);
         CKL();
     }
     return KMM_OK;

@@ -119,9 +119,10 @@ __global__ void k_tab_block(const double *__restrict__ src, double *__restrict__
     }
 }
 
-// the blocked copies of one configuration's td (as 1 / d), te, tb1, tb2 (tf is per column, unchanged)
+// copies of one configuration's td (as 1 / d), te, tb1, tb2 (tf is per column, unchanged), lane-blocked
+// for the ny of the blocked kernels, else (K = 0) in the canonical order
 static int block_tables(kmm_ctx *ctx, const double *const src[4], double *dst[4], int ncols) {
-    const int K = ctx->ny / 16;
+    const int K = kmm_blocked_ny(ctx->ny) ? ctx->ny / 16 : 0;
     const size_t n = (size_t)ncols * ctx->nyp;
     const int nb = (int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
     for (int a = 0; a < 4; ++a) {
@@ -203,7 +204,7 @@ static int build_tables(kmm_ctx *ctx) {
     }
     // reciprocals of the tau row coefficients (the same divisions as the device's tau_rhs)
     RET(upload_rj(ctx, &F->rj, false));
-    if (ctx->ny % 16 == 0) {   // the blocked column kernels' copies
+    if (kmm_blocked_ny(ctx->ny)) {   // the blocked column kernels' copies
         for (int c = 0; c < TB_N; ++c) {
             const int nc = (c == TB_U0 || c == TB_W0) ? 1 : ncols;
             const double *src[4] = {T.td[c], T.te[c], T.tb1[c], T.tb2[c]};
@@ -214,6 +215,16 @@ static int build_tables(kmm_ctx *ctx) {
             F->btabs.g[c] = T.g[c];
         }
         RET(upload_rj(ctx, &F->brj, true));
+    }
+    for (int c = 0; c < TB_N; ++c) {   // the canonical pivots become 1 / d too (K = 0: positions kept)
+        const size_t n = (size_t)((c == TB_U0 || c == TB_W0) ? 1 : ncols) * ctx->nyp;
+        double *r = NULL;
+        CK(cudaMalloc(&r, sizeof(double) * n));
+        k_tab_block<<<(int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184), 256, 0, ctx->stream>>>(T.td[c], r, (int)(n / ctx->nyp),
+                                                                                                 ctx->nyp, 0, 1);
+        CKL();
+        CK(cudaFree(T.td[c]));
+        T.td[c] = r;
     }
     RET(make_twf(ctx, 2 * ctx->ny, &F->twf_y2));
     RET(make_twf(ctx, ctx->mz, &F->twf_mz));
@@ -236,8 +247,8 @@ static int build_tables(kmm_ctx *ctx) {
 struct TauCache {
     int n;
     TabCfg cfg[KMM_TAU_SETS];
-    double *tabs[KMM_TAU_SETS][5];   // td (as 1 / d), te, tb1, tb2 in the lane-blocked order; tf
-    double *rj;                      // lane-blocked rj rows
+    double *tabs[KMM_TAU_SETS][5];   // td (as 1 / d), te, tb1, tb2 (lane-blocked for the blocked ny); tf
+    double *rj;                      // rj rows in the same order
 };
 
 int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, double ab, double bb, const double **tabs,
@@ -247,7 +258,7 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
         C = (TauCache *)calloc(1, sizeof(TauCache));
         if (!C) return KMM_ERR_NOMEM;
         ctx->tauc = C;
-        RET(upload_rj(ctx, &C->rj, true));
+        RET(upload_rj(ctx, &C->rj, kmm_blocked_ny(ctx->ny)));
     }
     const TabCfg want = {g, robin, robin ? at : 0.0, robin ? bt : 0.0, robin ? ab : 0.0, robin ? bb : 0.0, 1.0};
     int s = -1;
@@ -263,8 +274,15 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
         const int ncols = ctx->nz * ctx->nxh;
         const size_t n = (size_t)ncols * ctx->nyp;
         double *canon[4] = {NULL, NULL, NULL, NULL};
-        for (int a = 0; a < 4; ++a) CK(cudaMalloc(&canon[a], sizeof(double) * n));
-        CK(cudaMalloc(&C->tabs[s][4], sizeof(double) * 4 * ncols));
+        cudaError_t me = cudaMalloc(&C->tabs[s][4], sizeof(double) * 4 * ncols);
+        for (int a = 0; a < 4 && me == cudaSuccess; ++a) me = cudaMalloc(&canon[a], sizeof(double) * n);
+        if (me != cudaSuccess) {   // no room for tables: the caller keeps the table-free kernels
+            for (int a = 0; a < 4; ++a) cudaFree(canon[a]);
+            cudaFree(C->tabs[s][4]);
+            C->tabs[s][4] = NULL;
+            cudaGetLastError();
+            return KMM_ERR_UNSUPPORTED;
+        }
         k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(canon[0], canon[1], canon[2], canon[3],
                                                                   C->tabs[s][4], want, ctx->d_wavx, ctx->d_wavz,
                                                                   ncols, ctx->nz, ctx->nyp, ctx->dyde);
@@ -349,6 +367,145 @@ __device__ __forceinline__ void col_phirhs(Col<E> &x, const Col<E> &fn, const Co
         x.v[e] = make_double2(w.v[e].x - (1.0 - th) * d2.v[e].x / th, w.v[e].y - (1.0 - th) * d2.v[e].y / th);
 }
 
+// ---------------------------------------------------------------------------
+// The routine path's solve / penta (ib = 0) and its phirhs with one or two solves for the ny without
+// blocked kernels: one warp per column on the cached tables.  A thread per column recomputing the pivots
+// (an FP64 division in each link of the elimination's chain) took 136 us (Dirichlet) and 164 us (Robin) a
+// field at 80 x 61 x 60, where these take 9.
+// ---------------------------------------------------------------------------
+#define WC_WARPS 4
+
+struct WarpColJobs {
+    double2 *x[KMM_SOLVE_BATCH];
+    const double2 *fn[KMM_SOLVE_BATCH], *fnm1[KMM_SOLVE_BATCH];
+};
+
+struct WarpColCfg {
+    const double *tab[5];
+    double g;
+    int robin;
+};
+
+struct WarpColArgs {
+    const double *rj, *wavx, *wavz;
+    int ncols, nz, nyp;
+    double re, var, dt, th, dyde, c0;
+};
+
+template <int E>
+__device__ __forceinline__ void wc_solve(Col<E> &x, const WarpColCfg &S, const WarpColArgs &A, int col, double w2,
+                                         double2 gt, double2 gb) {
+    const TauTab T = {S.tab[0] + (size_t)col * A.nyp, S.tab[1] + (size_t)col * A.nyp, S.tab[2] + (size_t)col * A.nyp,
+                      S.tab[3] + (size_t)col * A.nyp, S.tab[4] + (size_t)col * 4};
+    if (S.robin) col_solve_robin<E>(x, T, gt, gb, w2 + S.g, A.nyp, A.c0, A.rj);
+    else col_solve_dirichlet<E>(x, T, gt, gb, w2 + S.g, A.nyp, A.c0, A.rj);
+}
+
+// rhs = 0: x <- solve(x) with boundary values gt, gb; rhs = 1: x <- solve(s)(phirhs([phi of] x)) with zero ones
+template <int E>
+__global__ void __launch_bounds__(WC_WARPS * 32) k_wc_solve(WarpColJobs J, WarpColCfg S0, WarpColCfg S1, int nsolve,
+                                                            int rhs, int phi, const double2 *gt, const double2 *gb,
+                                                            WarpColArgs A) {
+    const int col = blockIdx.x * WC_WARPS + (threadIdx.x >> 5);
+    if (col >= A.ncols) return;
+    const size_t off = (size_t)col * A.nyp;
+    double2 *X = J.x[blockIdx.y] + off;
+    const double kz = A.wavz[col % A.nz], kx = A.wavx[col / A.nz], w2 = kz * kz + kx * kx;
+    Col<E> x;
+    col_load<E>(x, X, A.nyp);
+    if (rhs) {
+        if (phi) {
+            Col<E> d1, d2;
+            col_cderiv<E>(d1, x, A.nyp, A.dyde);
+            col_cderiv<E>(d2, d1, A.nyp, A.dyde);
+#pragma unroll
+            for (int e = 0; e < E; ++e) x.v[e] = make_double2(d2.v[e].x - w2 * x.v[e].x, d2.v[e].y - w2 * x.v[e].y);
+        }
+        Col<E> f1, f0;
+        col_load<E>(f1, J.fn[blockIdx.y] + off, A.nyp);
+        if (J.fnm1[blockIdx.y]) {
+            col_load<E>(f0, J.fnm1[blockIdx.y] + off, A.nyp);
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e) f0.v[e] = make_double2(2.0 * f1.v[e].x, 2.0 * f1.v[e].y);
+        }
+        col_phirhs<E>(x, f1, f0, A.re, A.var, A.dt, A.th, w2, A.nyp, A.dyde);
+        const double2 zero = make_double2(0.0, 0.0);
+        wc_solve<E>(x, S0, A, col, w2, zero, zero);
+        if (nsolve > 1) wc_solve<E>(x, S1, A, col, w2, zero, zero);
+    } else {
+        wc_solve<E>(x, S0, A, col, w2, gt[col], gb[col]);
+    }
+    col_store<E>(X, x, A.nyp);
+}
+
+static int wc_launch(kmm_ctx *ctx, const WarpColJobs &J, int nf, const WarpColCfg *S, int nsolve, int rhs, int phi,
+                     double var, const double2 *gt, const double2 *gb, const double *rj) {
+    WarpColArgs A = {rj, ctx->d_wavx, ctx->d_wavz, ctx->nz * ctx->nxh, ctx->nz, ctx->nyp, ctx->re, var, ctx->dt,
+                     ctx->theta, ctx->dyde, ctx->h_c[0]};
+    const dim3 grid((A.ncols + WC_WARPS - 1) / WC_WARPS, nf);
+#define WC(EE) k_wc_solve<EE><<<grid, WC_WARPS * 32, 0, ctx->stream>>>(J, S[0], S[1], nsolve, rhs, phi, gt, gb, A)
+    switch ((ctx->nyp + 31) / 32) {
+    case 1: WC(1); break;
+    case 2: WC(2); break;
+    case 3: WC(3); break;
+    case 4: WC(4); break;
+    case 5: WC(5); break;
+    case 6: WC(6); break;
+    case 9: WC(9); break;
+    default: return KMM_ERR_UNSUPPORTED;
+    }
+#undef WC
+    CKL();
+    return KMM_OK;
+}
+
+static bool wc_has(const kmm_ctx *ctx) {
+    const int E = (ctx->nyp + 31) / 32;
+    return E <= 6 || E == 9;
+}
+
+int kmm_warpcol_solve_many(kmm_ctx *ctx, double2 *const *u, int nf, double g, int robin, double at, double bt,
+                           double ab, double bb, const double2 *gt, const double2 *gb) {
+    if (!wc_has(ctx)) return KMM_ERR_UNSUPPORTED;
+    WarpColCfg S[2];
+    const double *rj = NULL;
+    RET(kmm_tau_tabset(ctx, g, robin, at, bt, ab, bb, S[0].tab, &rj));
+    S[0].g = g;
+    S[0].robin = robin;
+    S[1] = S[0];
+    for (int f0 = 0; f0 < nf; f0 += KMM_SOLVE_BATCH) {
+        const int nb = nf - f0 < KMM_SOLVE_BATCH ? nf - f0 : KMM_SOLVE_BATCH;
+        WarpColJobs J;
+        memset(&J, 0, sizeof(J));
+        for (int m = 0; m < nb; ++m) J.x[m] = u[f0 + m];
+        RET(wc_launch(ctx, J, nb, S, 1, 0, 0, 1.0, gt, gb, rj));
+    }
+    return KMM_OK;
+}
+
+int kmm_warpcol_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
+                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec) {
+    if (!wc_has(ctx)) return KMM_ERR_UNSUPPORTED;
+    if (nf < 1 || nf > KMM_SOLVE_BATCH || nsolve < 1 || nsolve > 2) return KMM_ERR_ARG;
+    WarpColCfg S[2];
+    const double *rj = NULL;
+    for (int k = 0; k < 2; ++k) {
+        const KmmSolveSpec &q = spec[k < nsolve ? k : 0];
+        RET(kmm_tau_tabset(ctx, q.g, q.robin, q.at, q.bt, q.ab, q.bb, S[k].tab, &rj));
+        S[k].g = q.g;
+        S[k].robin = q.robin;
+    }
+    WarpColJobs J;
+    memset(&J, 0, sizeof(J));
+    for (int m = 0; m < nf; ++m) {
+        J.x[m] = x[m];
+        J.fn[m] = fn[m];
+        J.fnm1[m] = fnm1[m];
+    }
+    return wc_launch(ctx, J, nf, S, nsolve, 1, phi, var, NULL, NULL, rj);
+}
+
 // norm (helpers.f90:91-158) on a column pair held by the two warps of the block.  The exchange
 // buffer holds one column per warp; kx = 0 pairs (j, nz-j) average, (0,0) becomes real, the
 // kz Nyquist column is zeroed.
@@ -419,7 +576,8 @@ __device__ __forceinline__ void col_dct(Col<E> &x, double2 *a, double2 *b, const
 
 // L0 > 0: 2 ny is the compile-time constant L0 (specialised DCT); L0 = 0: runtime plan
 template <int E, int L0>
-__global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const __grid_constant__ DevPlan P) {
+__global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
+                                                const __grid_constant__ DevPlan P) {
     extern __shared__ double2 sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nyp = A.nyp, ny = nyp - 1, L = 2 * ny;
@@ -436,16 +594,23 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
     const bool mean = (kx == 0 && j == 0);
     const size_t ncols = (size_t)A.nz * A.nxh;
 
-    // ---- passive scalar (main_dns.f90:325-359)
-    Col<E> s;
-    if (A.scalar) {
+    // ---- passive scalar (main_dns.f90:325-359), independent of the velocity: the blocks of blockIdx.y = 1
+    if (blockIdx.y == 1) {
+        Col<E> s, n1, n0;
         col_load<E>(s, A.scal + off, nyp);
-        Col<E> n1, n0;
         col_load<E>(n1, A.scn + off, nyp);
         col_load<E>(n0, A.scnm1 + off, nyp);
         col_phirhs<E>(s, n1, n0, A.re, A.diff, A.dt, A.th, w2, nyp, A.dyde);
         const TauTab ts = tab_at(T, TB_SCL, col, nyp);
-        col_solve_robin<E>(s, ts, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + T.g[TB_SCL], nyp, A.c0);
+        col_solve_robin<E>(s, ts, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + T.g[TB_SCL], nyp, A.c0, rj);
+        col_norm<E>(s, xbuf, kx, j, A.nzh);
+        col_store<E>(A.scal + off, s, nyp);
+        col_cderiv<E>(n1, s, nyp, A.dyde);
+        col_dct<E, L0>(s, fa, fb, P, nyp, true);
+        col_store<E>(A.yp + 6 * ncols * nyp + off, s, nyp);
+        col_dct<E, L0>(n1, fa, fb, P, nyp, true);
+        col_store<E>(A.yp + 7 * ncols * nyp + off, n1, nyp);
+        return;
     }
     Col<E> v, d1, d2, om;
     if (kx == 0 && q == 0) {
@@ -475,7 +640,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         }
         const TauTab tm = tab_at(T, warp == 0 ? TB_U0 : TB_W0, 0, nyp);
         const double gt = warp == 0 ? A.gtu : A.gtw, gb = warp == 0 ? A.gbu : A.gbw;
-        col_solve_robin<E>(uc, tm, make_double2(gt, 0.0), make_double2(gb, 0.0), g1, nyp, A.c0);
+        col_solve_robin<E>(uc, tm, make_double2(gt, 0.0), make_double2(gb, 0.0), g1, nyp, A.c0, rj);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const int i = lane + 32 * e;
@@ -502,9 +667,9 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         }
         {
             const TauTab tp = tab_at(T, TB_PHI, col, nyp);
-            col_solve_dirichlet<E>(v, tp, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0);
+            col_solve_dirichlet<E>(v, tp, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0, rj);
             const TauTab tv = tab_at(T, TB_V, col, nyp);
-            col_solve_dirichlet<E>(v, tv, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2, nyp, A.c0);
+            col_solve_dirichlet<E>(v, tv, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2, nyp, A.c0, rj);
         }
         // ---- normal vorticity phirhs (main_dns.f90:411-422)
         col_load<E>(om, A.omy + off, nyp);
@@ -548,7 +713,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         // ---- normal vorticity Robin solve (main_dns.f90:479-484)
         {
             const TauTab to = tab_at(T, TB_OMY, col, nyp);
-            col_solve_robin<E>(om, to, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0);
+            col_solve_robin<E>(om, to, make_double2(0.0, 0.0), make_double2(0.0, 0.0), w2 + g1, nyp, A.c0, rj);
         }
     }
     // ---- norm(v), norm(omy); veloc (main_dns.f90:520-526, solvers.f90:1576-1659)
@@ -608,15 +773,6 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
     col_store<E>(yp + 2 * ncols * nyp + off, w, nyp);
     col_dct<E, L0>(d1, fa, fb, P, nyp, true);
     col_store<E>(yp + 5 * ncols * nyp + off, d1, nyp);
-    if (A.scalar) {
-        col_norm<E>(s, xbuf, kx, j, A.nzh);
-        col_store<E>(A.scal + off, s, nyp);
-        col_cderiv<E>(d1, s, nyp, A.dyde);
-        col_dct<E, L0>(s, fa, fb, P, nyp, true);
-        col_store<E>(yp + 6 * ncols * nyp + off, s, nyp);
-        col_dct<E, L0>(d1, fa, fb, P, nyp, true);
-        col_store<E>(yp + 7 * ncols * nyp + off, d1, nyp);
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1199,7 +1355,7 @@ static int fused_launch(kmm_ctx *ctx) {
 #define COLF(EE, LL)                                                                                  \
     do {                                                                                              \
         RET(kmm_smem_attr(ctx, (const void *)k_col_fwd<EE, LL>, smc));                                \
-        k_col_fwd<EE, LL><<<nblk, 64, smc, ctx->stream>>>(F, FU->tabs, ctx->wy2);                       \
+        k_col_fwd<EE, LL><<<dim3(nblk, scalar ? 2 : 1), 64, smc, ctx->stream>>>(F, FU->tabs, FU->rj, ctx->wy2);                \
     } while (0)
     switch (2 * ctx->ny) {   // specialised lengths: ny = 32, 64, 96, 128
     case 64: COLF(2, 64); break;

@@ -223,6 +223,13 @@ struct KmmSolveSpec {
 };
 int kmm_colblk_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec);
+// both for the other ny (a warp per column; ny up to 191 and 256 .. 287), called by the two above (kmm_fused.cu)
+int kmm_warpcol_solve_many(kmm_ctx *ctx, double2 *const *u, int nf, double g, int robin, double at, double bt,
+                           double ab, double bb, const double2 *gt, const double2 *gb);
+int kmm_warpcol_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
+                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec);
+// the ny whose column kernels and tau tables are in the blocked layout of kmm_colblk.cuh
+static inline bool kmm_blocked_ny(int ny) { return ny == 32 || ny == 64 || ny == 96 || ny == 128 || ny == 256; }
 // penta (ib = 0) of nf distinct fields of one configuration
 int kmm_internal_penta_many(kmm_ctx *ctx, double2 *const *u, int nf, double g, double at, double bt, double ab,
                             double bb, const double2 *gt, const double2 *gb);

@@ -118,7 +118,7 @@ __device__ __forceinline__ void col_nbr2(const Col<E> &s, Col<E> &sp2, Col<E> &s
 // tau right-hand-side rows for both parities in place (evns/odds without the BC row,
 // solvers.f90:387-496 / pntevns/pntodds 807-902); position i = p (row 1) is left as is
 template <int E>
-__device__ __forceinline__ void col_tau_rhs(Col<E> &s, int nyp, double c0) {
+__device__ __forceinline__ void col_tau_rhs(Col<E> &s, int nyp, double c0, const double *__restrict__ rj) {
     const int ny = nyp - 1;
     const int lane = threadIdx.x & 31;
     Col<E> sp2, sm2;
@@ -127,9 +127,7 @@ __device__ __forceinline__ void col_tau_rhs(Col<E> &s, int nyp, double c0) {
     for (int e = 0; e < E; ++e) {
         const int j = lane + 32 * e;
         if (j < 2 || j >= nyp) continue;
-        const double rj1 = 1.0 / (double)(4 * j * (j - 1));
-        const double rj2 = 1.0 / (double)(2 * (j * j - 1));
-        const double rj3 = 1.0 / (double)(4 * j * (j + 1));
+        const double rj1 = rj[j], rj2 = rj[nyp + j], rj3 = rj[2 * nyp + j];
         const double2 a = sm2.v[e], b = s.v[e], c = sp2.v[e];
         double2 w;
         if ((j & 1) == 0) {
@@ -160,16 +158,8 @@ __device__ __forceinline__ void col_tau_rhs(Col<E> &s, int nyp, double c0) {
     }
 }
 
-// tau matrix row coefficient a1(i) of evnc / oddc (solvers.f90:324-383), i = 1..m
-__device__ __forceinline__ double tau_a1(int i, int par, double wn) {
-    const int j = par == 0 ? 2 * i : 2 * i + 1;
-    double a1 = wn * (1.0 / (double)(4 * j * (j - 1)));
-    if (par == 0 && i == 1) a1 = 2.0 * a1;
-    return a1;
-}
-
 // Tables per column and configuration, indexed by coefficient position P = 2i + parity:
-//   td[P] = d(i) (i >= 1), te[P] = a3(i)/d(i+1) (forward multiplier), tb1/tb2[P] = border weights
+//   td[P] = 1 / d(i) (i >= 1; the pivots are used only as divisors), te[P] = a3(i)/d(i+1) (forward multiplier), tb1/tb2[P] = border weights
 //   of rows 2..n (for Dirichlet tb1 only), tf[0..3] = final f values:
 //   Dirichlet: tf[par] ; Robin: tf[2*(js-1) + par] = f(js, par)  (js 1 = top / tt, 2 = bottom / tb)
 struct TauTab {
@@ -237,7 +227,8 @@ __device__ __forceinline__ double2 col_border(const Col<E> &y, const double *__r
 
 // back substitution (affine prefix scan) from x at the BC position (row 1)
 template <int E>
-__device__ __forceinline__ void col_backsub(Col<E> &y, double2 x1, const double *__restrict__ td, double wn, int nyp) {
+__device__ __forceinline__ void col_backsub(Col<E> &y, double2 x1, const double *__restrict__ td, double wn, int nyp,
+                                            const double *__restrict__ rj) {
     const int lane = threadIdx.x & 31, par = lane & 1;
     const int ny = nyp - 1;
     const int n = par == 0 ? ny / 2 + 1 : ny / 2;
@@ -251,11 +242,11 @@ __device__ __forceinline__ void col_backsub(Col<E> &y, double2 x1, const double 
             b0 = x1.x;
             b1 = x1.y;
         } else if (P >= 2 + par && P <= top) {
-            const int i = (P - par) / 2;
-            const double d = td[P];
-            a = -tau_a1(i, par, wn) / d;
-            b0 = y.v[e].x / d;
-            b1 = y.v[e].y / d;
+            // a1(i) = wn / (4P(P-1)), doubled for P = 2 (evnc / oddc, solvers.f90:324-383)
+            const double r = td[P], a1 = wn * rj[P];
+            a = -(P == 2 ? 2.0 * a1 : a1) * r;
+            b0 = y.v[e].x * r;
+            b1 = y.v[e].y * r;
         }
         // inclusive prefix composition: (a,b) <- (a,b) o (a',b') with (a',b') from lane - off
 #pragma unroll
@@ -279,9 +270,9 @@ __device__ __forceinline__ void col_backsub(Col<E> &y, double2 x1, const double 
 // solve(...) with ib = 0 (Dirichlet), solvers.f90:174-283; s holds the right-hand side column
 template <int E>
 __device__ __forceinline__ void col_solve_dirichlet(Col<E> &s, const TauTab &T, double2 bct, double2 bcb, double wn,
-                                                    int nyp, double c0) {
+                                                    int nyp, double c0, const double *__restrict__ rj) {
     const int lane = threadIdx.x & 31, par = lane & 1;
-    col_tau_rhs<E>(s, nyp, c0);
+    col_tau_rhs<E>(s, nyp, c0, rj);
     col_forward<E>(s, T.te, nyp);
     const double2 sig = col_border<E>(s, T.tb1, nyp);
     // BC row: even 0.5(top + bot), odd 0.5(top - bot)
@@ -289,15 +280,15 @@ __device__ __forceinline__ void col_solve_dirichlet(Col<E> &s, const TauTab &T, 
                                 : make_double2(0.5 * (bct.x - bcb.x), 0.5 * (bct.y - bcb.y));
     const double f = T.tf[par];
     const double2 x1 = make_double2((w1.x - sig.x) / f, (w1.y - sig.y) / f);
-    col_backsub<E>(s, x1, T.td, wn, nyp);
+    col_backsub<E>(s, x1, T.td, wn, nyp, rj);
 }
 
 // penta(...) Robin BCs, solvers.f90:680-1061
 template <int E>
 __device__ __forceinline__ void col_solve_robin(Col<E> &s, const TauTab &T, double2 gtop, double2 gbot, double wn,
-                                                int nyp, double c0) {
+                                                int nyp, double c0, const double *__restrict__ rj) {
     const int lane = threadIdx.x & 31, par = lane & 1;
-    col_tau_rhs<E>(s, nyp, c0);
+    col_tau_rhs<E>(s, nyp, c0, rj);
     col_forward<E>(s, T.te, nyp);
     const double2 st = col_border<E>(s, T.tb1, nyp);   // top row (tt) contributions of this parity
     const double2 sb = col_border<E>(s, T.tb2, nyp);   // bottom row (tb)
@@ -312,7 +303,7 @@ __device__ __forceinline__ void col_solve_robin(Col<E> &s, const TauTab &T, doub
     double2 x1;
     if (par == 0) x1 = make_double2((s1.x * f22 - s2.x * f12) / det, (s1.y * f22 - s2.y * f12) / det);
     else x1 = make_double2((s2.x * f11 - s1.x * f21) / det, (s2.y * f11 - s1.y * f21) / det);
-    col_backsub<E>(s, x1, T.td, wn, nyp);
+    col_backsub<E>(s, x1, T.td, wn, nyp, rj);
 }
 
 // wall functionals c1derbw / c1dertw (derivatives.f90:362-401, 522-560)
