@@ -409,8 +409,11 @@ int kmm_fast_x(kmm_ctx *ctx, const double2 *q, double2 *r, int ic, int nout, boo
     case 1: FX_LAUNCH(1, 0);
     case 2: FX_LAUNCH(2, 0);
     case 3: FX_LAUNCH(3, 0);
+    case 4: FX_LAUNCH(4, 0);
     case 5: FX_LAUNCH(5, 0);
     case 6: FX_LAUNCH(6, 0);
+    case 7: FX_LAUNCH(7, 0);
+    case 8: FX_LAUNCH(8, 0);
     case 9: FX_LAUNCH(9, 0);
     case 12: FX_LAUNCH(12, 0);
     default: return KMM_ERR_UNSUPPORTED;

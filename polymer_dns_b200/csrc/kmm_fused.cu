@@ -800,7 +800,7 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb(const double2 *__restrict_
     double2 *stage = sm + (size_t)ZT_WARPS * 2 * mz;   // [y][z][kx] tile for the store
     const double kxv = act ? wavx[kx] : 0.0;
     auto SW = [](int x) { return MZ > 0 ? swz<double2>(x) : x; };
-    for (int g = 0; g < nout; ++g) {
+    for (int g = blockIdx.z; g < nout; g += gridDim.z) {
         if (act) {
             for (int z = lane; z < mz; z += 32) a[SW(z)] = make_double2(0.0, 0.0);
             __syncwarp();
@@ -861,7 +861,7 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zf(const double2 *__restrict_
     double2 *a = sm + (size_t)warp * 2 * mz, *b = a + mz;
     double2 *stage = sm + (size_t)ZT_WARPS * 2 * mz;   // [kx][kz][y] tile for the store
     auto SW = [](int x) { return MZ > 0 ? swz<double2>(x) : x; };
-    for (int o = 0; o < nout; ++o) {
+    for (int o = blockIdx.z; o < nout; o += gridDim.z) {
         if (act) {
             for (int z = lane; z < mz; z += 32) a[SW(z)] = __ldg(r + (((size_t)o * nyp + y) * mz + z) * nxh + kx);
             __syncwarp();
@@ -1125,10 +1125,12 @@ bool kmm_fused_applicable(const kmm_ctx *ctx) {
     if (ctx->p.scalar_on && ctx->p.scl_flag >= 2) return false;
     if (ctx->p.particle_flag > 0 && ctx->p.npart > 0) return false;   // inertial particles: routine vcw3dp
     const int E = (ctx->nyp + 31) / 32;
-    if (!(E == 2 || E == 3 || E == 4 || E == 5 || E == 9)) return false;
+    if (!(E <= 6 || E == 9)) return false;
     const int Ex = (ctx->mx + 31) / 32;
-    if (!(Ex == 1 || Ex == 2 || Ex == 3 || Ex == 5 || Ex == 6 || Ex == 9 || Ex == 12)) return false;
-    return true;
+    if (!(Ex <= 9 || Ex == 12)) return false;
+    // the plain-load z kernels' tiles must fit in shared memory (mz up to 300)
+    const bool ct_mz = ctx->mz == 48 || ctx->mz == 96 || ctx->mz == 144 || ctx->mz == 192;
+    return ct_mz || sizeof(double2) * (size_t)ctx->mz * (2 * ZT_WARPS + ZT_Y * ZT_KX) <= 227 * 1024;
 }
 
 
@@ -1364,10 +1366,12 @@ static int fused_launch(kmm_ctx *ctx) {
     case 256: COLF(5, 256); break;
     default:
         switch (E) {
+        case 1: COLF(1, 0); break;
         case 2: COLF(2, 0); break;
         case 3: COLF(3, 0); break;
         case 4: COLF(4, 0); break;
         case 5: COLF(5, 0); break;
+        case 6: COLF(6, 0); break;
         case 9: COLF(9, 0); break;
         default: return KMM_ERR_UNSUPPORTED;
         }
@@ -1412,7 +1416,7 @@ static int fused_launch(kmm_ctx *ctx) {
         case 192: ZB2(192, double2); break;
         default:
             RET(kmm_smem_attr(ctx, (const void *)k_zb<0>, smz));
-            k_zb<0><<<gz, ZT_WARPS * 32, smz, ctx->stream>>>(g_yp, g_q, ctx->d_wavx, ctx->d_wavz, ctx->wmz, nq, nyp, nz,
+            k_zb<0><<<dim3(gz.x, gz.y, nq), ZT_WARPS * 32, smz, ctx->stream>>>(g_yp, g_q, ctx->d_wavx, ctx->d_wavz, ctx->wmz, nq, nyp, nz,
                                                            nxh, mz);
             break;
         }
@@ -1469,7 +1473,7 @@ static int fused_launch(kmm_ctx *ctx) {
         case 192: ZF2(192, double2); break;
         default:
             RET(kmm_smem_attr(ctx, (const void *)k_zf<0>, smzf));
-            k_zf<0><<<gz, ZT_WARPS * 32, smzf, ctx->stream>>>(g_r, g_yo, ctx->wmz, nout, nyp, nz, nxh, mz,
+            k_zf<0><<<dim3(gz.x, gz.y, nout), ZT_WARPS * 32, smzf, ctx->stream>>>(g_r, g_yo, ctx->wmz, nout, nyp, nz, nxh, mz,
                                                             (double)ctx->mx * (double)mz);
             break;
         }
@@ -1500,10 +1504,12 @@ static int fused_launch(kmm_ctx *ctx) {
     case 256: COLB(5, 256); break;
     default:
         switch (E) {
+        case 1: COLB(1, 0); break;
         case 2: COLB(2, 0); break;
         case 3: COLB(3, 0); break;
         case 4: COLB(4, 0); break;
         case 5: COLB(5, 0); break;
+        case 6: COLB(6, 0); break;
         case 9: COLB(9, 0); break;
         default: return KMM_ERR_UNSUPPORTED;
         }
