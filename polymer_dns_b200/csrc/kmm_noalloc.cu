@@ -12,9 +12,8 @@
 
 #include "kmm_internal.cuh"
 
-__global__ void k_xyz_y(double *__restrict__ b, DevPlan P, int nyp, int ncols);
-__global__ void k_xyz_x(const double *__restrict__ b, double2 *__restrict__ a, DevPlan P, int nyp, int nz, int nx);
-__global__ void k_xyz_z(double2 *__restrict__ a, DevPlan P, int nyp, int nz);
+cudaError_t kmm_xyz_passes(const double *in, double *b, double2 *a, const DevPlan &py, const DevPlan &px,
+                           const DevPlan &pz, int nyp, int nz, int nx, cudaStream_t st);   // kmm_tracer.cu
 
 #define NOALLOC_TW_MAX 4096   // longest transform: 2 ny, nx and nz each at most this
 
@@ -84,26 +83,12 @@ extern "C" int kmm_xyzfft_noalloc(const double *phys, double *spec, int nx, int 
         }
         plans[t]->tw = s_tw[dev] + t * NOALLOC_TW_MAX;
     }
-    // shared memory of each kernel (at most 128 KiB at the 4096 limit): lengths past the 48 KiB
-    // default opt in once; setting a function attribute allocates nothing
-    const size_t sy = sizeof(double2) * 4 * (size_t)ny, sx = sizeof(double2) * 2 * (size_t)nx,
-                 sz = sizeof(double2) * 2 * (size_t)nz;
-    const void *kern[3] = {(const void *)k_xyz_y, (const void *)k_xyz_x, (const void *)k_xyz_z};
-    const size_t need[3] = {sy, sx, sz};
-    for (int t = 0; t < 3; ++t)
-        if (need[t] > 48 * 1024 &&
-            cudaFuncSetAttribute(kern[t], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need[t]) != cudaSuccess)
-            return KMM_ERR_CUDA;
-    // same sequence as kmm_xyzfft: copy, y DCT-I (/ny, halved ends), x r2c (/nx), z c2c (/nz)
-    double *b = s_scratch[dev];
-    if (cudaMemcpyAsync(b, phys, sizeof(double) * nyp * (size_t)nz * (size_t)nx, cudaMemcpyDeviceToDevice, st) !=
-        cudaSuccess)
+    // same passes as kmm_xyzfft: y DCT-I (/ny, halved ends) into the scratch, x r2c (/nx), z c2c (/nz)
+    DevPlan qy, qx, qz;
+    kmm_plan_r8(&py2, &qy);
+    kmm_plan_r8(&pnx, &qx);
+    kmm_plan_r8(&pnz, &qz);
+    if (kmm_xyz_passes(phys, s_scratch[dev], (double2 *)spec, qy, qx, qz, (int)nyp, nz, nx, st) != cudaSuccess)
         return KMM_ERR_CUDA;
-    k_xyz_y<<<nz * nx, 128, sy, st>>>(b, py2, (int)nyp, nz * nx);
-    if (cudaGetLastError() != cudaSuccess) return KMM_ERR_CUDA;
-    k_xyz_x<<<(int)nyp * nz, 128, sx, st>>>(b, (double2 *)spec, pnx, (int)nyp, nz, nx);
-    if (cudaGetLastError() != cudaSuccess) return KMM_ERR_CUDA;
-    k_xyz_z<<<(int)nyp * (nx / 2), 128, sz, st>>>((double2 *)spec, pnz, (int)nyp, nz);
-    if (cudaGetLastError() != cudaSuccess) return KMM_ERR_CUDA;
     return KMM_OK;
 }

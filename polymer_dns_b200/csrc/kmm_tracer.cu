@@ -464,57 +464,123 @@ extern "C" int kmm_tracer_cells(kmm_ctx *ctx, int *cells, size_t n) {
 // ---------------------------------------------------------------------------
 // xyzfft(a,b,-1), helpers.f90:6-87: physical (nyp,nz,nx) -> spectral (nyp,nz,nxh)
 // ---------------------------------------------------------------------------
-// y: DCT-I of each real column, /ny, halve the end values (in place on a real copy)
-__global__ void k_xyz_y(double *__restrict__ b, const __grid_constant__ DevPlan P, int nyp, int ncols) {
+// One warp per transform, two real lines in each as real and imaginary part of one complex FFT; a block's
+// warps take neighbouring lines, so that every pass moves runs of consecutive y (64 bytes in x, 128 in z).
+// With a block per real line, strided 8- and 16-byte accesses and a copy of the input first, the three
+// passes took 65 us a call at 64 x 97 x 64 where these take 29.
+
+// y: DCT-I of each real column, /ny, halve the end values
+__global__ void k_xyz_y(const double *__restrict__ in, double *__restrict__ b, const __grid_constant__ DevPlan P, int nyp,
+                        int ncols) {
     extern __shared__ double2 sm[];
     const int ny = nyp - 1, L = 2 * ny;
-    const int col = blockIdx.x;
-    if (col >= ncols) return;
-    double2 *a = sm, *c = sm + L;
-    double *src = b + (size_t)col * nyp;
-    for (int i = threadIdx.x; i < nyp; i += blockDim.x) {
-        const double v = src[i];
-        a[i] = make_double2(v, 0.0);
-        if (i > 0 && i < ny) a[L - i] = make_double2(v, 0.0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = 2 * (blockIdx.x * (blockDim.x >> 5) + warp);
+    if (c0 >= ncols) return;
+    const bool two = c0 + 1 < ncols;
+    double2 *a = sm + (size_t)warp * 2 * L, *c = a + L;
+    const double *src = in + (size_t)c0 * nyp;
+    for (int i = lane; i < nyp; i += 32) {
+        const double2 v = make_double2(src[i], two ? src[nyp + i] : 0.0);
+        a[i] = v;
+        if (i > 0 && i < ny) a[L - i] = v;
     }
-    __syncthreads();
-    double2 *r = fft_smem(P, a, c, 1, L, -1);
-    for (int i = threadIdx.x; i < nyp; i += blockDim.x) {
-        double v = r[i].x / (double)ny;
-        if (i == 0 || i == ny) v = v / 2.0;
-        src[i] = v;
+    __syncwarp();
+    const double2 *r = fft_warp(P, a, c, -1);
+    double *dst = b + (size_t)c0 * nyp;
+    for (int i = lane; i < nyp; i += 32) {
+        double2 v = make_double2(r[i].x / (double)ny, r[i].y / (double)ny);
+        if (i == 0 || i == ny) v = make_double2(v.x / 2.0, v.y / 2.0);
+        dst[i] = v.x;
+        if (two) dst[nyp + i] = v.y;
     }
 }
 
-// x: r2c over nx for each (i,j) line (stride nz*nyp), /nx, keep k < nxh -> complex work (nyp,nz,nxh)
+// x: r2c over nx for each (i,j) line (stride nz*nyp), /nx, keep k < nxh -> complex work (nyp,nz,nxh).
+// blockIdx.y is j; a block's W warps take the 2 W lines i0 .. i0 + 2 W - 1
 __global__ void k_xyz_x(const double *__restrict__ b, double2 *__restrict__ a, const __grid_constant__ DevPlan P, int nyp, int nz, int nx) {
     extern __shared__ double2 sm[];
-    const int line = blockIdx.x;   // i + nyp*j
-    const int i = line % nyp, j = line / nyp;
-    double2 *s = sm, *t = sm + nx;
-    for (int k = threadIdx.x; k < nx; k += blockDim.x) s[k] = make_double2(b[((size_t)k * nz + j) * nyp + i], 0.0);
+    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i0 = blockIdx.x * 2 * W, j = blockIdx.y;
+    const unsigned mW = div_magic(2 * W);
+    double *t = reinterpret_cast<double *>(sm);
+    for (int e = threadIdx.x; e < 2 * W * nx; e += blockDim.x) {
+        const int k = div_by(e, mW), il = e - k * 2 * W;
+        // line i0 + il: part il & 1 of element k of the warp's sequence il / 2
+        t[((size_t)(il >> 1) * 2 * nx + k) * 2 + (il & 1)] = i0 + il < nyp ? b[((size_t)k * nz + j) * nyp + i0 + il] : 0.0;
+    }
     __syncthreads();
-    double2 *r = fft_smem(P, s, t, 1, nx, -1);
+    double2 *s = sm + (size_t)warp * 2 * nx;
+    double2 *r = fft_warp(P, s, s + nx, -1);
+    // Z = A + i B -> A_k = (Z_k + conj Z_(n-k)) / 2, B_k = (Z_k - conj Z_(n-k)) / 2i, left in the other buffer:
+    // element 2 k + line
+    double2 *o = r == s ? s + nx : s;
     const int nxh = nx / 2;
-    for (int k = threadIdx.x; k < nxh; k += blockDim.x) {
-        double2 v = r[k];
-        a[((size_t)k * nz + j) * nyp + i] = make_double2(v.x / (double)nx, v.y / (double)nx);
+    for (int k = lane; k < nxh; k += 32) {
+        const double2 z = r[k], zc = cconj(r[k ? nx - k : 0]);
+        const double2 p = cadd(z, zc), m = csub(z, zc);
+        o[2 * k] = make_double2(0.5 * p.x / (double)nx, 0.5 * p.y / (double)nx);
+        o[2 * k + 1] = make_double2(0.5 * m.y / (double)nx, -0.5 * m.x / (double)nx);
+    }
+    __syncthreads();
+    const size_t half = (size_t)(o - s);   // the same for every warp (a stage count)
+    for (int e = threadIdx.x; e < 2 * W * nxh; e += blockDim.x) {
+        const int k = div_by(e, mW), il = e - k * 2 * W;
+        if (i0 + il < nyp)
+            a[((size_t)k * nz + j) * nyp + i0 + il] = sm[(size_t)(il >> 1) * 2 * nx + half + 2 * k + (il & 1)];
     }
 }
 
-// z: forward c2c over nz for each (i,k) line, /nz
+// z: forward c2c over nz for each (i,k) line, /nz; blockIdx.y is k, a block's W warps take the lines i0 .. i0 + W - 1
 __global__ void k_xyz_z(double2 *__restrict__ a, const __grid_constant__ DevPlan P, int nyp, int nz) {
     extern __shared__ double2 sm[];
-    const int line = blockIdx.x;   // i + nyp*k
-    const int i = line % nyp, k = line / nyp;
-    double2 *s = sm, *t = sm + nz;
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) s[j] = a[((size_t)k * nz + j) * nyp + i];
-    __syncthreads();
-    double2 *r = fft_smem(P, s, t, 1, nz, -1);
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        double2 v = r[j];
-        a[((size_t)k * nz + j) * nyp + i] = make_double2(v.x / (double)nz, v.y / (double)nz);
+    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const int i0 = blockIdx.x * W;
+    double2 *A = a + (size_t)blockIdx.y * nz * nyp;
+    const unsigned mW = div_magic(W);
+    for (int e = threadIdx.x; e < W * nz; e += blockDim.x) {
+        const int j = div_by(e, mW), il = e - j * W;
+        if (i0 + il < nyp) sm[(size_t)il * 2 * nz + j] = A[(size_t)j * nyp + i0 + il];
     }
+    __syncthreads();
+    double2 *s = sm + (size_t)warp * 2 * nz;
+    const size_t half = (size_t)(fft_warp(P, s, s + nz, -1) - s);
+    __syncthreads();
+    for (int e = threadIdx.x; e < W * nz; e += blockDim.x) {
+        const int j = div_by(e, mW), il = e - j * W;
+        if (i0 + il < nyp) {
+            const double2 v = sm[(size_t)il * 2 * nz + half + j];
+            A[(size_t)j * nyp + i0 + il] = make_double2(v.x / (double)nz, v.y / (double)nz);
+        }
+    }
+}
+
+// warps per block of a pass over lines of length n: `most` of them while their buffers (two of n values each)
+// stay within 96 KB, so that two blocks share an SM; one warp at the longest lengths (4096: 128 KB)
+static int xyz_warps(int n, int most) {
+    int w = most;
+    while (w > 1 && sizeof(double2) * 2 * (size_t)n * w > 96 * 1024) w /= 2;
+    return w;
+}
+
+// the three passes on stream st: in (nyp, nz, nx) real -> b (a real copy's space) -> a; py, px, pz: plans of
+// 2 ny, nx, nz (radix 8 first).  Nothing is allocated.
+cudaError_t kmm_xyz_passes(const double *in, double *b, double2 *a, const DevPlan &py, const DevPlan &px,
+                           const DevPlan &pz, int nyp, int nz, int nx, cudaStream_t st) {
+    const int wy = xyz_warps(py.n, 4), wx = xyz_warps(nx, 4), wz = xyz_warps(nz, 8), ncols = nz * nx;
+    const size_t sy = sizeof(double2) * 2 * (size_t)py.n * wy, sx = sizeof(double2) * 2 * (size_t)nx * wx,
+                 sz = sizeof(double2) * 2 * (size_t)nz * wz;
+    const void *kern[3] = {(const void *)k_xyz_y, (const void *)k_xyz_x, (const void *)k_xyz_z};
+    const size_t need[3] = {sy, sx, sz};
+    for (int t = 0; t < 3; ++t)   // setting a function attribute allocates nothing
+        if (need[t] > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(kern[t], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need[t]);
+            if (e != cudaSuccess) return e;
+        }
+    k_xyz_y<<<(ncols + 2 * wy - 1) / (2 * wy), wy * 32, sy, st>>>(in, b, py, nyp, ncols);
+    k_xyz_x<<<dim3((nyp + 2 * wx - 1) / (2 * wx), nz), wx * 32, sx, st>>>(b, a, px, nyp, nz, nx);
+    k_xyz_z<<<dim3((nyp + wz - 1) / wz, nx / 2), wz * 32, sz, st>>>(a, pz, nyp, nz);
+    return cudaGetLastError();
 }
 
 extern "C" int kmm_xyzfft(kmm_ctx *ctx, int dst, int src) {
@@ -525,13 +591,11 @@ extern "C" int kmm_xyzfft(kmm_ctx *ctx, int dst, int src) {
     const size_t np = (size_t)ctx->nyp * ctx->nz * ctx->nx;
     double *b = NULL;
     CK(cudaMallocAsync((void **)&b, sizeof(double) * np, ctx->stream));
-    CK(cudaMemcpyAsync(b, b0, sizeof(double) * np, cudaMemcpyDeviceToDevice, ctx->stream));
-    k_xyz_y<<<ctx->nz * ctx->nx, 128, sizeof(double2) * 4 * ctx->ny, ctx->stream>>>(b, ctx->py2, ctx->nyp, ctx->nz * ctx->nx);
-    CKL();
-    k_xyz_x<<<ctx->nyp * ctx->nz, 128, sizeof(double2) * 2 * ctx->nx, ctx->stream>>>(b, a, ctx->pnx, ctx->nyp, ctx->nz, ctx->nx);
-    CKL();
-    k_xyz_z<<<ctx->nyp * ctx->nxh, 128, sizeof(double2) * 2 * ctx->nz, ctx->stream>>>(a, ctx->pnz, ctx->nyp, ctx->nz);
-    CKL();
+    DevPlan px, pz;
+    kmm_plan_r8(&ctx->pnx, &px);
+    kmm_plan_r8(&ctx->pnz, &pz);
+    CK(kmm_xyz_passes(b0, b, a, ctx->wy2, px, pz, ctx->nyp, ctx->nz, ctx->nx, ctx->stream));
+    ctx->launches += 3;
     CK(cudaFreeAsync(b, ctx->stream));
     return KMM_OK;
 }
