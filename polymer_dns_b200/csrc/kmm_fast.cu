@@ -334,6 +334,123 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
     }
 }
 
+// The x stage for rows too long for a lane's registers (mx = 576): one block per (y, z) row and one
+// warp per field pair (NP = 3, or 5 with the scalar).  Each warp builds its pair's Hermitian extension
+// in a shared buffer of MX complex values, transforms it in place (the last stage through registers) and
+// leaves the two physical rows there; the block forms the pointwise terms of k_fx2, holding its points'
+// results in registers, and puts (h1, h2) and (h3, scalar term) into the first two buffers, which two warps
+// transform back.  The buffers are the only copy of a row: 46 KB a block, so three blocks of five warps share an SM.
+// It reads q and writes r once; the passes through HBM buffers of the physical inputs and outputs that it
+// replaces (k_xinv_big2, k_xpoint, k_xfwd2) took 8.1 ms at 384 x 257 x 384 with a scalar, this takes TBD.
+template <int MX, int NP>
+__global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
+    k_fx_row(const double2 *__restrict__ q, double2 *__restrict__ r, double *__restrict__ up3, double *__restrict__ vp3,
+             double *__restrict__ wp3, const double *__restrict__ seght, double *__restrict__ cfl,
+             double *__restrict__ umax, const double2 *__restrict__ tw, FxArgs A, int nyp, int mz) {
+    typedef double2 C;
+    constexpr int NXH = MX / 3, L = kct::nfac(MX), E = MX / 32, IT = (MX + NP * 32 - 1) / (NP * 32);
+    static_assert(MX % 32 == 0 && kct::stride(MX, L - 1) % 32 == 0, "the last stage's output x = lane + 32 e stays in its lane");
+    extern __shared__ double2 smd[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int z = blockIdx.x, y = blockIdx.y;
+    // ---- c2r of the pair (f, g): q fields 0..5, then A.ic, A.ic + 1 and A.ic + 2 alone
+    {
+        C *a = smd + (size_t)warp * MX;
+        const int f = warp < 3 ? 2 * warp : A.ic + 2 * (warp - 3);
+        const bool two = warp < 4;
+        const C *qa = q + (((size_t)f * nyp + y) * mz + z) * NXH, *qb = qa + (two ? (size_t)nyp * mz * NXH : 0);
+        const C zc = make_double2(0.0, 0.0);
+        for (int k = NXH + lane; k <= MX - NXH; k += 32) a[swz<C>(k)] = zc;   // modes nxh .. mx-nxh are not carried
+#pragma unroll
+        for (int e = 0; e < NXH / 32; ++e) {
+            const int k = lane + 32 * e;
+            C Av = __ldg(qa + k), Bv = two ? __ldg(qb + k) : zc;
+            if (k == 0) { Av.y = 0.0; Bv.y = 0.0; }   // c2r ignores Im of DC
+            a[swz<C>(k)] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
+            if (k > 0) a[swz<C>(MX - k)] = make_double2(Av.x + Bv.y, -Av.y + Bv.x);
+        }
+        __syncwarp();
+        kct::IpSteps<C, MX, 0, +1, 1, (1 >= L)>::go(a, tw, lane);
+        C rv[E];
+        auto ld = [&](int x) { return a[swz<C>(x)]; };
+        auto st = [&](int x, C v) { rv[x >> 5] = v; };
+        kct::stage_io<C, MX, L - 1, +1, 1>(ld, st, tw, lane);
+        __syncwarp();
+        double *pa = reinterpret_cast<double *>(a);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            pa[lane + 32 * e] = rv[e].x;
+            pa[MX + lane + 32 * e] = rv[e].y;
+        }
+    }
+    __syncthreads();
+    // ---- pointwise terms (solvers.f90:2891-3063)
+    const double *ph = reinterpret_cast<const double *>(smd);
+    double cmax = 0.0, umx = 0.0;
+    double h1[IT], h2[IT], h3[IT], sc[IT];
+    const double sg = seght[y];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+        const int x = threadIdx.x + i * NP * 32;
+        if (MX % (NP * 32) == 0 || x < MX) {
+            const double up = ph[x], vp = ph[MX + x], wp = ph[2 * MX + x];
+            const double wxp = ph[3 * MX + x], wyp = ph[4 * MX + x], wzp = ph[5 * MX + x];
+            h1[i] = vp * wzp - wp * wyp;
+            h2[i] = -up * wzp + wp * wxp;
+            h3[i] = up * wyp - vp * wxp;
+            if (A.flow_select == 1) h1[i] = h1[i] - A.dPdx;
+            if (NP == 5) {
+                double vc = -(up * ph[6 * MX + x] + vp * ph[7 * MX + x] + wp * ph[8 * MX + x]);
+                if (A.scalar_q != 0.0) vc = vc + A.scalar_q;
+                sc[i] = vc;
+            } else {
+                sc[i] = 0.0;
+            }
+            const double cc = (fabs(up) / A.delxm + fabs(vp) / sg + fabs(wp) / A.delzm) * A.dt;
+            cmax = (cc != cc) ? cc : fmax(cmax, cc);
+            umx = fmax(umx, fabs(up));
+            if (A.save_uvw) {
+                const size_t g3 = ((size_t)y * mz + z) * MX + x;
+                up3[g3] = up;
+                vp3[g3] = vp;
+                wp3[g3] = wp;
+            }
+        }
+    }
+    __syncthreads();   // every point has been read
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+        const int x = threadIdx.x + i * NP * 32;
+        if (MX % (NP * 32) == 0 || x < MX) {
+            smd[swz<C>(x)] = make_double2(h1[i], h2[i]);
+            smd[MX + swz<C>(x)] = make_double2(h3[i], sc[i]);
+        }
+    }
+    for (int off = 16; off; off >>= 1) {
+        const double c2 = __shfl_down_sync(0xffffffffu, cmax, off);
+        const double u2 = __shfl_down_sync(0xffffffffu, umx, off);
+        cmax = (c2 != c2) ? c2 : fmax(cmax, c2);
+        umx = fmax(umx, u2);
+    }
+    if (lane == 0) {
+        atomicMax((unsigned long long *)&cfl[y], (unsigned long long)__double_as_longlong(cmax));
+        atomicMax((unsigned long long *)&umax[y], (unsigned long long)__double_as_longlong(umx));
+    }
+    __syncthreads();
+    // ---- r2c of (h1, h2) and (h3, scalar term), modes kx < nxh
+    if (warp < 2) {
+        C *a = smd + (size_t)warp * MX;
+        fft_warp_ct_inplace<C, MX, -1>(a, tw);
+        C *oa = r + (((size_t)(2 * warp) * nyp + y) * mz + z) * NXH, *ob = oa + (size_t)nyp * mz * NXH;
+        const bool two = warp == 0 || NP == 5;
+        for (int k = lane; k < NXH; k += 32) {
+            const C Z = a[swz<C>(k)], Zc = cconj(a[swz<C>(k == 0 ? 0 : MX - k)]);
+            oa[k] = make_double2(0.5 * (Z.x + Zc.x), 0.5 * (Z.y + Zc.y));
+            if (two) ob[k] = make_double2(0.5 * (Z.y - Zc.y), -0.5 * (Z.x - Zc.x));
+        }
+    }
+}
+
 static FxArgs fx_args(const kmm_ctx *ctx, int ic, int nout, bool save_uvw) {
     FxArgs A;
     A.ic = ic;
@@ -393,6 +510,21 @@ int kmm_fast_x(kmm_ctx *ctx, const double2 *q, double2 *r, int ic, int nout, boo
     if (st2 != KMM_ERR_UNSUPPORTED) return st2;
     const FxArgs A = fx_args(ctx, ic, nout, save_uvw);
     const int mx = ctx->mx, mz = ctx->mz;
+    if (mx == 576) {   // nx = 384
+        const int np = nout > 3 ? 5 : 3;
+        const size_t sr = sizeof(double2) * (size_t)np * mx;
+#define FXR(NP)                                                                                        \
+    do {                                                                                               \
+        RET(kmm_smem_attr(ctx, (const void *)k_fx_row<576, NP>, sr));                                  \
+        k_fx_row<576, NP><<<dim3(mz, ctx->nyp), NP * 32, sr, ctx->stream>>>(                           \
+            q, r, up3, vp3, wp3, ctx->d_seght, ctx->d_cfl, ctx->d_umax, ctx->wmx.tw, A, ctx->nyp, mz);  \
+    } while (0)
+        if (np == 5) FXR(5);
+        else FXR(3);
+#undef FXR
+        CKL();
+        return KMM_OK;
+    }
     const size_t smem = sizeof(double2) * 2 * (size_t)mx * FX_WARPS;
     const dim3 grid((mz + FX_WARPS - 1) / FX_WARPS, ctx->nyp);
     const int E = (mx + 31) / 32;

@@ -1372,7 +1372,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     static const int fl[6] = {KMM_U, KMM_V, KMM_W, KMM_OMX, KMM_OMY, KMM_OMZ};
     for (int m = 0; m < 6; ++m) RET(add_in(S_U + m, fl[m]));
     if (scal) {
-        RET(add_in(S_SC, KMM_SCALAR));
+        if (poly) RET(add_in(S_SC, KMM_SCALAR));   // the scalar itself enters only the polymer's beta (itarget)
         if (derived) {
             RET(add_in_from(S_CX, KMM_SCALAR, 1));
             RET(add_in(S_CY, KMM_SCLY));
@@ -1559,7 +1559,13 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     const bool mx_compiled = mx == 48 || mx == 96 || mx == 144 || mx == 192;
     const bool xbig = (!mx_compiled && (sm_x + 1024 > 227 * 1024 || mx == 576)) ||
                       (ctx->force_xbig && ctx->p.precision == 0);
-    if (xbig) {
+    // the fused x stage (kmm_fast_x): no polymer, no immersed boundary, no inertial particles, no particle
+    // or targeted scalar source, FP64
+    const bool f32 = ctx->p.precision == 1 && ctx->in_step;
+    const bool fast_x = !poly && !ib_any && !inertial && !(scal && ctx->p.scl_flag >= 2) && !f32;
+    if (xbig && fast_x && mx == 576) {
+        // k_fx_row needs no buffer of the physical inputs
+    } else if (xbig) {
         RET(ensure_xbig(ctx, nin));
         RET(kmm_smem_attr(ctx, (const void *)k_xinv_big, sm_xf));
     } else {
@@ -1571,7 +1577,6 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
 
     // the mixed form (FP32 transforms and plane intermediates, pointwise terms evaluated in FP64 from
     // the FP32 values, FP64 state) inside kmm_step; FP64 elsewhere (initial, diagnostics)
-    const bool f32 = ctx->p.precision == 1 && ctx->in_step;
     const float2 *tw_y2 = NULL, *tw_mz = NULL, *tw_mx = NULL;
     if (f32) RET(kmm_routine_tw32(ctx, &tw_y2, &tw_mz, &tw_mx));
     float2 *pl_in32 = (float2 *)ctx->pl_in, *q_in32 = (float2 *)ctx->q_in;
@@ -1628,10 +1633,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     CKL();
     kmm_toc(ctx, KMM_STAGE_ZFFT_BWD);
     bool fast_done = false, xstat = false;
-    const bool sc_source = scal && ctx->p.scl_flag >= 2;
-    if (!poly && !ib_any && !inertial && !sc_source && !f32) {
-        // fused warp-per-row x stage (no polymer, no immersed boundary, no inertial particles, no
-        // particle scalar source)
+    if (fast_x) {
         kmm_tic(ctx);
         const bool save = ctx->p.npart > 0 || !ctx->in_step;
         const int fst = kmm_fast_x(ctx, ctx->q_in, ctx->q_out, scal ? A.slot_of_in[S_CX] : -1, nout, save, up3, vp3, wp3);
