@@ -4,6 +4,7 @@
 #include <stdlib.h>
 
 #include "kmm_internal.cuh"
+#include "kmm_fft.cuh"
 
 void kmm_set_error(kmm_ctx *ctx, const char *fmt, ...) {
     if (!ctx) return;
@@ -151,14 +152,16 @@ int kmm_plan_init(kmm_ctx *ctx, DevPlan *p, int n, int slot) {
     }
     p->n = n;
     p->nf = nf;
-    double2 *h = (double2 *)malloc(sizeof(double2) * (size_t)n);
+    const size_t nt = (size_t)kct::tw_total(n);
+    double2 *h = (double2 *)malloc(sizeof(double2) * nt);
     for (int k = 0; k < n; ++k) {
         long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
         h[k] = make_double2((double)cosl(a), -(double)sinl(a));
     }
+    tw_pack(h, n);
     double2 *d = NULL;
-    cudaError_t e = cudaMalloc(&d, sizeof(double2) * (size_t)n);
-    if (e == cudaSuccess) e = cudaMemcpy(d, h, sizeof(double2) * (size_t)n, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc(&d, sizeof(double2) * nt);
+    if (e == cudaSuccess) e = cudaMemcpy(d, h, sizeof(double2) * nt, cudaMemcpyHostToDevice);
     free(h);
     if (e != cudaSuccess) {
         kmm_set_error(ctx, "plan %d: %s", n, cudaGetErrorString(e));

@@ -7,7 +7,11 @@
 // and the twiddle index r k tstep never reaches N, so it needs no modulo.  The arithmetic per
 // butterfly is the same as fft_warp's: twiddle multiply of inputs r >= 1, then the radix-R DFT.
 //
-// C is double2 or float2; the twiddle table holds exp(-2 pi i m / N), m = 0..N-1, in the same type.
+// C is double2 or float2; the twiddle table holds exp(-2 pi i m / N), m = 0..N-1, in the same type, and
+// after it the packed tables of the stages (tw_off below): stage f's twiddles w^(r k) at (r - 1) NS + k.
+// A warp's lanes then read NS consecutive values per r (one to four 128-byte lines), where the strided
+// entries r k TSTEP of the natural table lie on up to eight.  At N = 192 the strided twiddle loads were
+// 27 % of the x stage's wavefronts in the load / store data pipe, which bound it (80 % busy).
 #pragma once
 
 #include "kmm_internal.cuh"
@@ -45,6 +49,19 @@ __host__ __device__ constexpr int stride(int n, int f) {
     for (int i = 0; i < f; ++i) p *= fac(n, i);
     return p;
 }
+
+// offset of stage f's twiddles in the packed table of length n (stage 0 has none), and its length tw_off(n, nfac(n))
+__host__ __device__ constexpr int tw_off(int n, int f) {
+    int o = 0;
+    for (int i = 1; i < f; ++i) o += (fac(n, i) - 1) * stride(n, i);
+    return o;
+}
+__host__ __device__ constexpr int tw_packed(int n) { return nfac(n) > 0 ? tw_off(n, nfac(n)) : 0; }
+// a table of length n: n natural entries, the packed table of n, and (n even) that of n / 2
+__host__ __device__ constexpr int tw_total(int n) { return n + tw_packed(n) + (n % 2 == 0 ? tw_packed(n / 2) : 0); }
+// where the packed table of length N starts in a table of length TWS N
+template <int N, int TWS>
+constexpr int tw_base = TWS == 1 ? N : 2 * N + tw_packed(2 * N);
 
 // ---- complex arithmetic on double2 / float2
 template <typename C>
@@ -186,7 +203,7 @@ __device__ __forceinline__ void stage(const C *__restrict__ src, C *__restrict__
     constexpr int R = fac(N, F);
     constexpr int NS = stride(N, F);
     constexpr int NR = N / R;
-    constexpr int TSTEP = N / (NS * R);
+    constexpr int TW0 = tw_base<N, TWS> + tw_off(N, F);
     constexpr int IT = (NQ * NR + 31) / 32;
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
@@ -202,7 +219,7 @@ __device__ __forceinline__ void stage(const C *__restrict__ src, C *__restrict__
                 const int xi = base + j + r * NR;
                 C x = src[SWZ ? swz<C>(xi) : xi];
                 if (NS > 1 && r > 0 && k) {
-                    C w = __ldg(&tw[r * k * TSTEP * TWS]);
+                    C w = __ldg(&tw[TW0 + (r - 1) * NS + k]);
                     if (S > 0) w.y = -w.y;
                     x = mul(x, w);
                 }
@@ -241,7 +258,7 @@ __device__ __forceinline__ void stage_io(LD &ld, ST &st, const C *__restrict__ t
     constexpr int R = fac(N, F);
     constexpr int NS = stride(N, F);
     constexpr int NR = N / R;
-    constexpr int TSTEP = N / (NS * R);
+    constexpr int TW0 = tw_base<N, TWS> + tw_off(N, F);
     constexpr int IT = (NR + 31) / 32;
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
@@ -253,7 +270,7 @@ __device__ __forceinline__ void stage_io(LD &ld, ST &st, const C *__restrict__ t
             for (int r = 0; r < R; ++r) {
                 C x = ld(j + r * NR);
                 if (NS > 1 && r > 0 && k) {
-                    C w = __ldg(&tw[r * k * TSTEP * TWS]);
+                    C w = __ldg(&tw[TW0 + (r - 1) * NS + k]);
                     if (S > 0) w.y = -w.y;
                     x = mul(x, w);
                 }
@@ -274,7 +291,7 @@ __device__ __forceinline__ void stage_ip(C *x, const C *__restrict__ tw, int lan
     constexpr int R = fac(N, F);
     constexpr int NS = stride(N, F);
     constexpr int NR = N / R;
-    constexpr int TSTEP = N / (NS * R);
+    constexpr int TW0 = tw_base<N, TWS> + tw_off(N, F);
     constexpr int IT = (NR + 31) / 32;
     C v[IT][R];
 #pragma unroll
@@ -286,7 +303,7 @@ __device__ __forceinline__ void stage_ip(C *x, const C *__restrict__ tw, int lan
             for (int r = 0; r < R; ++r) {
                 C u = x[swz<C>(j + r * NR)];
                 if (NS > 1 && r > 0 && k) {
-                    C w = __ldg(&tw[r * k * TSTEP * TWS]);
+                    C w = __ldg(&tw[TW0 + (r - 1) * NS + k]);
                     if (S > 0) w.y = -w.y;
                     u = mul(u, w);
                 }
@@ -344,8 +361,8 @@ struct MidSteps<C, N, F, S, TWS, false> {
 // S = -1: exp(-2 pi i jk/N) (FFTW_FORWARD), +1: exp(+...) (FFTW_BACKWARD).  NQ sequences of
 // length N lie N apart in a; b is a scratch buffer of the same size (both private to the calling
 // warp); the input must be visible to the whole warp (__syncwarp after writing it).  Returns the
-// buffer holding the result.  SWZ: the buffers are swizzled (element x at swz<C>(x)).  TWS: the
-// table holds the twiddles of length TWS N (exp(-2 pi i m/N) is entry TWS m).
+// buffer holding the result.  SWZ: the buffers are swizzled (element x at swz<C>(x)).  TWS (1 or 2): the
+// table is that of length TWS N.
 template <typename C, int N, int S, int NQ = 1, bool SWZ = false, int TWS = 1>
 __device__ __forceinline__ C *fft_warp_ct(C *a, C *b, const C *tw) {
     static_assert(kct::nfac(N) > 0, "transform length must be 2^a 3^b 5^c");
@@ -394,6 +411,22 @@ __device__ __forceinline__ void fft_warp_ct_inplace(C *a, const C *tw) {
     const int lane = threadIdx.x & 31;
     kct::IpSteps<C, N, 0, S, TWS, (1 >= L)>::go(a, tw, lane);
     kct::stage_ip<C, N, L - 1, S, TWS>(a, tw, lane);
+}
+
+// the packed tables behind the n natural entries of a host table t of tw_total(n) values
+template <typename C>
+inline void tw_pack(C *t, int n) {
+    int o = n;
+    for (int h = 1; h <= 2; ++h) {   // lengths n and n / 2
+        const int N = n / h;
+        if (h == 2 && n % 2) break;
+        if (kct::nfac(N) <= 0) continue;
+        for (int f = 1; f < kct::nfac(N); ++f) {
+            const int R = kct::fac(N, f), ns = kct::stride(N, f), step = N / (ns * R);
+            for (int r = 1; r < R; ++r)
+                for (int k = 0; k < ns; ++k) t[o++] = t[r * k * step * h];
+        }
+    }
 }
 
 // the transform lengths with compiled instances (3/2-rule grids of nx, nz = 32, 64, 96, 128, 384

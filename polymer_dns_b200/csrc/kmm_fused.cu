@@ -159,13 +159,15 @@ static int upload_rj(kmm_ctx *ctx, double **out, bool blocked) {
 
 // FP32 twiddles exp(-2 pi i m/n), rounded from long double, for the mixed-precision transforms
 static int make_twf(kmm_ctx *ctx, int n, float2 **out) {
-    float2 *h = (float2 *)malloc(sizeof(float2) * (size_t)n);
+    const size_t nt = (size_t)kct::tw_total(n);
+    float2 *h = (float2 *)malloc(sizeof(float2) * nt);
     for (int k = 0; k < n; ++k) {
         const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
         h[k] = make_float2((float)cosl(a), -(float)sinl(a));
     }
-    cudaError_t e = cudaMalloc(out, sizeof(float2) * (size_t)n);
-    if (e == cudaSuccess) e = cudaMemcpy(*out, h, sizeof(float2) * (size_t)n, cudaMemcpyHostToDevice);
+    tw_pack(h, n);
+    cudaError_t e = cudaMalloc(out, sizeof(float2) * nt);
+    if (e == cudaSuccess) e = cudaMemcpy(*out, h, sizeof(float2) * nt, cudaMemcpyHostToDevice);
     free(h);
     CK(e);
     return KMM_OK;
