@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int y = blockIdx.y;
     const int z = blockIdx.x * FX_WARPS + warp;
-    C *a = sm + (size_t)warp * 2 * MX, *b = a + MX;
+    C *a = sm + (size_t)warp * 2 * flen<C>(MX), *b = a + flen<C>(MX);
     double cmax = 0.0, umx = 0.0;
     const C zc = kct::mk<C>((T)0, (T)0);
     C pa[NE], pb[NE];   // coefficients of the pair in flight
@@ -196,15 +196,15 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
     // Hermitian c2r of the fetched pair: Z_k = A_k + i B_k (k <= HX), conj(A) + i conj(B) mirrored
     auto inv = [&](T *ra, T *rb) {
         for (int k = lane; k <= MX - NXH; k += 32)
-            if (k >= NXH) a[swz<C>(k)] = zc;   // modes nxh .. mx-nxh are not carried
+            if (k >= NXH) a[fpos<C>(k)] = zc;   // modes nxh .. mx-nxh are not carried
 #pragma unroll
         for (int e = 0; e < NE; ++e) {
             const int k = lane + 32 * e;
             if (k < NXH) {
                 C Av = pa[e], Bv = pb[e];
                 if (k == 0) { Av.y = (T)0; Bv.y = (T)0; }   // c2r ignores Im of DC
-                a[swz<C>(k)] = kct::mk<C>(Av.x - Bv.y, Av.y + Bv.x);
-                if (k > 0) a[swz<C>(MX - k)] = kct::mk<C>(Av.x + Bv.y, -Av.y + Bv.x);
+                a[fpos<C>(k)] = kct::mk<C>(Av.x - Bv.y, Av.y + Bv.x);
+                if (k > 0) a[fpos<C>(MX - k)] = kct::mk<C>(Av.x + Bv.y, -Av.y + Bv.x);
             }
         }
         __syncwarp();
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
     constexpr bool REG_OUT = kct::stride(MX, kct::nfac(MX) - 1) % 32 == 0;
     auto run_inv = [&](T *ra, T *rb) {
         if constexpr (REG_OUT) {
-            auto ld = [&](int x) { return a[swz<C>(x)]; };
+            const FftBuf<C> ld{a};
             auto st = [&](int x, C v) {
                 ra[x >> 5] = v.x;
                 rb[x >> 5] = v.y;
@@ -222,12 +222,12 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
             auto pre = [] {};
             fft_warp_ct_io<C, MX, +1>(ld, st, pre, b, a, tw);
         } else {
-            const C *res = fft_warp_ct<C, MX, +1, 1, true>(a, b, tw);
+            const C *res = fft_warp_ct<C, MX, +1, 1, FMODE<C>>(a, b, tw);
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const int x = lane + 32 * e;
                 if (x < MX) {
-                    const C v = res[swz<C>(x)];
+                    const C v = res[fpos<C>(x)];
                     ra[e] = v.x;
                     rb[e] = v.y;
                 }
@@ -239,18 +239,18 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const int x = lane + 32 * e;
-            if (x < MX) a[swz<C>(x)] = kct::mk<C>(ra[e], has_g ? rb[e] : (T)0);
+            if (x < MX) a[fpos<C>(x)] = kct::mk<C>(ra[e], has_g ? rb[e] : (T)0);
         }
         __syncwarp();
-        const C *res = fft_warp_ct<C, MX, -1, 1, true>(a, b, tw);
+        const C *res = fft_warp_ct<C, MX, -1, 1, FMODE<C>>(a, b, tw);
         C *oa = r + (((size_t)o * nyp + y) * mz + z) * NXH;
         C *ob = r + (((size_t)(o + 1) * nyp + y) * mz + z) * NXH;
 #pragma unroll
         for (int e = 0; e < NE; ++e) {
             const int k = lane + 32 * e;
             if (k < NXH) {
-                const C Z = res[swz<C>(k)];
-                C Zc = res[swz<C>(k == 0 ? 0 : MX - k)];
+                const C Z = res[fpos<C>(k)];
+                C Zc = res[fpos<C>(k == 0 ? 0 : MX - k)];
                 Zc.y = -Zc.y;
                 oa[k] = kct::mk<C>((T)0.5 * (Z.x + Zc.x), (T)0.5 * (Z.y + Zc.y));
                 if (has_g) ob[k] = kct::mk<C>((T)0.5 * (Z.y - Zc.y), (T)-0.5 * (Z.x - Zc.x));
@@ -348,31 +348,31 @@ __global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
              double *__restrict__ wp3, const double *__restrict__ seght, double *__restrict__ cfl,
              double *__restrict__ umax, const double2 *__restrict__ tw, FxArgs A, int nyp, int mz) {
     typedef double2 C;
-    constexpr int NXH = MX / 3, L = kct::nfac(MX), E = MX / 32, IT = (MX + NP * 32 - 1) / (NP * 32);
+    constexpr int NXH = MX / 3, L = kct::nfac(MX), E = MX / 32, FL = flen<C>(MX), IT = (MX + NP * 32 - 1) / (NP * 32);
     static_assert(MX % 32 == 0 && kct::stride(MX, L - 1) % 32 == 0, "the last stage's output x = lane + 32 e stays in its lane");
     extern __shared__ double2 smd[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int z = blockIdx.x, y = blockIdx.y;
     // ---- c2r of the pair (f, g): q fields 0..5, then A.ic, A.ic + 1 and A.ic + 2 alone
     {
-        C *a = smd + (size_t)warp * MX;
+        C *a = smd + (size_t)warp * FL;
         const int f = warp < 3 ? 2 * warp : A.ic + 2 * (warp - 3);
         const bool two = warp < 4;
         const C *qa = q + (((size_t)f * nyp + y) * mz + z) * NXH, *qb = qa + (two ? (size_t)nyp * mz * NXH : 0);
         const C zc = make_double2(0.0, 0.0);
-        for (int k = NXH + lane; k <= MX - NXH; k += 32) a[swz<C>(k)] = zc;   // modes nxh .. mx-nxh are not carried
+        for (int k = NXH + lane; k <= MX - NXH; k += 32) a[fpos<C>(k)] = zc;   // modes nxh .. mx-nxh are not carried
 #pragma unroll
         for (int e = 0; e < NXH / 32; ++e) {
             const int k = lane + 32 * e;
             C Av = __ldg(qa + k), Bv = two ? __ldg(qb + k) : zc;
             if (k == 0) { Av.y = 0.0; Bv.y = 0.0; }   // c2r ignores Im of DC
-            a[swz<C>(k)] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
-            if (k > 0) a[swz<C>(MX - k)] = make_double2(Av.x + Bv.y, -Av.y + Bv.x);
+            a[fpos<C>(k)] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
+            if (k > 0) a[fpos<C>(MX - k)] = make_double2(Av.x + Bv.y, -Av.y + Bv.x);
         }
         __syncwarp();
         kct::IpSteps<C, MX, 0, +1, 1, (1 >= L)>::go(a, tw, lane);
         C rv[E];
-        auto ld = [&](int x) { return a[swz<C>(x)]; };
+        const FftBuf<C> ld{a};
         auto st = [&](int x, C v) { rv[x >> 5] = v; };
         kct::stage_io<C, MX, L - 1, +1, 1>(ld, st, tw, lane);
         __syncwarp();
@@ -385,7 +385,8 @@ __global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
     }
     __syncthreads();
     // ---- pointwise terms (solvers.f90:2891-3063)
-    const double *ph = reinterpret_cast<const double *>(smd);
+    // field f's row: half of pair f / 2's buffer
+    auto row = [&](int f) { return reinterpret_cast<const double *>(smd) + (size_t)(f >> 1) * 2 * FL + (f & 1) * MX; };
     double cmax = 0.0, umx = 0.0;
     double h1[IT], h2[IT], h3[IT], sc[IT];
     const double sg = seght[y];
@@ -393,14 +394,14 @@ __global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
     for (int i = 0; i < IT; ++i) {
         const int x = threadIdx.x + i * NP * 32;
         if (MX % (NP * 32) == 0 || x < MX) {
-            const double up = ph[x], vp = ph[MX + x], wp = ph[2 * MX + x];
-            const double wxp = ph[3 * MX + x], wyp = ph[4 * MX + x], wzp = ph[5 * MX + x];
+            const double up = row(0)[x], vp = row(1)[x], wp = row(2)[x];
+            const double wxp = row(3)[x], wyp = row(4)[x], wzp = row(5)[x];
             h1[i] = vp * wzp - wp * wyp;
             h2[i] = -up * wzp + wp * wxp;
             h3[i] = up * wyp - vp * wxp;
             if (A.flow_select == 1) h1[i] = h1[i] - A.dPdx;
             if (NP == 5) {
-                double vc = -(up * ph[6 * MX + x] + vp * ph[7 * MX + x] + wp * ph[8 * MX + x]);
+                double vc = -(up * row(6)[x] + vp * row(7)[x] + wp * row(8)[x]);
                 if (A.scalar_q != 0.0) vc = vc + A.scalar_q;
                 sc[i] = vc;
             } else {
@@ -422,8 +423,8 @@ __global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
     for (int i = 0; i < IT; ++i) {
         const int x = threadIdx.x + i * NP * 32;
         if (MX % (NP * 32) == 0 || x < MX) {
-            smd[swz<C>(x)] = make_double2(h1[i], h2[i]);
-            smd[MX + swz<C>(x)] = make_double2(h3[i], sc[i]);
+            smd[fpos<C>(x)] = make_double2(h1[i], h2[i]);
+            smd[FL + fpos<C>(x)] = make_double2(h3[i], sc[i]);
         }
     }
     for (int off = 16; off; off >>= 1) {
@@ -439,12 +440,12 @@ __global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
     __syncthreads();
     // ---- r2c of (h1, h2) and (h3, scalar term), modes kx < nxh
     if (warp < 2) {
-        C *a = smd + (size_t)warp * MX;
+        C *a = smd + (size_t)warp * FL;
         fft_warp_ct_inplace<C, MX, -1>(a, tw);
         C *oa = r + (((size_t)(2 * warp) * nyp + y) * mz + z) * NXH, *ob = oa + (size_t)nyp * mz * NXH;
         const bool two = warp == 0 || NP == 5;
         for (int k = lane; k < NXH; k += 32) {
-            const C Z = a[swz<C>(k)], Zc = cconj(a[swz<C>(k == 0 ? 0 : MX - k)]);
+            const C Z = a[fpos<C>(k)], Zc = cconj(a[fpos<C>(k == 0 ? 0 : MX - k)]);
             oa[k] = make_double2(0.5 * (Z.x + Zc.x), 0.5 * (Z.y + Zc.y));
             if (two) ob[k] = make_double2(0.5 * (Z.y - Zc.y), -0.5 * (Z.x - Zc.x));
         }
@@ -472,7 +473,7 @@ int kmm_fast_x2(kmm_ctx *ctx, const void *q, void *r, const void *tw, bool fp32,
     if (nout < 3 || nout > 4 || (nout == 4) != (ic >= 0)) return KMM_ERR_UNSUPPORTED;
     const FxArgs A = fx_args(ctx, ic, nout, save_uvw);
     const int mx = ctx->mx, mz = ctx->mz;
-    const size_t smem = (fp32 ? sizeof(float2) : sizeof(double2)) * 2 * (size_t)mx * FX_WARPS;
+    const size_t smem = (fp32 ? sizeof(float2) * flen<float2>(mx) : sizeof(double2) * flen<double2>(mx)) * 2 * FX_WARPS;
     const dim3 grid((mz + FX_WARPS - 1) / FX_WARPS, ctx->nyp);
 #define FX2(MM, CC)                                                                                     \
     do {                                                                                                \
@@ -512,7 +513,7 @@ int kmm_fast_x(kmm_ctx *ctx, const double2 *q, double2 *r, int ic, int nout, boo
     const int mx = ctx->mx, mz = ctx->mz;
     if (mx == 576) {   // nx = 384
         const int np = nout > 3 ? 5 : 3;
-        const size_t sr = sizeof(double2) * (size_t)np * mx;
+        const size_t sr = sizeof(double2) * (size_t)np * flen<double2>(mx);
 #define FXR(NP)                                                                                        \
     do {                                                                                               \
         RET(kmm_smem_attr(ctx, (const void *)k_fx_row<576, NP>, sr));                                  \

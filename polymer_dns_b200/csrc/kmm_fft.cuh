@@ -14,6 +14,8 @@
 // 27 % of the x stage's wavefronts in the load / store data pipe, which bound it (80 % busy).
 #pragma once
 
+#include <type_traits>
+
 #include "kmm_internal.cuh"
 
 namespace kct {
@@ -105,6 +107,31 @@ __device__ __forceinline__ int swz(int x) {
     return x ^ ((x >> RB) & RM);
 }
 
+// The FFT buffers in FP64 are padded instead, one element after every eight (128 bytes): element x at
+// x + x / 8.  The accesses above are as free of conflicts, and where a stage's strides are multiples of
+// eight (all but the first stages of 48, 96 and 144) its addresses are one base plus constants, where the
+// swizzle takes three or four integer instructions an access: 40 % of the FP64 transforms' instructions.
+// FP32 buffers keep the swizzle (their 16-element rows do not match the stages' strides).
+template <typename C>
+constexpr int FMODE = sizeof(C) == 16 ? 2 : 1;   // 0: plain, 1: swizzled, 2: padded
+
+template <typename C, int MODE = FMODE<C>>
+__device__ __forceinline__ int fpos(int x) {
+    return MODE == 2 ? x + (x >> 3) : MODE == 1 ? swz<C>(x) : x;
+}
+
+// elements of a buffer of n values (n a multiple of 8 where padded)
+template <typename C, int MODE = FMODE<C>>
+__host__ __device__ constexpr int flen(int n) {
+    return MODE == 2 ? n + n / 8 : n;
+}
+
+// a transform's buffer as the source or target of a stage
+template <typename C, int MODE = FMODE<C>>
+struct FftBuf {
+    C *p;
+};
+
 namespace kct {
 
 // radix-R DFTs, X_q = sum_r v_r exp(S 2 pi i r q / R); the same operation sequence as radix_dft /
@@ -195,9 +222,46 @@ struct Dft<C, 8, S> {
     }
 };
 
+// element j + r D of a stage's source, r = 0 .. R-1
+template <typename C, int D, typename LD>
+struct Src {
+    LD &ld;
+    int j;
+    __device__ __forceinline__ Src(LD &l, int jj) : ld(l), j(jj) {}
+    __device__ __forceinline__ C operator()(int r) const { return ld(j + r * D); }
+};
+template <typename C, int D, int MODE>
+struct Src<C, D, const FftBuf<C, MODE>> {
+    static constexpr bool AFF = MODE == 0 || (MODE == 2 && D % 8 == 0);
+    const C *p;
+    int j;
+    __device__ __forceinline__ Src(const FftBuf<C, MODE> &b, int jj) : p(b.p + (AFF ? fpos<C, MODE>(jj) : 0)), j(jj) {}
+    __device__ __forceinline__ C operator()(int r) const {
+        return AFF ? p[r * flen<C, MODE>(D)] : p[fpos<C, MODE>(j + r * D)];
+    }
+};
+// element x + q D of its target; x a multiple of R D plus something below D
+template <typename C, int R, int D, typename ST>
+struct Dst {
+    ST &st;
+    int x;
+    __device__ __forceinline__ Dst(ST &s, int xx) : st(s), x(xx) {}
+    __device__ __forceinline__ void operator()(int q, C v) const { st(x + q * D, v); }
+};
+template <typename C, int R, int D, int MODE>
+struct Dst<C, R, D, const FftBuf<C, MODE>> {
+    static constexpr bool AFF = MODE == 0 || (MODE == 2 && (D % 8 == 0 || (D == 1 && R == 8)));
+    C *p;
+    int x;
+    __device__ __forceinline__ Dst(const FftBuf<C, MODE> &b, int xx) : p(b.p + (AFF ? fpos<C, MODE>(xx) : 0)), x(xx) {}
+    __device__ __forceinline__ void operator()(int q, C v) const {
+        p[AFF ? (D == 1 ? q : q * flen<C, MODE>(D)) : fpos<C, MODE>(x + q * D)] = v;
+    }
+};
+
 // one Stockham stage: butterflies j = 0..N/R-1 of each of the NQ sequences (stored N apart)
 // spread over the 32 lanes
-template <typename C, int N, int F, int S, int NQ, bool SWZ, int TWS>
+template <typename C, int N, int F, int S, int NQ, int MODE, int TWS>
 __device__ __forceinline__ void stage(const C *__restrict__ src, C *__restrict__ dst, const C *__restrict__ tw,
                                       int lane) {
     constexpr int R = fac(N, F);
@@ -214,10 +278,10 @@ __device__ __forceinline__ void stage(const C *__restrict__ src, C *__restrict__
             const int base = sq * N;
             const int k = j % NS;
             C v[R];
+            const Src<C, NR, const FftBuf<C, MODE>> in(FftBuf<C, MODE>{const_cast<C *>(src)}, base + j);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const int xi = base + j + r * NR;
-                C x = src[SWZ ? swz<C>(xi) : xi];
+                C x = in(r);
                 if (NS > 1 && r > 0 && k) {
                     C w = __ldg(&tw[TW0 + (r - 1) * NS + k]);
                     if (S > 0) w.y = -w.y;
@@ -226,35 +290,34 @@ __device__ __forceinline__ void stage(const C *__restrict__ src, C *__restrict__
                 v[r] = x;
             }
             Dft<C, R, S>::run(v);
-            const int idxD = base + (j - k) * R + k;
+            const Dst<C, R, NS, const FftBuf<C, MODE>> out(FftBuf<C, MODE>{dst}, base + (j - k) * R + k);
 #pragma unroll
-            for (int q = 0; q < R; ++q) {
-                const int xo = idxD + q * NS;
-                dst[SWZ ? swz<C>(xo) : xo] = v[q];
-            }
+            for (int q = 0; q < R; ++q) out(q, v[q]);
         }
     }
 }
 
-template <typename C, int N, int F, int S, int NQ, bool SWZ, int TWS, bool END>
+template <typename C, int N, int F, int S, int NQ, int MODE, int TWS, bool END>
 struct Step;
-template <typename C, int N, int F, int S, int NQ, bool SWZ, int TWS>
-struct Step<C, N, F, S, NQ, SWZ, TWS, true> {
+template <typename C, int N, int F, int S, int NQ, int MODE, int TWS>
+struct Step<C, N, F, S, NQ, MODE, TWS, true> {
     static __device__ __forceinline__ C *go(C *src, C *, const C *, int) { return src; }
 };
-template <typename C, int N, int F, int S, int NQ, bool SWZ, int TWS>
-struct Step<C, N, F, S, NQ, SWZ, TWS, false> {
+template <typename C, int N, int F, int S, int NQ, int MODE, int TWS>
+struct Step<C, N, F, S, NQ, MODE, TWS, false> {
     static __device__ __forceinline__ C *go(C *src, C *dst, const C *tw, int lane) {
-        stage<C, N, F, S, NQ, SWZ, TWS>(src, dst, tw, lane);
+        stage<C, N, F, S, NQ, MODE, TWS>(src, dst, tw, lane);
         __syncwarp();
-        return Step<C, N, F + 1, S, NQ, SWZ, TWS, (F + 1 >= nfac(N))>::go(dst, src, tw, lane);
+        return Step<C, N, F + 1, S, NQ, MODE, TWS, (F + 1 >= nfac(N))>::go(dst, src, tw, lane);
     }
 };
 
 // stage F of one sequence with its inputs from ld(x) and its outputs to st(x, value): the same
 // butterflies, twiddles and operation order as stage()
 template <typename C, int N, int F, int S, int TWS, typename LD, typename ST>
-__device__ __forceinline__ void stage_io(LD &ld, ST &st, const C *__restrict__ tw, int lane) {
+__device__ __forceinline__ void stage_io(LD &&ld, ST &&st, const C *__restrict__ tw, int lane) {
+    typedef typename std::remove_reference<LD>::type L;
+    typedef typename std::remove_reference<ST>::type T;
     constexpr int R = fac(N, F);
     constexpr int NS = stride(N, F);
     constexpr int NR = N / R;
@@ -266,9 +329,10 @@ __device__ __forceinline__ void stage_io(LD &ld, ST &st, const C *__restrict__ t
         if (NR % 32 == 0 || j < NR) {
             const int k = j % NS;
             C v[R];
+            const Src<C, NR, L> in(ld, j);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                C x = ld(j + r * NR);
+                C x = in(r);
                 if (NS > 1 && r > 0 && k) {
                     C w = __ldg(&tw[TW0 + (r - 1) * NS + k]);
                     if (S > 0) w.y = -w.y;
@@ -277,14 +341,14 @@ __device__ __forceinline__ void stage_io(LD &ld, ST &st, const C *__restrict__ t
                 v[r] = x;
             }
             Dft<C, R, S>::run(v);
-            const int idxD = (j - k) * R + k;
+            const Dst<C, R, NS, T> out(st, (j - k) * R + k);
 #pragma unroll
-            for (int q = 0; q < R; ++q) st(idxD + q * NS, v[q]);
+            for (int q = 0; q < R; ++q) out(q, v[q]);
         }
     }
 }
 
-// stage F of one sequence in place in the swizzled buffer x: every lane reads and transforms all
+// stage F of one sequence in place in the buffer x (FMODE layout): every lane reads and transforms all
 // its butterflies' inputs before the warp writes any output (the same arithmetic as stage())
 template <typename C, int N, int F, int S, int TWS>
 __device__ __forceinline__ void stage_ip(C *x, const C *__restrict__ tw, int lane) {
@@ -299,9 +363,10 @@ __device__ __forceinline__ void stage_ip(C *x, const C *__restrict__ tw, int lan
         const int j = lane + 32 * it;
         if (NR % 32 == 0 || j < NR) {
             const int k = j % NS;
+            const Src<C, NR, const FftBuf<C>> in(FftBuf<C>{x}, j);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                C u = x[swz<C>(j + r * NR)];
+                C u = in(r);
                 if (NS > 1 && r > 0 && k) {
                     C w = __ldg(&tw[TW0 + (r - 1) * NS + k]);
                     if (S > 0) w.y = -w.y;
@@ -318,9 +383,9 @@ __device__ __forceinline__ void stage_ip(C *x, const C *__restrict__ tw, int lan
         const int j = lane + 32 * it;
         if (NR % 32 == 0 || j < NR) {
             const int k = j % NS;
-            const int idxD = (j - k) * R + k;
+            const Dst<C, R, NS, const FftBuf<C>> out(FftBuf<C>{x}, (j - k) * R + k);
 #pragma unroll
-            for (int q = 0; q < R; ++q) x[swz<C>(idxD + q * NS)] = v[it][q];
+            for (int q = 0; q < R; ++q) out(q, v[it][q]);
         }
     }
     __syncwarp();
@@ -340,20 +405,20 @@ struct IpSteps<C, N, F, S, TWS, false> {
     }
 };
 
-// the stages between the first and the last, ping-ponging between two swizzled buffers; returns
+// the stages between the first and the last, ping-ponging between two buffers; returns
 // the buffer holding the output of the last of them
-template <typename C, int N, int F, int S, int TWS, bool END>
+template <typename C, int N, int F, int S, int TWS, int MODE, bool END>
 struct MidSteps;
-template <typename C, int N, int F, int S, int TWS>
-struct MidSteps<C, N, F, S, TWS, true> {
+template <typename C, int N, int F, int S, int TWS, int MODE>
+struct MidSteps<C, N, F, S, TWS, MODE, true> {
     static __device__ __forceinline__ C *go(C *src, C *, const C *, int) { return src; }
 };
-template <typename C, int N, int F, int S, int TWS>
-struct MidSteps<C, N, F, S, TWS, false> {
+template <typename C, int N, int F, int S, int TWS, int MODE>
+struct MidSteps<C, N, F, S, TWS, MODE, false> {
     static __device__ __forceinline__ C *go(C *src, C *dst, const C *tw, int lane) {
-        stage<C, N, F, S, 1, true, TWS>(src, dst, tw, lane);
+        stage<C, N, F, S, 1, MODE, TWS>(src, dst, tw, lane);
         __syncwarp();
-        return MidSteps<C, N, F + 1, S, TWS, (F + 2 >= nfac(N))>::go(dst, src, tw, lane);
+        return MidSteps<C, N, F + 1, S, TWS, MODE, (F + 2 >= nfac(N))>::go(dst, src, tw, lane);
     }
 };
 }   // namespace kct
@@ -361,50 +426,50 @@ struct MidSteps<C, N, F, S, TWS, false> {
 // S = -1: exp(-2 pi i jk/N) (FFTW_FORWARD), +1: exp(+...) (FFTW_BACKWARD).  NQ sequences of
 // length N lie N apart in a; b is a scratch buffer of the same size (both private to the calling
 // warp); the input must be visible to the whole warp (__syncwarp after writing it).  Returns the
-// buffer holding the result.  SWZ: the buffers are swizzled (element x at swz<C>(x)).  TWS (1 or 2): the
+// buffer holding the result.  Element x of a buffer is at fpos<C, MODE>(x).  TWS (1 or 2): the
 // table is that of length TWS N.
-template <typename C, int N, int S, int NQ = 1, bool SWZ = false, int TWS = 1>
+template <typename C, int N, int S, int NQ = 1, int MODE = 0, int TWS = 1>
 __device__ __forceinline__ C *fft_warp_ct(C *a, C *b, const C *tw) {
     static_assert(kct::nfac(N) > 0, "transform length must be 2^a 3^b 5^c");
-    return kct::Step<C, N, 0, S, NQ, SWZ, TWS, false>::go(a, b, tw, threadIdx.x & 31);
+    return kct::Step<C, N, 0, S, NQ, MODE, TWS, false>::go(a, b, tw, threadIdx.x & 31);
 }
 
 // fft_warp_ct of one sequence whose first stage reads its input through ld(x) (element x of the
 // sequence) and whose last stage writes its output through st(x, value), natural order, so that
-// neither needs a copy pass through shared memory; the stages in between use the swizzled
-// buffers a and b (private to the warp).  pre() runs between the second-last and the last stage
+// neither needs a copy pass through shared memory; the stages in between use the buffers a and b
+// (private to the warp).  pre() runs between the second-last and the last stage
 // in every thread of the warp (a block-wide barrier there must be reached by every warp).  Same
 // arithmetic as fft_warp_ct.  The last stage reads buffer a when nfac(N) is even, else b; st may
 // write the other one.
-template <typename C, int N, int S, int TWS = 1, typename LD, typename ST, typename PRE>
-__device__ __forceinline__ void fft_warp_ct_io(LD ld, ST st, PRE pre, C *a, C *b, const C *tw) {
+template <typename C, int N, int S, int TWS = 1, int MODE = FMODE<C>, typename LD, typename ST, typename PRE>
+__device__ __forceinline__ void fft_warp_ct_io(const LD ld, const ST st, PRE pre, C *a, C *b, const C *tw) {
     constexpr int L = kct::nfac(N);
     static_assert(L >= 2, "fft_warp_ct_io needs at least two stages");
     const int lane = threadIdx.x & 31;
-    auto to_a = [&](int x, C v) { a[swz<C>(x)] = v; };
+    const FftBuf<C, MODE> to_a{a};
     kct::stage_io<C, N, 0, S, TWS>(ld, to_a, tw, lane);
     __syncwarp();
-    const C *src = kct::MidSteps<C, N, 1, S, TWS, (2 >= L)>::go(a, b, tw, lane);
+    C *src = kct::MidSteps<C, N, 1, S, TWS, MODE, (2 >= L)>::go(a, b, tw, lane);
     pre();
-    auto from_src = [&](int x) { return src[swz<C>(x)]; };
+    const FftBuf<C, MODE> from_src{src};
     kct::stage_io<C, N, L - 1, S, TWS>(from_src, st, tw, lane);
 }
 
-// fft_warp_ct of one sequence held in one swizzled buffer a (the input visible to the whole warp):
+// fft_warp_ct of one sequence held in one buffer a (FMODE layout) (the input visible to the whole warp):
 // every stage but the last runs in place (stage_ip), and the last reads a and writes its output
-// through st(x, value), so a warp needs one buffer of N elements instead of two.  Same arithmetic
+// through st(x, value), so a warp needs one buffer instead of two.  Same arithmetic
 // as fft_warp_ct.
 template <typename C, int N, int S, int TWS = 1, typename ST>
-__device__ __forceinline__ void fft_warp_ct_ip(C *a, ST st, const C *tw) {
+__device__ __forceinline__ void fft_warp_ct_ip(C *a, const ST st, const C *tw) {
     constexpr int L = kct::nfac(N);
     static_assert(L >= 1, "transform length must be 2^a 3^b 5^c");
     const int lane = threadIdx.x & 31;
     kct::IpSteps<C, N, 0, S, TWS, (1 >= L)>::go(a, tw, lane);
-    auto from_a = [&](int x) { return a[swz<C>(x)]; };
+    const FftBuf<C> from_a{a};
     kct::stage_io<C, N, L - 1, S, TWS>(from_a, st, tw, lane);
 }
 
-// the same with every stage in place: the result is left in a (natural order, swizzled)
+// the same with every stage in place: the result is left in a (natural order)
 template <typename C, int N, int S, int TWS = 1>
 __device__ __forceinline__ void fft_warp_ct_inplace(C *a, const C *tw) {
     constexpr int L = kct::nfac(N);

@@ -904,8 +904,8 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb2(const C *__restrict__ yp,
     const bool act = kx < nxh && y < nyp;
     const int ldc = col_ld<C>(nyp);
     const size_t fs = (size_t)NZ * nxh * ldc;   // field stride of the column layout
-    C *a = sm + (size_t)warp * 2 * MZ, *b = a + MZ;
-    C *stage = sm + (size_t)ZT_WARPS * 2 * MZ;   // [y][z][kx] tile for the store
+    C *a = sm + (size_t)warp * 2 * flen<C>(MZ), *b = a + flen<C>(MZ);
+    C *stage = sm + (size_t)ZT_WARPS * 2 * flen<C>(MZ);   // [y][z][kx] tile for the store
     const T kxv = act ? (T)wavx[kx] : (T)0;
     const C zc = kct::mk<C>((T)0, (T)0);
     C pf[NE];
@@ -946,18 +946,18 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb2(const C *__restrict__ yp,
     fetch(0);
     for (int g = 0; g < nout; ++g) {
         if (act) {
-            for (int z = NZH + lane; z < MZ - NZH; z += 32) a[swz<C>(z)] = zc;   // padding modes
+            for (int z = NZH + lane; z < MZ - NZH; z += 32) a[fpos<C>(z)] = zc;   // padding modes
 #pragma unroll
             for (int e = 0; e < NE; ++e) {
                 const int kz = lane + 32 * e;
-                if (kz < NZ) a[swz<C>(kz < NZH ? kz : (MZ - NZ) + kz)] = pf[e];
+                if (kz < NZ) a[fpos<C>(kz < NZH ? kz : (MZ - NZ) + kz)] = pf[e];
             }
             __syncwarp();
         }
         if (g + 1 < nout) fetch(g + 1);
         if (act) {
-            const C *r = fft_warp_ct<C, MZ, +1, 1, true>(a, b, tw);
-            for (int z = lane; z < MZ; z += 32) stage[((size_t)yl * MZ + z) * ZT_KX + kl] = r[swz<C>(z)];
+            const C *r = fft_warp_ct<C, MZ, +1, 1, FMODE<C>>(a, b, tw);
+            for (int z = lane; z < MZ; z += 32) stage[((size_t)yl * MZ + z) * ZT_KX + kl] = r[fpos<C>(z)];
         }
         __syncthreads();
         // store rows of ZT_KX consecutive kx
@@ -984,8 +984,8 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zf2(const C *__restrict__ r, 
     const int kx = blockIdx.x * ZT_KX + kl, y = blockIdx.y * ZT_Y + yl;
     const bool act = kx < nxh && y < nyp;
     const size_t ncols = (size_t)NZ * nxh;
-    C *a = sm + (size_t)warp * 2 * MZ, *b = a + MZ;
-    C *stage = sm + (size_t)ZT_WARPS * 2 * MZ;   // [kx][kz][y] tile for the store
+    C *a = sm + (size_t)warp * 2 * flen<C>(MZ), *b = a + flen<C>(MZ);
+    C *stage = sm + (size_t)ZT_WARPS * 2 * flen<C>(MZ);   // [kx][kz][y] tile for the store
     const T rs = (T)(1.0 / scale);
     C pf[NE];
     auto fetch = [&](int o) {
@@ -1001,15 +1001,15 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zf2(const C *__restrict__ r, 
 #pragma unroll
             for (int e = 0; e < NE; ++e) {
                 const int z = lane + 32 * e;
-                if (z < MZ) a[swz<C>(z)] = pf[e];
+                if (z < MZ) a[fpos<C>(z)] = pf[e];
             }
             __syncwarp();
         }
         if (o + 1 < nout) fetch(o + 1);
         if (act) {
-            const C *res = fft_warp_ct<C, MZ, -1, 1, true>(a, b, tw);
+            const C *res = fft_warp_ct<C, MZ, -1, 1, FMODE<C>>(a, b, tw);
             for (int kz = lane; kz < NZ; kz += 32) {
-                const C v = res[swz<C>(kz < NZH ? kz : (MZ - NZ) + kz)];
+                const C v = res[fpos<C>(kz < NZH ? kz : (MZ - NZ) + kz)];
                 // FP64 divides by mx mz as the reference normalises; FP32 multiplies by the reciprocal
                 stage[((size_t)kl * NZ + kz) * ZT_Y + yl] =
                     sizeof(T) == 8 ? kct::mk<C>((T)(v.x / scale), (T)(v.y / scale)) : kct::mk<C>(v.x * rs, v.y * rs);
@@ -1388,8 +1388,9 @@ static int fused_launch(kmm_ctx *ctx) {
     if (scalar) { ctx->f[KMM_SCNM1] = sn_old; ctx->f[KMM_SCN] = snm1_old; }
 
     // z inverse transforms
-    const size_t smz = sizeof(double2) * ((size_t)ZT_WARPS * 2 * mz + (size_t)ZT_Y * mz * ZT_KX);
-    const size_t smzf = sizeof(double2) * ((size_t)ZT_WARPS * 2 * mz + (size_t)ZT_KX * nz * ZT_Y);
+    const size_t zbuf = (size_t)ZT_WARPS * 2 * (ct_mz ? flen<double2>(mz) : mz);   // the warps' FFT buffers
+    const size_t smz = sizeof(double2) * (zbuf + (size_t)ZT_Y * mz * ZT_KX);
+    const size_t smzf = sizeof(double2) * (zbuf + (size_t)ZT_KX * nz * ZT_Y);
     const dim3 gz((nxh + ZT_KX - 1) / ZT_KX, (nyp + ZT_Y - 1) / ZT_Y);
     kmm_tic(ctx);
 #define ZB2(MM, CC)                                                                                   \

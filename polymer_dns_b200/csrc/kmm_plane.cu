@@ -30,7 +30,7 @@ struct FieldPtrs { const double2 *p[MAXIO]; };
 struct FieldPtrsW { double2 *p[MAXIO]; };
 
 // Block FFT buffers.  At the compiled lengths each of the 8 warps owns NQ = NB / 8 consecutive
-// sequences, stored swizzled (swz<C>, kmm_fft.cuh) within the warp's region, and the warps'
+// sequences, stored conflict-free (fpos<C>, kmm_fft.cuh) within the warp's region, and the warps'
 // regions lie FB_PAD elements further apart than NQ n: the radix stages then run free of bank
 // conflicts, and so do the transposing loads and stores around the transform, whose 8 (or 16)
 // concurrent sequences would otherwise sit n apart on the same banks.  The runtime FFT of the
@@ -38,11 +38,11 @@ struct FieldPtrsW { double2 *p[MAXIO]; };
 #define FB_PAD 1
 
 // elements of one buffer (a or b) of NB sequences of length n
-__host__ __device__ constexpr int fb_len(int nb, int n) { return nb * n + 8 * FB_PAD; }
-
-__device__ __forceinline__ bool fb_compiled(int n) {
+// (at the compiled lengths the padded layout's, which also holds the FP32 forms')
+__host__ __device__ constexpr bool fb_compiled(int n) {
     return n == 48 || n == 64 || n == 96 || n == 128 || n == 144 || n == 192 || n == 256 || n == 576;
 }
+__host__ __device__ constexpr int fb_len(int nb, int n) { return nb * (fb_compiled(n) ? n + n / 8 : n) + 8 * FB_PAD; }
 
 // position of element i of sequence c (ct: n is a compiled length)
 template <typename C, int NB>
@@ -50,7 +50,7 @@ __device__ __forceinline__ int fb_at(int c, int i, int n, bool ct) {
     constexpr int NQ = NB / 8;
     if (!ct) return c * n + i;
     const int wq = c / NQ, q = c - wq * NQ;
-    return wq * (NQ * n + FB_PAD) + swz<C>(q * n + i);
+    return wq * (flen<C>(NQ * n) + FB_PAD) + fpos<C>(q * n + i);
 }
 
 // batched FFT of NB sequences of length N (layout of fb_at) by the block's 8 warps, NB / 8
@@ -60,9 +60,9 @@ template <typename C, int N, int S, int NB>
 __device__ __forceinline__ C *fft_block_ct(C *a, C *b, const C *tw) {
     constexpr int NQ = NB / 8;
     static_assert(NB % 8 == 0, "8 warps share the sequences");
-    static_assert(N % (sizeof(C) == 16 ? 8 : 16) == 0, "swizzle rows of 128 bytes");
-    const size_t w = (size_t)(threadIdx.x >> 5) * (NQ * N + FB_PAD);
-    C *r = fft_warp_ct<C, N, S, NQ, true>(a + w, b + w, tw);
+    static_assert(N % (sizeof(C) == 16 ? 8 : 16) == 0, "padding, or swizzle rows, of 128 bytes");
+    const size_t w = (size_t)(threadIdx.x >> 5) * (flen<C>(NQ * N) + FB_PAD);
+    C *r = fft_warp_ct<C, N, S, NQ, FMODE<C>>(a + w, b + w, tw);
     __syncthreads();
     return r - w;
 }
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(256) k_dct_fwd(const __grid_constant__ FieldPt
 //   X_1 = x_0 - x_N + 2 sum_{n=1}^{N-1} x_n cos(pi n / N)
 // (the half-length form of the DCT-I; the real and imaginary parts of the column are two real
 // sequences, carried together).  x: the column's N + 1 values in shared memory, overwritten by X;
-// a, b: the warp's FFT buffers (N elements, swizzled); tw: the 2N-point twiddles exp(-i pi m / N).
+// a, b: the warp's FFT buffers (flen<C>(N) elements); tw: the 2N-point twiddles exp(-i pi m / N).
 template <typename C, int N>
 __device__ __forceinline__ void dct1_half(C *x, C *a, C *b, const C *__restrict__ tw) {
     typedef typename kct::Real<C>::T T;
@@ -156,7 +156,7 @@ __device__ __forceinline__ void dct1_half(C *x, C *a, C *b, const C *__restrict_
         const C w = tw[j];   // (cos, -sin) of pi j / N
         const C sm = kct::add(xj, xr), df = kct::sub(xj, xr);
         const T sn = -w.y;
-        a[swz<C>(j)] = kct::mk<C>((T)0.5 * sm.x + sn * df.x, (T)0.5 * sm.y + sn * df.y);
+        a[fpos<C>(j)] = kct::mk<C>((T)0.5 * sm.x + sn * df.x, (T)0.5 * sm.y + sn * df.y);
         seed = j == 0 ? kct::add(seed, df) : kct::add(seed, kct::scl(xj, (T)2 * w.x));
     }
 #pragma unroll
@@ -169,7 +169,7 @@ __device__ __forceinline__ void dct1_half(C *x, C *a, C *b, const C *__restrict_
         fft_warp_ct_inplace<C, N, -1, 2>(a, tw);
         Y = a;
     } else {
-        Y = fft_warp_ct<C, N, -1, 1, true, 2>(a, b, tw);
+        Y = fft_warp_ct<C, N, -1, 1, FMODE<C>, 2>(a, b, tw);
     }
     // odd outputs: X_{2m+1} = seed + sum_{t=1}^{m} d_t, d_t = -i (Y_t - Y_{N-t}); lane holds m = lane Q .. lane Q + Q - 1
     C d[Q];
@@ -179,7 +179,7 @@ __device__ __forceinline__ void dct1_half(C *x, C *a, C *b, const C *__restrict_
         const int m = lane * Q + q;
         C v = kct::mk<C>((T)0, (T)0);
         if (m >= 1 && m < H) {
-            const C df = kct::sub(Y[swz<C>(m)], Y[swz<C>(N - m)]);
+            const C df = kct::sub(Y[fpos<C>(m)], Y[fpos<C>(N - m)]);
             v = kct::mk<C>(df.y, -df.x);
         }
         tot = kct::add(tot, v);
@@ -197,7 +197,7 @@ __device__ __forceinline__ void dct1_half(C *x, C *a, C *b, const C *__restrict_
 #pragma unroll
     for (int e = 0; e < (H + 1 + 31) / 32; ++e) {
         const int m = lane + 32 * e;
-        if (m <= H) ev[e] = kct::add(Y[swz<C>(m)], Y[swz<C>(m == 0 ? 0 : N - m)]);
+        if (m <= H) ev[e] = kct::add(Y[fpos<C>(m)], Y[fpos<C>(m == 0 ? 0 : N - m)]);
     }
     __syncwarp();
 #pragma unroll
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(256) k_dct_fwd_h(const __grid_constant__ Field
     }
     __syncthreads();
     const int c = threadIdx.x >> 5;
-    if (c < ncb) dct1_half<C, N>(xs + c * NYP, a + c * (N + FB_PAD), b + c * (N + FB_PAD), tw);
+    if (c < ncb) dct1_half<C, N>(xs + c * NYP, a + c * (flen<C>(N) + FB_PAD), b + c * (flen<C>(N) + FB_PAD), tw);
     __syncthreads();
     // PL[f][y][kx][kz]: col = kx*nz + kz
     for (int e = threadIdx.x; e < ncb * NYP; e += blockDim.x) {
@@ -286,7 +286,7 @@ __device__ __forceinline__ C *zbwd_io(const C *__restrict__ src, C *a, C *b, con
     C *res = kct::nfac(N) % 2 == 1 ? a : b;
     const int c = threadIdx.x >> 5;
     if (c < nk) {
-        const size_t w = (size_t)c * (N + FB_PAD);
+        const size_t w = (size_t)c * (flen<C>(N) + FB_PAD);
         const C *col = src + (size_t)c * nz;
         const int nzh = nz / 2, hi = N - nz + nzh;
         auto ld = [&](int z) {
@@ -301,7 +301,7 @@ __device__ __forceinline__ C *zbwd_io(const C *__restrict__ src, C *a, C *b, con
             }
             return v;
         };
-        auto st = [&](int x, C v) { res[w + swz<C>(x)] = v; };
+        const FftBuf<C> st{res + w};
         auto pre = [] {};
         fft_warp_ct_io<C, N, +1>(ld, st, pre, a + w, b + w, tw);
     }
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 4) k_zfft_bwd(const C *__restri
         __syncthreads();
         if constexpr (BIG) {
             const int w = threadIdx.x >> 5;
-            if (w < nk) fft_warp_ct_inplace<C, 576, +1>(a + (size_t)w * (576 + FB_PAD), tw);
+            if (w < nk) fft_warp_ct_inplace<C, 576, +1>(a + (size_t)w * (flen<C>(576) + FB_PAD), tw);
             __syncthreads();
             r = a;
         } else {
@@ -639,13 +639,13 @@ __global__ void __launch_bounds__(XBW * 32, sizeof(C) == 16 ? 4 : 6) k_xinv_big2
     if (z >= mz) return;   // whole warps: no block barrier below
     // FP64: one buffer per warp, the FFT in place; FP32: two (its registers allow six blocks per SM)
     constexpr int NBUF = sizeof(C) == 16 ? 1 : 2;
-    C *a = reinterpret_cast<C *>(smd) + (size_t)warp * NBUF * MX;
+    C *a = reinterpret_cast<C *>(smd) + (size_t)warp * NBUF * flen<C>(MX);
     const int pr = blockIdx.z;
     const bool xd = X.xd[pr];
     const C *qa = q + (((size_t)X.qa[pr] * nyp + y) * mz + z) * NXH;
     const C *qb = q + (((size_t)((g >= 0 && !xd) ? X.qb[pr] : X.qa[pr]) * nyp + y) * mz + z) * NXH;
     const C zc = kct::mk<C>((T)0, (T)0);
-    for (int k = NXH + lane; k <= MX - NXH; k += 32) a[swz<C>(k)] = zc;
+    for (int k = NXH + lane; k <= MX - NXH; k += 32) a[fpos<C>(k)] = zc;
     for (int kk = lane; kk < NXH; kk += 32) {
         C A_ = qa[kk], B_ = g >= 0 ? qb[kk] : zc;
         if (xd) {   // the pair's second input is i kx times the first
@@ -653,8 +653,8 @@ __global__ void __launch_bounds__(XBW * 32, sizeof(C) == 16 ? 4 : 6) k_xinv_big2
             B_ = kct::mk<C>(-kx * A_.y, kx * A_.x);
         }
         if (kk == 0) { A_.y = (T)0; B_.y = (T)0; }   // c2r ignores Im of the mean mode
-        a[swz<C>(kk)] = kct::mk<C>(A_.x - B_.y, A_.y + B_.x);
-        if (kk > 0) a[swz<C>(MX - kk)] = kct::mk<C>(A_.x + B_.y, -A_.y + B_.x);
+        a[fpos<C>(kk)] = kct::mk<C>(A_.x - B_.y, A_.y + B_.x);
+        if (kk > 0) a[fpos<C>(MX - kk)] = kct::mk<C>(A_.x + B_.y, -A_.y + B_.x);
     }
     __syncwarp();
     const size_t nphys = (size_t)nyp * mz * MX, g3 = ((size_t)y * mz + z) * MX;
@@ -668,9 +668,9 @@ __global__ void __launch_bounds__(XBW * 32, sizeof(C) == 16 ? 4 : 6) k_xinv_big2
     if constexpr (NBUF == 1) {
         fft_warp_ct_ip<C, MX, +1>(a, st, tw);
     } else {
-        auto ld = [&](int x) { return a[swz<C>(x)]; };
+        const FftBuf<C> ld{a};
         auto pre = [] {};
-        fft_warp_ct_io<C, MX, +1>(ld, st, pre, a + MX, a, tw);
+        fft_warp_ct_io<C, MX, +1>(ld, st, pre, a + flen<C>(MX), a, tw);
     }
 }
 
@@ -808,15 +808,15 @@ __global__ void __launch_bounds__(XpW<C>::n * 32) k_xphys2(const C *__restrict__
             // buffer), the second reads them back into a, and the last reads a and writes the
             // two real rows straight into the rows it no longer needs
             T *pf = phys + (size_t)f * MX, *pg = phys + (size_t)(g >= 0 ? g : f) * MX;
-            auto ld = [&](int x) { return a[swz<C>(x)]; };
+            const FftBuf<C, 1> ld{a};   // swizzled: the pair's rows hold MX values, no padding
             auto st = [&](int x, C v) {
                 pf[x] = v.x;
                 if (g >= 0) pg[x] = v.y;
             };
             auto pre = [] {};
-            fft_warp_ct_io<C, MX, +1>(ld, st, pre, b, a, tw);
+            fft_warp_ct_io<C, MX, +1, 1, 1>(ld, st, pre, b, a, tw);
         } else {
-            const C *r = fft_warp_ct<C, MX, +1, 1, true>(a, b, tw);
+            const C *r = fft_warp_ct<C, MX, +1, 1, 1>(a, b, tw);
             // the result may sit in the pair's own rows: read it all before writing the real rows
             constexpr int E = (MX + 31) / 32;
             C rv[E];
@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(XW * 32) k_xfwd2(const typename kct::Real<C>::
     C *sm = reinterpret_cast<C *>(smd);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int z = blockIdx.x, y = blockIdx.y;
-    C *a = sm + (size_t)warp * 2 * MX, *b = a + MX;
+    C *a = sm + (size_t)warp * 2 * flen<C>(MX), *b = a + flen<C>(MX);
     const size_t n3 = (size_t)nyp * mz * MX, g3 = ((size_t)y * mz + z) * MX;
     for (int pr = warp; pr < (nout + 1) / 2; pr += XW) {
         const int o = 2 * pr, g = o + 1 < nout ? o + 1 : -1;
@@ -888,13 +888,13 @@ __global__ void __launch_bounds__(XW * 32) k_xfwd2(const typename kct::Real<C>::
         const T *ro = po + (size_t)o * n3 + g3, *rg = po + (size_t)(g >= 0 ? g : o) * n3 + g3;
         auto ld = [&](int x) { return kct::mk<C>(ro[x], g >= 0 ? rg[x] : (T)0); };
         C *r = kct::nfac(MX) % 2 == 0 ? b : a;
-        auto st = [&](int x, C v) { r[swz<C>(x)] = v; };
+        const FftBuf<C> st{r};
         auto pre = [] {};
         fft_warp_ct_io<C, MX, -1>(ld, st, pre, a, b, tw);
         __syncwarp();
         for (int k = lane; k < NXH; k += 32) {
-            const C Z = r[swz<C>(k)];
-            C Zc = r[swz<C>(k == 0 ? 0 : MX - k)];
+            const C Z = r[fpos<C>(k)];
+            C Zc = r[fpos<C>(k == 0 ? 0 : MX - k)];
             Zc.y = -Zc.y;
             q[(((size_t)o * nyp + y) * mz + z) * NXH + k] = kct::mk<C>((T)0.5 * (Z.x + Zc.x), (T)0.5 * (Z.y + Zc.y));
             if (g >= 0)   // -i/2 (Z - Zc)
@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 4) k_zfft_fwd(const C *__restri
     C *r;
     if constexpr (BIG) {
         const int w = threadIdx.x >> 5;
-        if (w < nk) fft_warp_ct_inplace<C, 576, -1>(a + (size_t)w * (576 + FB_PAD), tw);
+        if (w < nk) fft_warp_ct_inplace<C, 576, -1>(a + (size_t)w * (flen<C>(576) + FB_PAD), tw);
         __syncthreads();
         r = a;
     } else {
@@ -1127,7 +1127,7 @@ __global__ void __launch_bounds__(256) k_dct_bwd_h(const C *__restrict__ pl, con
     }
     __syncthreads();
     const int c = threadIdx.x >> 5;
-    if (c < ncb) dct1_half<C, N>(xs + c * NYP, a + c * (N + FB_PAD), b + c * (N + FB_PAD), tw);
+    if (c < ncb) dct1_half<C, N>(xs + c * NYP, a + c * (flen<C>(N) + FB_PAD), b + c * (flen<C>(N) + FB_PAD), tw);
     __syncthreads();
     double2 *dst = out.p[f] + (size_t)col0 * NYP;
     for (int e = threadIdx.x; e < ncb * NYP; e += blockDim.x) {
@@ -1672,7 +1672,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
                     ctx->d_cfl, ctx->d_umax, ctx->pmx, A, sv, nyp, mz, mx, nxh);
             } else {
                 const dim3 g1((mz + XBW - 1) / XBW, nyp, (nin + 1) / 2);
-                const size_t sm_b2 = 2 * eb * (f32 ? 2 : 1) * XBW * (size_t)mx;   // complex rows per warp
+                const size_t sm_b2 = 2 * eb * XBW * (size_t)(f32 ? 2 * flen<float2>(mx) : flen<double2>(mx));   // complex rows per warp
                 if (mx == 576 && f32) {
                     RET(kmm_smem_attr(ctx, (const void *)k_xinv_big2<576, float2>, sm_b2));
                     k_xinv_big2<576, float2><<<g1, XBW * 32, sm_b2, ctx->stream>>>(q_in32, (float *)ctx->xbig, tw_mx,
@@ -1725,7 +1725,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
         }
         kmm_toc(ctx, KMM_STAGE_XPHYS);   // the spreading counts with the pointwise stage
         kmm_tic(ctx);
-        const size_t sm_xf2 = 2 * eb * 2 * XW * (size_t)mx;
+        const size_t sm_xf2 = 2 * eb * 2 * XW * (size_t)(f32 ? flen<float2>(mx) : flen<double2>(mx));
 #define XF2(MM, CC, PO, QQ, TW)                                                                                 \
     do {                                                                                                        \
         RET(kmm_smem_attr(ctx, (const void *)k_xfwd2<MM, CC>, sm_xf2));                                         \

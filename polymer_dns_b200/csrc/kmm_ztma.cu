@@ -92,22 +92,21 @@ template <int MZ, typename C, int S, typename LD, typename OUT, typename BEFORE>
 __device__ __forceinline__ void z_column(LD ld, OUT out, BEFORE before, C *a, const C *__restrict__ tw) {
     constexpr int L = kct::nfac(MZ);
     const int lane = threadIdx.x & 31;
-    auto to_a = [&](int x, C v) { a[swz<C>(x)] = v; };
-    kct::stage_io<C, MZ, 0, S, 1>(ld, to_a, tw, lane);
+    const FftBuf<C> buf{a};
+    kct::stage_io<C, MZ, 0, S, 1>(ld, buf, tw, lane);
     __syncwarp();
     kct::IpSteps<C, MZ, 1, S, 1, (2 >= L)>::go(a, tw, lane);
-    auto from_a = [&](int x) { return a[swz<C>(x)]; };
     if constexpr (ZREG<MZ>) {
         C rv[MZ / 32];
         auto st = [&](int z, C v) { rv[z >> 5] = v; };
-        kct::stage_io<C, MZ, L - 1, S, 1>(from_a, st, tw, lane);
+        kct::stage_io<C, MZ, L - 1, S, 1>(buf, st, tw, lane);
         before();
 #pragma unroll
         for (int e = 0; e < MZ / 32; ++e) out(lane + 32 * e, rv[e]);
     } else {
         kct::stage_ip<C, MZ, L - 1, S, 1>(a, tw, lane);
         before();
-        for (int z = lane; z < MZ; z += 32) out(z, from_a(z));
+        for (int z = lane; z < MZ; z += 32) out(z, a[fpos<C>(z)]);
     }
 }
 
@@ -135,7 +134,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
     C *tiles = reinterpret_cast<C *>((reinterpret_cast<uintptr_t>(zsm_raw) + 1023) & ~(uintptr_t)1023);
     C *stage = tiles + (size_t)ZB_SLOTS * TILE;
     C *scr = stage + (size_t)W * MZ;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(scr + (size_t)W * MZ);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(scr + (size_t)W * flen<C>(MZ));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kx0 = blockIdx.x * KX, y0 = blockIdx.y * YT;
     const int kl = warp / YT, y = warp % YT;
@@ -153,7 +152,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
     }
     const T kxv = kx0 + kl < nxh ? (T)wavx[kx0 + kl] : (T)0;
     const double beta = wavz[1];
-    C *a = scr + (size_t)warp * MZ;
+    C *a = scr + (size_t)warp * flen<C>(MZ);
     bool ok = true;
     const C zc = kct::mk<C>((T)0, (T)0);
     for (int k = 0; k < ZB_SLOTS; ++k) {
@@ -218,7 +217,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
     C *tiles = reinterpret_cast<C *>((reinterpret_cast<uintptr_t>(zsm_raw) + 1023) & ~(uintptr_t)1023);
     C *stage = tiles + (size_t)ZF_SLOTS * TIN;
     C *scr = stage + TOUT;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(scr + (size_t)W * MZ);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(scr + (size_t)W * flen<C>(MZ));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kx0 = blockIdx.x * KX, y0 = blockIdx.y * YT;
     const int kl = warp / YT, y = warp % YT;
@@ -241,7 +240,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
     }
     const T rs = (T)(1.0 / scale);
     const C zc = kct::mk<C>((T)0, (T)0);
-    C *a = scr + (size_t)warp * MZ;
+    C *a = scr + (size_t)warp * flen<C>(MZ);
     bool ok = true;
     for (int o = 0; o < nper; ++o) {
         ok = mbar_wait(&bar[o], 0) && ok;
@@ -406,7 +405,7 @@ static int zb_launch(kmm_ctx *ctx, const C *yp, C *q, int nbase, int nq, const C
     ZtmaMaps *M = ztma_maps(ctx);
     if (!M) return KMM_ERR_NOMEM;
     RET(pair_encode(ctx, M->inv, true, yp, q, nbase, nq, f32, KX, YT));
-    const size_t smem = 1024 + sizeof(C) * W * ((size_t)ZB_SLOTS * NZ + 2 * MZ) + 8 * sizeof(uint64_t);
+    const size_t smem = 1024 + sizeof(C) * W * ((size_t)ZB_SLOTS * NZ + MZ + flen<C>(MZ)) + 8 * sizeof(uint64_t);
     const dim3 grid((ctx->nxh + KX - 1) / KX, (ctx->nyp + YT - 1) / YT, nq / ZB_SLOTS);
     RET(kmm_smem_attr(ctx, (const void *)k_zb_tma<MZ, C, KX, YT, MINB>, smem));
     k_zb_tma<MZ, C, KX, YT, MINB><<<grid, W * 32, smem, ctx->stream>>>(M->inv.in, M->inv.out, ctx->d_wavx, ctx->d_wavz,
@@ -422,7 +421,7 @@ static int zf_launch(kmm_ctx *ctx, const C *r, C *yo, int nout, const C *tw) {
     ZtmaMaps *M = ztma_maps(ctx);
     if (!M) return KMM_ERR_NOMEM;
     RET(pair_encode(ctx, M->fwd, false, r, yo, nout, nout, f32, KX, YT));
-    const size_t smem = 1024 + sizeof(C) * W * ((size_t)ZF_SLOTS * MZ + NZ + MZ) + 8 * sizeof(uint64_t);
+    const size_t smem = 1024 + sizeof(C) * W * ((size_t)ZF_SLOTS * MZ + NZ + flen<C>(MZ)) + 8 * sizeof(uint64_t);
     // Fields per CTA: all of them in FP64 (58 us at 128 x 129 x 128 against 59 with two and 67 with one,
     // as the ring's loads overlap), two in FP32 (35 against 39 and 44).  A grid of small CTAs' chains
     // that leaves SMs idle is split further: 32 x 33 x 32 (136 tiles) 8.7 us with one field per CTA
