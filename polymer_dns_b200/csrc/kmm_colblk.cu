@@ -3,6 +3,7 @@
 // operations is that of k_col_fwd / k_col_bwd (main_dns.f90:325-544 and 606-771 with
 // solvers.f90:555-1722, 3279-3416); only the data layout and the scan structure differ.
 #include <math.h>
+#include <string.h>
 
 #include "kmm_fft.cuh"
 #include "kmm_colblk.cuh"
@@ -751,7 +752,8 @@ template <int K>
 __global__ void __launch_bounds__(CB_WARPS * 32, K > 8 ? 2 : CB_MINB)
     k_bphirhs_solve(PhiSolveJobs J, PhiSolveCfg S0, PhiSolveCfg S1, int nsolve, int phi,
                     const double *__restrict__ rj, const double *__restrict__ wavx, const double *__restrict__ wavz,
-                    int nz, int nzh, int nxh, double re, double var, double dt, double th, double dyde, double c0) {
+                    int nz, int nzh, int nxh, double re, double var, double dt, double th, double dyde, double c0,
+                    double2 *bt, double2 *bb) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ double2 sbuf[CB_WARPS][2 * (16 * K + 8)];
     double2 *wsm = sbuf[threadIdx.x >> 5];   // bload_s / bstore_s scratch
@@ -769,7 +771,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, K > 8 ? 2 : CB_MINB)
         for (int m = 0; m <= K; ++m)
             x.v[m] = make_double2(d2.v[m].x - P.w2 * x.v[m].x, d2.v[m].y - P.w2 * x.v[m].y);
     }
-    {
+    if (F) {
         BCol<K> f1, f0;
         bload_s<K>(f1, F + P.off, wsm);
         if (FM) {
@@ -780,20 +782,23 @@ __global__ void __launch_bounds__(CB_WARPS * 32, K > 8 ? 2 : CB_MINB)
         }
         bphirhs<K>(x, f1, f0, re, var, dt, th, P.w2, dyde, FULL);
     }
-    bsolve_cfg<K>(x, S0, P, c0, rj);
+    if (bt && bl_t() == 0) bt[P.col] = bb[P.col] = make_double2(0.0, 0.0);
+    if (nsolve > 0) bsolve_cfg<K>(x, S0, P, c0, rj);
     if (nsolve > 1) bsolve_cfg<K>(x, S1, P, c0, rj);
     bstore_s<K>(X + P.off, x, wsm);
 }
 
 int kmm_colblk_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
-                            int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec) {
+                            int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec, double2 *bt,
+                            double2 *bb) {
     const int K = colblk_k(ctx);
-    if (!K) return kmm_warpcol_phirhs_solve(ctx, x, fn, fnm1, nf, var, phi, nsolve, spec);
+    if (!K) return kmm_warpcol_phirhs_solve(ctx, x, fn, fnm1, nf, var, phi, nsolve, spec, bt, bb);
     if (!ctx->use_colblk) return KMM_ERR_UNSUPPORTED;
-    if (nf < 1 || nf > KMM_SOLVE_BATCH || nsolve < 1 || nsolve > 2) return KMM_ERR_ARG;
+    if (nf < 1 || nf > KMM_SOLVE_BATCH || nsolve < 0 || nsolve > 2) return KMM_ERR_ARG;
     PhiSolveCfg S[2];
+    memset(S, 0, sizeof(S));
     const double *rj = NULL;
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < (nsolve ? 2 : 0); ++k) {
         const KmmSolveSpec &q = spec[k < nsolve ? k : 0];
         const int st = kmm_tau_tabset(ctx, q.g, q.robin, q.at, q.bt, q.ab, q.bb, S[k].tab, &rj);
         if (st != KMM_OK) return st;
@@ -811,7 +816,7 @@ int kmm_colblk_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *cons
 #define PS(KK)                                                                                                    \
     k_bphirhs_solve<KK><<<grid, CB_WARPS * 32, 0, ctx->stream>>>(J, S[0], S[1], nsolve, phi, rj, ctx->d_wavx,   \
                                                                 ctx->d_wavz, ctx->nz, ctx->nzh, ctx->nxh, ctx->re, \
-                                                                var, ctx->dt, ctx->theta, ctx->dyde, ctx->h_c[0])
+                                                                var, ctx->dt, ctx->theta, ctx->dyde, ctx->h_c[0], bt, bb)
     switch (K) {
     case 2: PS(2); break;
     case 4: PS(4); break;
@@ -823,6 +828,117 @@ int kmm_colblk_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *cons
 #undef PS
     CKL();
     return KMM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// veloc (solvers.f90:1576-1659), vort (1663-1722) and gradscl (derivatives.f90:90-144) of the routine path
+// in one pass per column pair: the y derivative stays in registers, where cderiv into a scratch field followed
+// by a pointwise kernel wrote and read it once more (veloc, vort and gradscl of 128 x 129 x 96 took 26, 30 and
+// 21 us in two kernels each).
+// ---------------------------------------------------------------------------
+struct BDerivArgs {
+    const double2 *a, *b, *c;   // OP 0: v, omy; 1: u, v, w; 2: s
+    double2 *o0, *o1, *o2;      // OP 0: u, w, v (its (0,0) column is zeroed); 1: omx, omz; 2: sx, sy, sz
+    const double *u0, *w0, *wavx, *wavz;
+    int nz, nzh, nxh;
+    double dyde;
+};
+
+template <int K, int OP>
+__global__ void __launch_bounds__(CB_WARPS * 32, K > 8 ? 2 : CB_MINB) k_bderiv(BDerivArgs A) {
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ double2 sbuf[CB_WARPS][2 * (16 * K + 8)];
+    double2 *wsm = sbuf[threadIdx.x >> 5];   // bload_s / bstore_s scratch
+    BPair P;
+    if (!bpair<K>(P, A.nz, A.nzh, A.nxh, A.wavx, A.wavz)) return;
+    const double kxv = P.kxv, kzv = P.kzv;
+    const double2 zero = make_double2(0.0, 0.0);
+    BCol<K> x, d;
+    if constexpr (OP == 0) {
+        BCol<K> om;
+        bload_s<K>(x, A.a + P.off, wsm);
+        bload_s<K>(om, A.b + P.off, wsm);
+        bcderiv<K>(d, x, A.dyde, FULL);
+#pragma unroll
+        for (int m = 0; m <= K; ++m) {
+            const double2 dv = d.v[m], o = om.v[m];
+            if (P.kx > 0) {
+                const double2 sa = cadd(cimul(dv, -kxv), cimul(o, kzv)), sb = csub(cimul(dv, -kzv), cimul(o, kxv));
+                x.v[m] = make_double2(-sa.x / P.w2, -sa.y / P.w2);
+                d.v[m] = make_double2(-sb.x / P.w2, -sb.y / P.w2);
+            } else if (P.j > 0) {
+                const double kz2 = kzv * kzv;
+                const double2 sa = cimul(o, kzv), sb = cimul(dv, -kzv);
+                x.v[m] = make_double2(-sa.x / kz2, -sa.y / kz2);
+                d.v[m] = make_double2(-sb.x / kz2, -sb.y / kz2);
+            } else {
+                x.v[m] = make_double2(A.u0[bidx<K>(m)], 0.0);
+                d.v[m] = make_double2(A.w0[bidx<K>(m)], 0.0);
+            }
+        }
+        bstore_s<K>(A.o0 + P.off, x, wsm);
+        bstore_s<K>(A.o1 + P.off, d, wsm);
+        if (P.mean) {   // half a warp: plain stores
+#pragma unroll
+            for (int m = 0; m <= K; ++m) A.o2[P.off + bidx<K>(m)] = zero;
+        }
+    } else if constexpr (OP == 1) {
+        BCol<K> v;
+        bload_s<K>(v, A.b + P.off, wsm);
+        bload_s<K>(x, A.a + P.off, wsm);
+        bcderiv<K>(d, x, A.dyde, FULL);
+#pragma unroll
+        for (int m = 0; m <= K; ++m) d.v[m] = csub(cimul(v.v[m], kxv), d.v[m]);   // i kx v - du/dy
+        bstore_s<K>(A.o1 + P.off, d, wsm);
+        bload_s<K>(x, A.c + P.off, wsm);
+        bcderiv<K>(d, x, A.dyde, FULL);
+#pragma unroll
+        for (int m = 0; m <= K; ++m) d.v[m] = csub(d.v[m], cimul(v.v[m], kzv));   // dw/dy - i kz v
+        bstore_s<K>(A.o0 + P.off, d, wsm);
+    } else {
+        bload_s<K>(x, A.a + P.off, wsm);
+        bcderiv<K>(d, x, A.dyde, FULL);
+        bstore_s<K>(A.o1 + P.off, d, wsm);
+#pragma unroll
+        for (int m = 0; m <= K; ++m) d.v[m] = cimul(x.v[m], kxv);
+        bstore_s<K>(A.o0 + P.off, d, wsm);
+#pragma unroll
+        for (int m = 0; m <= K; ++m) d.v[m] = cimul(x.v[m], kzv);
+        bstore_s<K>(A.o2 + P.off, d, wsm);
+    }
+}
+
+template <int OP>
+static int bderiv_launch(kmm_ctx *ctx, BDerivArgs A) {
+    const int K = colblk_k(ctx);
+    if (!K || !ctx->use_colblk) return KMM_ERR_UNSUPPORTED;
+    A.wavx = ctx->d_wavx; A.wavz = ctx->d_wavz;
+    A.nz = ctx->nz; A.nzh = ctx->nzh; A.nxh = ctx->nxh; A.dyde = ctx->dyde;
+    const int nblk = (ctx->nxh * (ctx->nz / 2) + CB_WARPS - 1) / CB_WARPS;
+    switch (K) {
+    case 2: k_bderiv<2, OP><<<nblk, CB_WARPS * 32, 0, ctx->stream>>>(A); break;
+    case 4: k_bderiv<4, OP><<<nblk, CB_WARPS * 32, 0, ctx->stream>>>(A); break;
+    case 6: k_bderiv<6, OP><<<nblk, CB_WARPS * 32, 0, ctx->stream>>>(A); break;
+    case 8: k_bderiv<8, OP><<<nblk, CB_WARPS * 32, 0, ctx->stream>>>(A); break;
+    case 16: k_bderiv<16, OP><<<nblk, CB_WARPS * 32, 0, ctx->stream>>>(A); break;
+    default: return KMM_ERR_UNSUPPORTED;
+    }
+    CKL();
+    return KMM_OK;
+}
+
+int kmm_colblk_veloc(kmm_ctx *ctx, double2 *u, double2 *v, double2 *w, const double2 *omy, const double *u0,
+                     const double *w0) {
+    BDerivArgs A = {v, omy, NULL, u, w, v, u0, w0};
+    return bderiv_launch<0>(ctx, A);
+}
+int kmm_colblk_vort(kmm_ctx *ctx, const double2 *u, const double2 *v, const double2 *w, double2 *omx, double2 *omz) {
+    BDerivArgs A = {u, v, w, omx, omz, NULL, NULL, NULL};
+    return bderiv_launch<1>(ctx, A);
+}
+int kmm_colblk_gradscl(kmm_ctx *ctx, const double2 *s, double2 *sx, double2 *sy, double2 *sz) {
+    BDerivArgs A = {s, NULL, NULL, sx, sy, sz, NULL, NULL};
+    return bderiv_launch<2>(ctx, A);
 }
 
 int kmm_colblk_bwd(kmm_ctx *ctx, const ColBwdArgs &B, const void *tw, bool fp32) {

@@ -1013,8 +1013,13 @@ __global__ void k_zero_wall(double2 *a, double2 *b, size_t n) {
 extern "C" int kmm_phirhs(kmm_ctx *ctx, int v, int fn, int fnm1, double var) {
     if (!ctx || v >= KMM_NSPECTRAL || fn >= KMM_NSPECTRAL || fnm1 >= KMM_NSPECTRAL) return KMM_ERR_ARG;
     double2 *V = SPEC(ctx, v), *F = SPEC(ctx, fn), *FM = SPEC(ctx, fnm1);
-    if (!V || !F || !FM) return KMM_ERR_NOMEM;
-    return kmm_internal_phirhs(ctx, V, F, FM, var);
+    double2 *bt = SPEC(ctx, KMM_BCTOP), *bb = SPEC(ctx, KMM_BCBOT);
+    if (!V || !F || !FM || !bt || !bb) return KMM_ERR_NOMEM;
+    // one pass per column where the blocked or warp-per-column kernels apply (128 x 129 x 96: five launches of
+    // 50 us become one of 21)
+    const double2 *f = F, *fm = FM;
+    const int st = kmm_colblk_phirhs_solve(ctx, &V, &f, &fm, 1, var, 0, 0, NULL, bt, bb);
+    return st != KMM_ERR_UNSUPPORTED ? st : kmm_internal_phirhs(ctx, V, F, FM, var);
 }
 
 int kmm_internal_phirhs_many(kmm_ctx *ctx, double2 *const *V, const double2 *const *F, const double2 *const *FM,
@@ -1062,6 +1067,9 @@ extern "C" int kmm_phi_from_v(kmm_ctx *ctx) {
     if (!ctx) return KMM_ERR_ARG;
     double2 *v = SPEC(ctx, KMM_V);
     if (!v) return KMM_ERR_NOMEM;
+    const double2 *none = NULL;
+    const int st = kmm_colblk_phirhs_solve(ctx, &v, &none, &none, 1, 1.0, 1, 0, NULL);
+    if (st != KMM_ERR_UNSUPPORTED) return st;
     RET(kmm_internal_cderiv(ctx, v, ctx->wrk[1]));
     RET(kmm_internal_cderiv(ctx, ctx->wrk[1], ctx->wrk[0]));
     k_phi<<<kmm_blocks(ctx->nspec, 256), 256, 0, ctx->stream>>>(v, ctx->wrk[0], ctx->d_wavx, ctx->d_wavz, ctx->nspec,
@@ -1090,9 +1098,51 @@ __global__ void k_influence(double2 *__restrict__ v, const double2 *__restrict__
     }
 }
 
+// the same with both wall derivatives of v (nb = nt = 1) formed in the kernel, a warp per column: one launch
+// instead of three, v read once
+__global__ void __launch_bounds__(128) k_influence_w(double2 *__restrict__ v, const double2 *__restrict__ gf1,
+                                                     const double2 *__restrict__ gf2, const double2 *__restrict__ d1b,
+                                                     const double2 *__restrict__ d1t, const double2 *__restrict__ d2b,
+                                                     const double2 *__restrict__ d2t, const double2 *__restrict__ den,
+                                                     double2 *c1o, double2 *c2o, int ncols, int nyp, double dyde) {
+    const int col = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (col >= ncols) return;
+    double2 *V = v + (size_t)col * nyp;
+    double2 b = make_double2(0.0, 0.0), t = b;   // c1derbw / c1dertw (derivatives.f90:362-401, 522-560)
+    for (int i = lane; i < nyp; i += 32) {
+        const double2 x = V[i];
+        const double wt = (double)i * (double)i, wb = (i & 1) ? wt : -wt;
+        b = make_double2(b.x + wb * x.x * dyde, b.y + wb * x.y * dyde);
+        t = make_double2(t.x + wt * x.x * dyde, t.y + wt * x.y * dyde);
+    }
+    for (int o = 16; o; o >>= 1) {
+        b.x += __shfl_xor_sync(0xffffffffu, b.x, o);
+        b.y += __shfl_xor_sync(0xffffffffu, b.y, o);
+        t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+        t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    const double2 c1 = cdiv(csub(cmul(b, d2t[col]), cmul(t, d2b[col])), den[col]);
+    const double2 c2 = cdiv(csub(cmul(t, d1b[col]), cmul(b, d1t[col])), den[col]);
+    if (lane == 0) { c1o[col] = c1; c2o[col] = c2; }
+    for (int i = lane; i < nyp; i += 32) {
+        const size_t x = (size_t)col * nyp + i;
+        const double2 p = cmul(c1, gf1[x]), q = cmul(c2, gf2[x]), vv = V[i];
+        V[i] = make_double2(vv.x + p.x + q.x, vv.y + p.y + q.y);
+    }
+}
+
 extern "C" int kmm_influence(kmm_ctx *ctx) {
     if (!ctx) return KMM_ERR_ARG;
     double2 *v = SPEC(ctx, KMM_V), *wrkc = ctx->wrk[2], *wrk1 = ctx->wrk[3];
+    if (ctx->nb == 1 && ctx->nt == 1) {
+        const int nc = ctx->nz * ctx->nxh;
+        k_influence_w<<<(nc + 3) / 4, 128, 0, ctx->stream>>>(
+            v, SPEC(ctx, KMM_GF1), SPEC(ctx, KMM_GF2), SPEC(ctx, KMM_DNV1B), SPEC(ctx, KMM_DNV1T),
+            SPEC(ctx, KMM_DNV2B), SPEC(ctx, KMM_DNV2T), SPEC(ctx, KMM_DENOM), SPEC(ctx, KMM_C1), SPEC(ctx, KMM_C2), nc,
+            ctx->nyp, ctx->dyde);
+        CKL();
+        return KMM_OK;
+    }
     const int iyb = 2, iyt = 4;
     if (ctx->nb == 1) {
         RET(kmm_internal_wallderiv(ctx, v, 1, 0, wrkc, iyb));
@@ -1149,6 +1199,8 @@ extern "C" int kmm_veloc(kmm_ctx *ctx) {
     double2 *u = SPEC(ctx, KMM_U), *v = SPEC(ctx, KMM_V), *w = SPEC(ctx, KMM_W), *omy = SPEC(ctx, KMM_OMY);
     double *u0 = REAL(ctx, KMM_U0), *w0 = REAL(ctx, KMM_W0);
     if (!u || !v || !w || !omy || !u0 || !w0) return KMM_ERR_NOMEM;
+    const int st = kmm_colblk_veloc(ctx, u, v, w, omy, u0, w0);
+    if (st != KMM_ERR_UNSUPPORTED) return st;
     RET(kmm_internal_cderiv(ctx, v, ctx->wrk[0]));
     k_veloc<<<kmm_blocks(ctx->nspec, 256), 256, 0, ctx->stream>>>(u, v, w, ctx->wrk[0], omy, u0, w0, ctx->d_wavx,
                                                                   ctx->d_wavz, ctx->nspec, ctx->nyp, ctx->nz);
@@ -1172,6 +1224,8 @@ extern "C" int kmm_vort(kmm_ctx *ctx) {
     double2 *u = SPEC(ctx, KMM_U), *v = SPEC(ctx, KMM_V), *w = SPEC(ctx, KMM_W);
     double2 *omx = SPEC(ctx, KMM_OMX), *omz = SPEC(ctx, KMM_OMZ);
     if (!u || !v || !w || !omx || !omz) return KMM_ERR_NOMEM;
+    const int st = kmm_colblk_vort(ctx, u, v, w, omx, omz);
+    if (st != KMM_ERR_UNSUPPORTED) return st;
     {
         const double2 *in[2] = {u, w};
         double2 *out[2] = {omz, omx};
@@ -1258,6 +1312,8 @@ __global__ void k_dxdz_many(DxdzList L, const double *__restrict__ wavx, const d
 extern "C" int kmm_gradscl(kmm_ctx *ctx) {
     if (!ctx) return KMM_ERR_ARG;
     double2 *s = SPEC(ctx, KMM_SCALAR);
+    const int st = kmm_colblk_gradscl(ctx, s, SPEC(ctx, KMM_SCLX), SPEC(ctx, KMM_SCLY), SPEC(ctx, KMM_SCLZ));
+    if (st != KMM_ERR_UNSUPPORTED) return st;
     RET(kmm_internal_cderiv(ctx, s, SPEC(ctx, KMM_SCLY)));
     k_dxdz<<<kmm_blocks(ctx->nspec, 256), 256, 0, ctx->stream>>>(s, SPEC(ctx, KMM_SCLX), SPEC(ctx, KMM_SCLZ),
                                                                  ctx->d_wavx, ctx->d_wavz, ctx->nspec, ctx->nyp, ctx->nz);

@@ -407,7 +407,7 @@ __device__ __forceinline__ void wc_solve(Col<E> &x, const WarpColCfg &S, const W
 template <int E>
 __global__ void __launch_bounds__(WC_WARPS * 32) k_wc_solve(WarpColJobs J, WarpColCfg S0, WarpColCfg S1, int nsolve,
                                                             int rhs, int phi, const double2 *gt, const double2 *gb,
-                                                            WarpColArgs A) {
+                                                            double2 *bt, double2 *bb, WarpColArgs A) {
     const int col = blockIdx.x * WC_WARPS + (threadIdx.x >> 5);
     if (col >= A.ncols) return;
     const size_t off = (size_t)col * A.nyp;
@@ -423,17 +423,20 @@ __global__ void __launch_bounds__(WC_WARPS * 32) k_wc_solve(WarpColJobs J, WarpC
 #pragma unroll
             for (int e = 0; e < E; ++e) x.v[e] = make_double2(d2.v[e].x - w2 * x.v[e].x, d2.v[e].y - w2 * x.v[e].y);
         }
-        Col<E> f1, f0;
-        col_load<E>(f1, J.fn[blockIdx.y] + off, A.nyp);
-        if (J.fnm1[blockIdx.y]) {
-            col_load<E>(f0, J.fnm1[blockIdx.y] + off, A.nyp);
-        } else {
+        if (J.fn[blockIdx.y]) {
+            Col<E> f1, f0;
+            col_load<E>(f1, J.fn[blockIdx.y] + off, A.nyp);
+            if (J.fnm1[blockIdx.y]) {
+                col_load<E>(f0, J.fnm1[blockIdx.y] + off, A.nyp);
+            } else {
 #pragma unroll
-            for (int e = 0; e < E; ++e) f0.v[e] = make_double2(2.0 * f1.v[e].x, 2.0 * f1.v[e].y);
+                for (int e = 0; e < E; ++e) f0.v[e] = make_double2(2.0 * f1.v[e].x, 2.0 * f1.v[e].y);
+            }
+            col_phirhs<E>(x, f1, f0, A.re, A.var, A.dt, A.th, w2, A.nyp, A.dyde);
         }
-        col_phirhs<E>(x, f1, f0, A.re, A.var, A.dt, A.th, w2, A.nyp, A.dyde);
         const double2 zero = make_double2(0.0, 0.0);
-        wc_solve<E>(x, S0, A, col, w2, zero, zero);
+        if (bt && (threadIdx.x & 31) == 0) bt[col] = bb[col] = zero;
+        if (nsolve > 0) wc_solve<E>(x, S0, A, col, w2, zero, zero);
         if (nsolve > 1) wc_solve<E>(x, S1, A, col, w2, zero, zero);
     } else {
         wc_solve<E>(x, S0, A, col, w2, gt[col], gb[col]);
@@ -442,11 +445,12 @@ __global__ void __launch_bounds__(WC_WARPS * 32) k_wc_solve(WarpColJobs J, WarpC
 }
 
 static int wc_launch(kmm_ctx *ctx, const WarpColJobs &J, int nf, const WarpColCfg *S, int nsolve, int rhs, int phi,
-                     double var, const double2 *gt, const double2 *gb, const double *rj) {
+                     double var, const double2 *gt, const double2 *gb, const double *rj, double2 *bt = NULL,
+                     double2 *bb = NULL) {
     WarpColArgs A = {rj, ctx->d_wavx, ctx->d_wavz, ctx->nz * ctx->nxh, ctx->nz, ctx->nyp, ctx->re, var, ctx->dt,
                      ctx->theta, ctx->dyde, ctx->h_c[0]};
     const dim3 grid((A.ncols + WC_WARPS - 1) / WC_WARPS, nf);
-#define WC(EE) k_wc_solve<EE><<<grid, WC_WARPS * 32, 0, ctx->stream>>>(J, S[0], S[1], nsolve, rhs, phi, gt, gb, A)
+#define WC(EE) k_wc_solve<EE><<<grid, WC_WARPS * 32, 0, ctx->stream>>>(J, S[0], S[1], nsolve, rhs, phi, gt, gb, bt, bb, A)
     switch ((ctx->nyp + 31) / 32) {
     case 1: WC(1); break;
     case 2: WC(2); break;
@@ -487,12 +491,14 @@ int kmm_warpcol_solve_many(kmm_ctx *ctx, double2 *const *u, int nf, double g, in
 }
 
 int kmm_warpcol_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
-                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec) {
+                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec, double2 *bt,
+                             double2 *bb) {
     if (!wc_has(ctx)) return KMM_ERR_UNSUPPORTED;
-    if (nf < 1 || nf > KMM_SOLVE_BATCH || nsolve < 1 || nsolve > 2) return KMM_ERR_ARG;
+    if (nf < 1 || nf > KMM_SOLVE_BATCH || nsolve < 0 || nsolve > 2) return KMM_ERR_ARG;
     WarpColCfg S[2];
+    memset(S, 0, sizeof(S));
     const double *rj = NULL;
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < (nsolve ? 2 : 0); ++k) {
         const KmmSolveSpec &q = spec[k < nsolve ? k : 0];
         RET(kmm_tau_tabset(ctx, q.g, q.robin, q.at, q.bt, q.ab, q.bb, S[k].tab, &rj));
         S[k].g = q.g;
@@ -505,7 +511,7 @@ int kmm_warpcol_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *con
         J.fn[m] = fn[m];
         J.fnm1[m] = fnm1[m];
     }
-    return wc_launch(ctx, J, nf, S, nsolve, 1, phi, var, NULL, NULL, rj);
+    return wc_launch(ctx, J, nf, S, nsolve, 1, phi, var, NULL, NULL, rj, bt, bb);
 }
 
 // norm (helpers.f90:91-158) on a column pair held by the two warps of the block.  The exchange

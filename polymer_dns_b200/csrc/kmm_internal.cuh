@@ -221,13 +221,21 @@ struct KmmSolveSpec {
     int robin;   // 1: penta (Robin coefficients at, bt, ab, bb), 0: solve (Dirichlet)
     double at, bt, ab, bb;
 };
+// (fn[0] = NULL: phi alone; nsolve = 0: no solve; bt, bb: wall rows to zero, as phirhs does, or NULL)
 int kmm_colblk_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
-                            int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec);
+                            int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec, double2 *bt = NULL,
+                            double2 *bb = NULL);
+// veloc, vort and gradscl in one pass per column pair; KMM_ERR_UNSUPPORTED where the blocked kernels do not apply
+int kmm_colblk_veloc(kmm_ctx *ctx, double2 *u, double2 *v, double2 *w, const double2 *omy, const double *u0,
+                     const double *w0);
+int kmm_colblk_vort(kmm_ctx *ctx, const double2 *u, const double2 *v, const double2 *w, double2 *omx, double2 *omz);
+int kmm_colblk_gradscl(kmm_ctx *ctx, const double2 *s, double2 *sx, double2 *sy, double2 *sz);
 // both for the other ny (a warp per column; ny up to 191 and 256 .. 287), called by the two above (kmm_fused.cu)
 int kmm_warpcol_solve_many(kmm_ctx *ctx, double2 *const *u, int nf, double g, int robin, double at, double bt,
                            double ab, double bb, const double2 *gt, const double2 *gb);
 int kmm_warpcol_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *const *fn, const double2 *const *fnm1,
-                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec);
+                             int nf, double var, int phi, int nsolve, const KmmSolveSpec *spec, double2 *bt,
+                             double2 *bb);
 // the ny whose column kernels and tau tables are in the blocked layout of kmm_colblk.cuh
 static inline bool kmm_blocked_ny(int ny) { return ny == 32 || ny == 64 || ny == 96 || ny == 128 || ny == 256; }
 // penta (ib = 0) of nf distinct fields of one configuration
