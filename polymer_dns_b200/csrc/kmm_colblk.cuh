@@ -479,7 +479,9 @@ __device__ __forceinline__ void bunstash(BCol<K> &x, const double2 *buf) {
 
 // The two passes on the warp's two columns.  In: xin[n1] = x[16 n1 + n2] on lane (h, n2).  Out, on
 // lane (h, k1 < M): xout[k2] = X[k1 + M k2] for k2 <= 8 (the indices up to N/2 = NY).  tw: the
-// N-point twiddles exp(-2 pi i m/N); s: the warp's shared buffer (2 N elements).
+// table of length N (its W_N^(n2 k1) lane by lane at tw_lane16: from the natural table, where a load's 16
+// entries lay on up to 16 lines, these loads took as many data-pipe wavefronts as the data's own passes);
+// s: the warp's shared buffer (2 N elements).
 template <int K, typename C>
 __device__ __forceinline__ void bdct_passes(const C (&xin)[2 * K], C (&xout)[9], C *s, const C *__restrict__ tw) {
     constexpr int M = 2 * K, N = 16 * M;
@@ -491,7 +493,7 @@ __device__ __forceinline__ void bdct_passes(const C (&xin)[2 * K], C (&xout)[9],
     // twiddle W_N^(n2 k1); transpose through s[h N + 16 k1 + n2]
 #pragma unroll
     for (int k1 = 0; k1 < M; ++k1) {
-        const C w = (t * k1) ? kct::mul(v[k1], __ldg(tw + t * k1)) : v[k1];
+        const C w = (t * k1) ? kct::mul(v[k1], __ldg(tw + kct::tw_lane16(N) + 16 * k1 + t)) : v[k1];
         s[swz<C>(h * N + 16 * k1 + t)] = w;
     }
     __syncwarp();

@@ -59,8 +59,10 @@ __host__ __device__ constexpr int tw_off(int n, int f) {
     return o;
 }
 __host__ __device__ constexpr int tw_packed(int n) { return nfac(n) > 0 ? tw_off(n, nfac(n)) : 0; }
-// a table of length n: n natural entries, the packed table of n, and (n even) that of n / 2
-__host__ __device__ constexpr int tw_total(int n) { return n + tw_packed(n) + (n % 2 == 0 ? tw_packed(n / 2) : 0); }
+// a table of length n: n natural entries, the packed table of n, (n even) that of n / 2, and (n a multiple of
+// 16) the n entries w^(t k) at 16 k + t, t < 16, k < n / 16, of the column kernels' two-pass transform
+__host__ __device__ constexpr int tw_lane16(int n) { return n + tw_packed(n) + (n % 2 == 0 ? tw_packed(n / 2) : 0); }
+__host__ __device__ constexpr int tw_total(int n) { return tw_lane16(n) + (n % 16 == 0 ? n : 0); }
 // where the packed table of length N starts in a table of length TWS N
 template <int N, int TWS>
 constexpr int tw_base = TWS == 1 ? N : 2 * N + tw_packed(2 * N);
@@ -492,6 +494,9 @@ inline void tw_pack(C *t, int n) {
                 for (int k = 0; k < ns; ++k) t[o++] = t[r * k * step * h];
         }
     }
+    if (n % 16 == 0)
+        for (int k = 0; k < n / 16; ++k)
+            for (int l = 0; l < 16; ++l) t[o++] = t[l * k];
 }
 
 // the transform lengths with compiled instances (3/2-rule grids of nx, nz = 32, 64, 96, 128, 384
