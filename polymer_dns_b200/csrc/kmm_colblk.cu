@@ -9,27 +9,18 @@
 #include "kmm_colblk.cuh"
 
 #define CB_WARPS 4   // column pairs per block
-#ifndef KMM_CB_MINB
-#define KMM_CB_MINB 3
-#endif
-#define CB_MINB KMM_CB_MINB   // blocks per SM the register budget is sized for
-// blocks per SM for the FP64 kernels that spill at CB_MINB's register budget: the scalar and u/w
-// kernels and the back kernel run faster with two blocks and no (or little) spilling
-#ifndef KMM_CB_MINB_FWD
-#define KMM_CB_MINB_FWD 2
-#endif
-#ifndef KMM_CB_MINB_BWD
-#define KMM_CB_MINB_BWD 2
-#endif
-// blocks per SM each kernel's register budget is sized for, as measured per kernel: FP64 scalar,
-// u/w and back kernels two, v three, omega_y four; in FP32 the scalar, u/w and omega_y kernels
-// four, v and the back kernel three
-template <typename C> struct CbMinB {
+#define CB_MINB 3   // blocks per SM the routine path's solves are register-sized for
+// Blocks per SM each fused kernel's register budget is sized for, as measured.  FP64: v and omega_y four (their
+// phirhs histories staged in shared memory: v at three with the histories in registers made a 128 x 129 x 128
+// step 643 us, this 633); the scalar and u / w kernels, one column variable live through each transform, three
+// at ny = 128 (two 628 us, three 617, four 629, where they spill) and four at the smaller ny (96: 344 us against
+// 363 with two); the back kernel two, at ny = 96 four (post stage 43 us against 48).  FP32: four, the back
+// kernel three.
+template <int K, typename C> struct CbMinB {
     static constexpr bool f64 = sizeof(C) == 16;
-    static constexpr int fwd = f64 ? KMM_CB_MINB_FWD : 4;   // k_bcol_scl, k_bcol_uw
-    static constexpr int omy = 4;   // with bphirhs_g (its histories staged in shared memory)
-    static constexpr int v = CB_MINB;
-    static constexpr int bwd = f64 ? KMM_CB_MINB_BWD : 3;
+    static constexpr int fwd = f64 && K == 8 ? 3 : 4;   // k_bcol_scl, k_bcol_uw
+    static constexpr int vom = 4;                       // k_bcol_v, k_bcol_omy
+    static constexpr int bwd = !f64 ? 3 : K == 6 ? 4 : 2;
 };
 
 // shared memory of one warp: region A holds the bload_s / bstore_s scratch (2 (NY + 8) double2)
@@ -181,7 +172,7 @@ __device__ __forceinline__ bool bpair(BPair &P, int nz, int nzh, int nxh, const 
 
 // passive scalar (main_dns.f90:325-359): CN/AB2 right-hand side, Robin solve, norm, store; y-physical c, dc/dy
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::fwd) k_bcol_scl(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_scl(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                             const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
@@ -214,7 +205,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::fwd) k_bcol_scl(ColF
 // normal vorticity (main_dns.f90:411-422, 479-502, 520-526): phirhs, Robin solve, norm, store;
 // y-physical omega_y; uzero for the mean modes in place of the (0,0) pair
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::omy) k_bcol_omy(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::vom) k_bcol_omy(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                             const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
@@ -278,7 +269,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::omy) k_bcol_omy(ColF
 // wall-normal velocity (main_dns.f90:363-407, 426-466, 489-502, 520): phi, phirhs, Helmholtz and
 // Poisson solves, influence-matrix correction, norm, store; y-physical v
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::v) k_bcol_v(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::vom) k_bcol_v(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                           const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
@@ -302,14 +293,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::v) k_bcol_v(ColFwdAr
 #pragma unroll
         for (int m = 0; m <= K; ++m) v.v[m] = make_double2(d2.v[m].x - w2 * v.v[m].x, d2.v[m].y - w2 * v.v[m].y);
     }
-    if constexpr (sizeof(C) == 16) {   // FP64: the register form (measured faster at this budget)
-        BCol<K> f1, f0;
-        bload_s<K>(f1, A.fn + P.off, wsm);
-        bload_s<K>(f0, A.fnm1 + P.off, wsm);
-        bphirhs<K>(v, f1, f0, A.re, 1.0, A.dt, A.th, w2, A.dyde, FULL);
-    } else {
-        bphirhs_g<K>(v, A.fn + P.off, A.fnm1 + P.off, wsm, A.re, 1.0, A.dt, A.th, w2, A.dyde, FULL);
-    }
+    bphirhs_g<K>(v, A.fn + P.off, A.fnm1 + P.off, wsm, A.re, 1.0, A.dt, A.th, w2, A.dyde, FULL);
     {
         const TauTab tp = tab_at(T, TB_PHI, P.tcol, NYP);
         bsolve_dirichlet<K>(v, tp, zero, zero, w2 + g1, A.c0, rj, FULL);
@@ -357,7 +341,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::v) k_bcol_v(ColFwdAr
 
 // veloc (solvers.f90:1576-1659) from the new v and omega_y; y-physical u, du/dy, w, dw/dy
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::fwd) k_bcol_uw(ColFwdArgs A, const C *__restrict__ tw) {
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_uw(ColFwdArgs A, const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ double2 sm[];
@@ -369,59 +353,44 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::fwd) k_bcol_uw(ColFw
     const size_t fstride = (size_t)A.nz * A.nxh * col_ld<C>(NYP), yoff = (size_t)P.col * col_ld<C>(NYP);
     const double2 zero = make_double2(0.0, 0.0);
     const double kxv = P.kxv, kzv = P.kzv, w2 = P.w2;
-    BCol<K> u, w;
+    // blockIdx.y: u or w.  v and omega_y are read twice (from L2), but one column variable is live through the
+    // transforms, and a small grid's two halves run side by side
     {
-        BCol<K> v, om, dv;
-        bload_s<K>(v, A.v + P.off, wsm);
-        bload_s<K>(om, A.omy + P.off, wsm);
-        bcderiv<K>(dv, v, A.dyde, FULL);
+        const int which = blockIdx.y;
+        BCol<K> x;
+        {
+            BCol<K> om, dv;
+            bload_s<K>(x, A.v + P.off, wsm);
+            bload_s<K>(om, A.omy + P.off, wsm);
+            bcderiv<K>(dv, x, A.dyde, FULL);
+            // u = -(-i kx dv + i kz om) / k^2, w = -(-i kz dv - i kx om) / k^2
+            const double cd = which == 0 ? -kxv : -kzv, co = which == 0 ? kzv : -kxv;
+            const double kk = P.kx > 0 ? w2 : kzv * kzv;
 #pragma unroll
-        for (int m = 0; m <= K; ++m) {
-            const double2 d = dv.v[m], o = om.v[m];
-            if (P.kx > 0) {
-                const double2 sa = cadd(cimul(d, -kxv), cimul(o, kzv));
-                u.v[m] = make_double2(-sa.x / w2, -sa.y / w2);
-                const double2 sb = csub(cimul(d, -kzv), cimul(o, kxv));
-                w.v[m] = make_double2(-sb.x / w2, -sb.y / w2);
-            } else if (P.j > 0) {
-                const double kz2 = kzv * kzv;
-                const double2 sa = cimul(o, kzv);
-                u.v[m] = make_double2(-sa.x / kz2, -sa.y / kz2);
-                const double2 sb = cimul(d, -kzv);
-                w.v[m] = make_double2(-sb.x / kz2, -sb.y / kz2);
-            } else {
-                u.v[m] = zero;
-                w.v[m] = zero;
+            for (int m = 0; m <= K; ++m) {
+                const double2 sa = cadd(cimul(dv.v[m], cd), cimul(om.v[m], co));
+                x.v[m] = make_double2(-sa.x / kk, -sa.y / kk);
             }
         }
-    }
-    if (P.mean) {
+        if (P.mean) {
+            const double *m0 = which == 0 ? A.u0 : A.w0;
 #pragma unroll
-        for (int m = 0; m <= K; ++m) {
-            const int i = bidx<K>(m);
-            u.v[m] = make_double2(A.u0[i], 0.0);
-            w.v[m] = make_double2(A.w0[i], 0.0);
+            for (int m = 0; m <= K; ++m) x.v[m] = make_double2(m0[bidx<K>(m)], 0.0);
         }
-    }
-    // norm(u), norm(w): the pair is conjugate-symmetric already; zero the kz Nyquist column
-    if (P.j == A.nzh) {
+        // norm(u), norm(w): the pair is conjugate-symmetric already; zero the kz Nyquist column
+        if (P.j == A.nzh) {
 #pragma unroll
-        for (int m = 0; m <= K; ++m) {
-            u.v[m] = zero;
-            w.v[m] = zero;
+            for (int m = 0; m <= K; ++m) x.v[m] = zero;
         }
+        bdct_store<K, C>(x, fa, fb, tw, (C *)A.yp + (which == 0 ? 0 : 2) * fstride + yoff);
+        BCol<K> d1;
+        bcderiv<K>(d1, x, A.dyde, FULL);
+        bdct_store<K, C>(d1, fa, fb, tw, (C *)A.yp + (which == 0 ? 4 : 5) * fstride + yoff);
     }
-    BCol<K> d1;
-    bcderiv<K>(d1, u, A.dyde, FULL);
-    bdct_store<K, C>(u, fa, fb, tw, (C *)A.yp + 0 * fstride + yoff);
-    bdct_store<K, C>(d1, fa, fb, tw, (C *)A.yp + 4 * fstride + yoff);
-    bcderiv<K>(d1, w, A.dyde, FULL);
-    bdct_store<K, C>(w, fa, fb, tw, (C *)A.yp + 2 * fstride + yoff);
-    bdct_store<K, C>(d1, fa, fb, tw, (C *)A.yp + 5 * fstride + yoff);
 }
 
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<C>::bwd) k_bcol_bwd(ColBwdArgs A, const C *__restrict__ tw) {
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::bwd) k_bcol_bwd(ColBwdArgs A, const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ double2 sm[];
@@ -612,7 +581,7 @@ int kmm_colblk_fwd(kmm_ctx *ctx, const ColFwdArgs &A, const FusedTabs &T, const 
         if (A.scalar) CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[0], 0));                      \
         CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[1], 0));                                    \
         RET(kmm_smem_attr(ctx, (const void *)k_bcol_uw<KK, CC>, smem));                               \
-        k_bcol_uw<KK, CC><<<nblk, CB_WARPS * 32, smem, ctx->stream>>>(A, twc);                         \
+        k_bcol_uw<KK, CC><<<dim3(nblk, 2), CB_WARPS * 32, smem, ctx->stream>>>(A, twc);                \
         CKL();                                                                                        \
         return KMM_OK;                                                                                \
     } while (0)
