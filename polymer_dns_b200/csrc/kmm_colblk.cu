@@ -14,12 +14,14 @@
 // phirhs histories staged in shared memory: v at three with the histories in registers made a 128 x 129 x 128
 // step 643 us, this 633); the scalar and u / w kernels, one column variable live through each transform, three
 // at ny = 128 (two 628 us, three 617, four 629, where they spill) and four at the smaller ny (96: 344 us against
-// 363 with two); the back kernel two, at ny = 96 four (post stage 43 us against 48).  FP32: four, the back
-// kernel three.
+// 363 with two); the back kernel two, at ny = 96 four (post stage 43 us against 48).  FP32: four (v at
+// three made a 128 x 129 x 128 mixed step 498 us, four 487; at ny = 96 it stays at three, where the budget of four
+// is compiled to another last bit of v and mixed runs would not repeat earlier ones), the back kernel three.
 template <int K, typename C> struct CbMinB {
     static constexpr bool f64 = sizeof(C) == 16;
     static constexpr int fwd = f64 && K == 8 ? 3 : 4;   // k_bcol_scl, k_bcol_uw
-    static constexpr int vom = 4;                       // k_bcol_v, k_bcol_omy
+    static constexpr int omy = 4;
+    static constexpr int v = !f64 && K == 6 ? 3 : 4;
     static constexpr int bwd = !f64 ? 3 : K == 6 ? 4 : 2;
 };
 
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_scl(C
 // normal vorticity (main_dns.f90:411-422, 479-502, 520-526): phirhs, Robin solve, norm, store;
 // y-physical omega_y; uzero for the mean modes in place of the (0,0) pair
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::vom) k_bcol_omy(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::omy) k_bcol_omy(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                             const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::vom) k_bcol_omy(C
 // wall-normal velocity (main_dns.f90:363-407, 426-466, 489-502, 520): phi, phirhs, Helmholtz and
 // Poisson solves, influence-matrix correction, norm, store; y-physical v
 template <int K, typename C>
-__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::vom) k_bcol_v(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
+__global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::v) k_bcol_v(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                           const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
@@ -368,7 +370,12 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_uw(Co
             const double kk = P.kx > 0 ? w2 : kzv * kzv;
 #pragma unroll
             for (int m = 0; m <= K; ++m) {
-                const double2 sa = cadd(cimul(dv.v[m], cd), cimul(om.v[m], co));
+                const double2 d = dv.v[m], o = om.v[m];
+                // which product stays unrounded is fixed here: the mixed form's FP32 transforms amplify a last
+                // bit of u or w to the rounding floor of fn, and a run is to repeat from build to build
+                const double2 sa = make_double2(__fma_rn(-cd, d.y, -__dmul_rn(co, o.y)),
+                                                which == 0 ? __fma_rn(co, o.x, __dmul_rn(cd, d.x))
+                                                           : __fma_rn(cd, d.x, __dmul_rn(co, o.x)));
                 x.v[m] = make_double2(-sa.x / kk, -sa.y / kk);
             }
         }

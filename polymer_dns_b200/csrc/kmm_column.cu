@@ -1010,6 +1010,11 @@ __global__ void k_zero_wall(double2 *a, double2 *b, size_t n) {
     GRID_LOOP(n) { a[idx] = make_double2(0.0, 0.0); b[idx] = make_double2(0.0, 0.0); }
 }
 
+// The one-pass forms below sum a derivative in another order than kmm_cderiv (the last bit differs).  A
+// mixed-precision context keeps the general forms: its FP32 transforms amplify a last bit to the rounding floor of
+// fn (1e-4 of its norm at 128 x 129 x 128), and its runs are to repeat those of the same initial state.
+static bool one_pass(const kmm_ctx *ctx) { return ctx->p.precision == 0; }
+
 extern "C" int kmm_phirhs(kmm_ctx *ctx, int v, int fn, int fnm1, double var) {
     if (!ctx || v >= KMM_NSPECTRAL || fn >= KMM_NSPECTRAL || fnm1 >= KMM_NSPECTRAL) return KMM_ERR_ARG;
     double2 *V = SPEC(ctx, v), *F = SPEC(ctx, fn), *FM = SPEC(ctx, fnm1);
@@ -1018,7 +1023,7 @@ extern "C" int kmm_phirhs(kmm_ctx *ctx, int v, int fn, int fnm1, double var) {
     // one pass per column where the blocked or warp-per-column kernels apply (128 x 129 x 96: five launches of
     // 50 us become one of 21)
     const double2 *f = F, *fm = FM;
-    const int st = kmm_colblk_phirhs_solve(ctx, &V, &f, &fm, 1, var, 0, 0, NULL, bt, bb);
+    const int st = one_pass(ctx) ? kmm_colblk_phirhs_solve(ctx, &V, &f, &fm, 1, var, 0, 0, NULL, bt, bb) : KMM_ERR_UNSUPPORTED;
     return st != KMM_ERR_UNSUPPORTED ? st : kmm_internal_phirhs(ctx, V, F, FM, var);
 }
 
@@ -1068,7 +1073,7 @@ extern "C" int kmm_phi_from_v(kmm_ctx *ctx) {
     double2 *v = SPEC(ctx, KMM_V);
     if (!v) return KMM_ERR_NOMEM;
     const double2 *none = NULL;
-    const int st = kmm_colblk_phirhs_solve(ctx, &v, &none, &none, 1, 1.0, 1, 0, NULL);
+    const int st = one_pass(ctx) ? kmm_colblk_phirhs_solve(ctx, &v, &none, &none, 1, 1.0, 1, 0, NULL) : KMM_ERR_UNSUPPORTED;
     if (st != KMM_ERR_UNSUPPORTED) return st;
     RET(kmm_internal_cderiv(ctx, v, ctx->wrk[1]));
     RET(kmm_internal_cderiv(ctx, ctx->wrk[1], ctx->wrk[0]));
@@ -1099,7 +1104,7 @@ __global__ void k_influence(double2 *__restrict__ v, const double2 *__restrict__
 }
 
 // the same with both wall derivatives of v (nb = nt = 1) formed in the kernel, a warp per column: one launch
-// instead of three, v read once
+// instead of three, v read once.  The sums are k_wallderiv's, in its order (bit for bit the same v).
 __global__ void __launch_bounds__(128) k_influence_w(double2 *__restrict__ v, const double2 *__restrict__ gf1,
                                                      const double2 *__restrict__ gf2, const double2 *__restrict__ d1b,
                                                      const double2 *__restrict__ d1t, const double2 *__restrict__ d2b,
@@ -1109,13 +1114,14 @@ __global__ void __launch_bounds__(128) k_influence_w(double2 *__restrict__ v, co
     if (col >= ncols) return;
     double2 *V = v + (size_t)col * nyp;
     double2 b = make_double2(0.0, 0.0), t = b;   // c1derbw / c1dertw (derivatives.f90:362-401, 522-560)
-    for (int i = lane; i < nyp; i += 32) {
+    const int chunk = (nyp + 31) / 32, i1 = min(nyp, (lane + 1) * chunk);
+    for (int i = lane * chunk; i < i1; ++i) {
         const double2 x = V[i];
         const double wt = (double)i * (double)i, wb = (i & 1) ? wt : -wt;
         b = make_double2(b.x + wb * x.x * dyde, b.y + wb * x.y * dyde);
         t = make_double2(t.x + wt * x.x * dyde, t.y + wt * x.y * dyde);
     }
-    for (int o = 16; o; o >>= 1) {
+    for (int o = 1; o < 32; o <<= 1) {
         b.x += __shfl_xor_sync(0xffffffffu, b.x, o);
         b.y += __shfl_xor_sync(0xffffffffu, b.y, o);
         t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
@@ -1199,7 +1205,7 @@ extern "C" int kmm_veloc(kmm_ctx *ctx) {
     double2 *u = SPEC(ctx, KMM_U), *v = SPEC(ctx, KMM_V), *w = SPEC(ctx, KMM_W), *omy = SPEC(ctx, KMM_OMY);
     double *u0 = REAL(ctx, KMM_U0), *w0 = REAL(ctx, KMM_W0);
     if (!u || !v || !w || !omy || !u0 || !w0) return KMM_ERR_NOMEM;
-    const int st = kmm_colblk_veloc(ctx, u, v, w, omy, u0, w0);
+    const int st = one_pass(ctx) ? kmm_colblk_veloc(ctx, u, v, w, omy, u0, w0) : KMM_ERR_UNSUPPORTED;
     if (st != KMM_ERR_UNSUPPORTED) return st;
     RET(kmm_internal_cderiv(ctx, v, ctx->wrk[0]));
     k_veloc<<<kmm_blocks(ctx->nspec, 256), 256, 0, ctx->stream>>>(u, v, w, ctx->wrk[0], omy, u0, w0, ctx->d_wavx,
@@ -1224,7 +1230,7 @@ extern "C" int kmm_vort(kmm_ctx *ctx) {
     double2 *u = SPEC(ctx, KMM_U), *v = SPEC(ctx, KMM_V), *w = SPEC(ctx, KMM_W);
     double2 *omx = SPEC(ctx, KMM_OMX), *omz = SPEC(ctx, KMM_OMZ);
     if (!u || !v || !w || !omx || !omz) return KMM_ERR_NOMEM;
-    const int st = kmm_colblk_vort(ctx, u, v, w, omx, omz);
+    const int st = one_pass(ctx) ? kmm_colblk_vort(ctx, u, v, w, omx, omz) : KMM_ERR_UNSUPPORTED;
     if (st != KMM_ERR_UNSUPPORTED) return st;
     {
         const double2 *in[2] = {u, w};
@@ -1312,7 +1318,8 @@ __global__ void k_dxdz_many(DxdzList L, const double *__restrict__ wavx, const d
 extern "C" int kmm_gradscl(kmm_ctx *ctx) {
     if (!ctx) return KMM_ERR_ARG;
     double2 *s = SPEC(ctx, KMM_SCALAR);
-    const int st = kmm_colblk_gradscl(ctx, s, SPEC(ctx, KMM_SCLX), SPEC(ctx, KMM_SCLY), SPEC(ctx, KMM_SCLZ));
+    const int st = one_pass(ctx) ? kmm_colblk_gradscl(ctx, s, SPEC(ctx, KMM_SCLX), SPEC(ctx, KMM_SCLY), SPEC(ctx, KMM_SCLZ))
+                                 : KMM_ERR_UNSUPPORTED;
     if (st != KMM_ERR_UNSUPPORTED) return st;
     RET(kmm_internal_cderiv(ctx, s, SPEC(ctx, KMM_SCLY)));
     k_dxdz<<<kmm_blocks(ctx->nspec, 256), 256, 0, ctx->stream>>>(s, SPEC(ctx, KMM_SCLX), SPEC(ctx, KMM_SCLZ),

@@ -511,20 +511,24 @@ extern "C" int kmm_tracer_cells(kmm_ctx *ctx, int *cells, size_t n) {
 // ---------------------------------------------------------------------------
 // xyzfft(a,b,-1), helpers.f90:6-87: physical (nyp,nz,nx) -> spectral (nyp,nz,nxh)
 // ---------------------------------------------------------------------------
-// One warp per transform, two real lines in each as real and imaginary part of one complex FFT; a block's
+// One warp per transform, NL = 2 real lines in each as real and imaginary part of one complex FFT; a block's
 // warps take neighbouring lines, so that every pass moves runs of consecutive y (64 bytes in x, 128 in z).
 // With a block per real line, strided 8- and 16-byte accesses and a copy of the input first, the three
 // passes took 65 us a call at 64 x 97 x 64 where these take 29.
+// NL = 1, one line per transform, forms the initial fields of a mixed-precision context: the steps that follow
+// amplify a last-bit difference to the FP32 rounding floor of fn (1e-4 at 128 x 129 x 128), so that a mixed run
+// repeats earlier runs of the same initial state only from the very same bits.
 
 // y: DCT-I of each real column, /ny, halve the end values
+template <int NL>
 __global__ void k_xyz_y(const double *__restrict__ in, double *__restrict__ b, const __grid_constant__ DevPlan P, int nyp,
                         int ncols) {
     extern __shared__ double2 sm[];
     const int ny = nyp - 1, L = 2 * ny;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c0 = 2 * (blockIdx.x * (blockDim.x >> 5) + warp);
+    const int c0 = NL * (blockIdx.x * (blockDim.x >> 5) + warp);
     if (c0 >= ncols) return;
-    const bool two = c0 + 1 < ncols;
+    const bool two = NL == 2 && c0 + 1 < ncols;
     double2 *a = sm + (size_t)warp * 2 * L, *c = a + L;
     const double *src = in + (size_t)c0 * nyp;
     for (int i = lane; i < nyp; i += 32) {
@@ -544,17 +548,20 @@ __global__ void k_xyz_y(const double *__restrict__ in, double *__restrict__ b, c
 }
 
 // x: r2c over nx for each (i,j) line (stride nz*nyp), /nx, keep k < nxh -> complex work (nyp,nz,nxh).
-// blockIdx.y is j; a block's W warps take the 2 W lines i0 .. i0 + 2 W - 1
+// blockIdx.y is j; a block's W warps take the NL W lines i0 .. i0 + NL W - 1
+template <int NL>
 __global__ void k_xyz_x(const double *__restrict__ b, double2 *__restrict__ a, const __grid_constant__ DevPlan P, int nyp, int nz, int nx) {
     extern __shared__ double2 sm[];
     const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = blockIdx.x * 2 * W, j = blockIdx.y;
-    const unsigned mW = div_magic(2 * W);
+    const int i0 = blockIdx.x * NL * W, j = blockIdx.y;
+    const unsigned mW = div_magic(NL * W);
     double *t = reinterpret_cast<double *>(sm);
-    for (int e = threadIdx.x; e < 2 * W * nx; e += blockDim.x) {
-        const int k = div_by(e, mW), il = e - k * 2 * W;
-        // line i0 + il: part il & 1 of element k of the warp's sequence il / 2
-        t[((size_t)(il >> 1) * 2 * nx + k) * 2 + (il & 1)] = i0 + il < nyp ? b[((size_t)k * nz + j) * nyp + i0 + il] : 0.0;
+    for (int e = threadIdx.x; e < NL * W * nx; e += blockDim.x) {
+        const int k = div_by(e, mW), il = e - k * NL * W;
+        // line i0 + il: part il % NL of element k of the warp's sequence il / NL
+        double *te = t + ((size_t)(il / NL) * 2 * nx + k) * 2 + il % NL;
+        *te = i0 + il < nyp ? b[((size_t)k * nz + j) * nyp + i0 + il] : 0.0;
+        if (NL == 1) te[1] = 0.0;
     }
     __syncthreads();
     double2 *s = sm + (size_t)warp * 2 * nx;
@@ -564,6 +571,10 @@ __global__ void k_xyz_x(const double *__restrict__ b, double2 *__restrict__ a, c
     double2 *o = r == s ? s + nx : s;
     const int nxh = nx / 2;
     for (int k = lane; k < nxh; k += 32) {
+        if (NL == 1) {
+            o[k] = make_double2(r[k].x / (double)nx, r[k].y / (double)nx);
+            continue;
+        }
         const double2 z = r[k], zc = cconj(r[k ? nx - k : 0]);
         const double2 p = cadd(z, zc), m = csub(z, zc);
         o[2 * k] = make_double2(0.5 * p.x / (double)nx, 0.5 * p.y / (double)nx);
@@ -571,10 +582,10 @@ __global__ void k_xyz_x(const double *__restrict__ b, double2 *__restrict__ a, c
     }
     __syncthreads();
     const size_t half = (size_t)(o - s);   // the same for every warp (a stage count)
-    for (int e = threadIdx.x; e < 2 * W * nxh; e += blockDim.x) {
-        const int k = div_by(e, mW), il = e - k * 2 * W;
+    for (int e = threadIdx.x; e < NL * W * nxh; e += blockDim.x) {
+        const int k = div_by(e, mW), il = e - k * NL * W;
         if (i0 + il < nyp)
-            a[((size_t)k * nz + j) * nyp + i0 + il] = sm[(size_t)(il >> 1) * 2 * nx + half + 2 * k + (il & 1)];
+            a[((size_t)k * nz + j) * nyp + i0 + il] = sm[(size_t)(il / NL) * 2 * nx + half + NL * k + il % NL];
     }
 }
 
@@ -611,23 +622,29 @@ static int xyz_warps(int n, int most) {
 }
 
 // the three passes on stream st: in (nyp, nz, nx) real -> b (a real copy's space) -> a; py, px, pz: plans of
-// 2 ny, nx, nz (radix 8 first).  Nothing is allocated.
-cudaError_t kmm_xyz_passes(const double *in, double *b, double2 *a, const DevPlan &py, const DevPlan &px,
+// 2 ny, nx, nz.  Nothing is allocated.
+template <int NL>
+static cudaError_t xyz_passes(const double *in, double *b, double2 *a, const DevPlan &py, const DevPlan &px,
                            const DevPlan &pz, int nyp, int nz, int nx, cudaStream_t st) {
     const int wy = xyz_warps(py.n, 4), wx = xyz_warps(nx, 4), wz = xyz_warps(nz, 8), ncols = nz * nx;
     const size_t sy = sizeof(double2) * 2 * (size_t)py.n * wy, sx = sizeof(double2) * 2 * (size_t)nx * wx,
                  sz = sizeof(double2) * 2 * (size_t)nz * wz;
-    const void *kern[3] = {(const void *)k_xyz_y, (const void *)k_xyz_x, (const void *)k_xyz_z};
+    const void *kern[3] = {(const void *)k_xyz_y<NL>, (const void *)k_xyz_x<NL>, (const void *)k_xyz_z};
     const size_t need[3] = {sy, sx, sz};
     for (int t = 0; t < 3; ++t)   // setting a function attribute allocates nothing
         if (need[t] > 48 * 1024) {
             const cudaError_t e = cudaFuncSetAttribute(kern[t], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need[t]);
             if (e != cudaSuccess) return e;
         }
-    k_xyz_y<<<(ncols + 2 * wy - 1) / (2 * wy), wy * 32, sy, st>>>(in, b, py, nyp, ncols);
-    k_xyz_x<<<dim3((nyp + 2 * wx - 1) / (2 * wx), nz), wx * 32, sx, st>>>(b, a, px, nyp, nz, nx);
+    k_xyz_y<NL><<<(ncols + NL * wy - 1) / (NL * wy), wy * 32, sy, st>>>(in, b, py, nyp, ncols);
+    k_xyz_x<NL><<<dim3((nyp + NL * wx - 1) / (NL * wx), nz), wx * 32, sx, st>>>(b, a, px, nyp, nz, nx);
     k_xyz_z<<<dim3((nyp + wz - 1) / wz, nx / 2), wz * 32, sz, st>>>(a, pz, nyp, nz);
     return cudaGetLastError();
+}
+
+cudaError_t kmm_xyz_passes(const double *in, double *b, double2 *a, const DevPlan &py, const DevPlan &px,
+                           const DevPlan &pz, int nyp, int nz, int nx, cudaStream_t st) {
+    return xyz_passes<2>(in, b, a, py, px, pz, nyp, nz, nx, st);
 }
 
 extern "C" int kmm_xyzfft(kmm_ctx *ctx, int dst, int src) {
@@ -638,10 +655,14 @@ extern "C" int kmm_xyzfft(kmm_ctx *ctx, int dst, int src) {
     const size_t np = (size_t)ctx->nyp * ctx->nz * ctx->nx;
     double *b = NULL;
     CK(cudaMallocAsync((void **)&b, sizeof(double) * np, ctx->stream));
-    DevPlan px, pz;
-    kmm_plan_r8(&ctx->pnx, &px);
-    kmm_plan_r8(&ctx->pnz, &pz);
-    CK(kmm_xyz_passes(b0, b, a, ctx->wy2, px, pz, ctx->nyp, ctx->nz, ctx->nx, ctx->stream));
+    if (ctx->p.precision == 1) {
+        CK(xyz_passes<1>(b0, b, a, ctx->py2, ctx->pnx, ctx->pnz, ctx->nyp, ctx->nz, ctx->nx, ctx->stream));
+    } else {
+        DevPlan px, pz;
+        kmm_plan_r8(&ctx->pnx, &px);
+        kmm_plan_r8(&ctx->pnz, &pz);
+        CK(xyz_passes<2>(b0, b, a, ctx->wy2, px, pz, ctx->nyp, ctx->nz, ctx->nx, ctx->stream));
+    }
     ctx->launches += 3;
     CK(cudaFreeAsync(b, ctx->stream));
     return KMM_OK;
