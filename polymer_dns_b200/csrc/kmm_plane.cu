@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256) k_xphys(const double2 *__restrict__ q, do
 }
 
 // 3''. the x stage for 3/2 grids too long for a row of every input field to fit in shared memory
-// (k_xphys needs nin x 2 rows x mx doubles: 507 KB for the 55 polymer inputs at mx = 576).  Two
+// (k_xphys needs nin x 2 rows x mx doubles: 387 KB for the 42 polymer inputs at mx = 576).  Two
 // passes through HBM: k_xinv_big takes the Hermitian c2r of one field pair for XZB rows with the
 // runtime block FFT (the same transform as k_xphys) into a physical buffer [f][y][z][x]; k_xpoint
 // evaluates the same pointwise terms (xphys_point) with one thread per 3/2-grid point, every block
@@ -721,12 +721,12 @@ __global__ void __launch_bounds__(256) k_xpoint(const T *__restrict__ pb, T *__r
 // compile-time warp FFT into the row's physical table in shared memory; then the block evaluates
 // the pointwise terms.  The two physical rows of a pair are one buffer of MX complex values, which
 // serves as the FFT's second (ping-pong) buffer once the pair's input has been read out of it, so
-// a warp needs only one private buffer and two 7-warp blocks fit on an SM even with 55 fields.
+// a warp needs only one private buffer and two 7-warp blocks fit on an SM with 42 to 55 fields.
 // The generic k_xphys tiles two rows per block and transforms them with the runtime block FFT.
 #define XW 4    // warps of k_xfwd2
-// warps of k_xphys2: 7 in FP64 (two blocks per SM, held by shared memory and registers; the 28
-// field pairs of the polymer + scalar inputs then take four full rounds, where 8 warps left half
-// of them idle in the last round before the block barrier: 3.8 % faster at 128^3); 4 in FP32,
+// warps of k_xphys2: 7 in FP64 (two blocks per SM, held by shared memory and registers; the 21
+// field pairs of the polymer + scalar inputs then take three full rounds, where 8 warps leave three
+// of them idle in the last round before the block barrier); 4 in FP32,
 // whose halved row buffer already lets four blocks share an SM, where 8-warp blocks would be held
 // to two by registers with more idle threads in the pointwise pass
 template <typename C>
@@ -1189,6 +1189,18 @@ static int dct_h_bwd(kmm_ctx *ctx, int nf, const C *pl, const FieldPtrsW &out, c
 #undef DH
 }
 
+// qp = zb str for the six components (blockIdx.y)
+struct StrQp {
+    const double2 *s[6];
+    double2 *q[6];
+};
+__global__ void k_qp_scale(StrQp L, size_t n, double zb) {
+    const double2 *__restrict__ s = L.s[blockIdx.y];
+    double2 *__restrict__ q = L.q[blockIdx.y];
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
+        q[e] = cscale(s[e], zb);
+}
+
 // ---------------------------------------------------------------------------
 // physical scratch (outputs, drag) sized on demand
 // ---------------------------------------------------------------------------
@@ -1327,6 +1339,13 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
 
     // inputs actually consumed by the physics (the reference also transforms u_ij and the
     // Laplacian every step; those only feed output, swirl and the inertial-particle path)
+    // FP64 only: two fields share each transform along x, so that another set of fields changes the last bits of
+    // all, which the mixed form's FP32 transforms amplify to the rounding floor of fn (4e-4 at 96 x 97 x 96)
+    const bool lean = ctx->p.precision == 0;
+    // qp_ij = (1 - beta) / (re beta tpoly) str_ij with a constant beta (itarget = 0): formed from str_ij's
+    // coefficients at the end instead of being transformed
+    const bool qp_scaled = poly && lean && ctx->p.itarget == 0;
+    static const int kQpOut[6] = {KMM_QP11, KMM_QP12, KMM_QP13, KMM_QP22, KMM_QP23, KMM_QP33};
     PhysArgs A;
     memset(&A, 0, sizeof(A));
     for (int s = 0; s < S_NSLOT; ++s) A.slot_of_in[s] = -1;
@@ -1338,7 +1357,8 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     // Inside a routine step without inertial particles the x and z derivatives among the inputs
     // (the velocity gradient's i kx / i kz columns, the scalar's, the conformation tensor's) are
     // formed in the z inverse from their field's plane, and the symmetric tensor's duplicate
-    // components share one plane: 23 y transforms instead of 55 with polymer and scalar.  The
+    // components share one plane: 23 y transforms instead of 55 with polymer and scalar.
+    // FP64 steps form 42 inputs from them (below).  The
     // step computes only the y derivatives for it (kmm_step).
     const bool derived = kmm_derived_inputs(ctx) && ctx->in_step;
     auto add_base = [&](int fid) -> int {
@@ -1372,7 +1392,8 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     static const int fl[6] = {KMM_U, KMM_V, KMM_W, KMM_OMX, KMM_OMY, KMM_OMZ};
     for (int m = 0; m < 6; ++m) RET(add_in(S_U + m, fl[m]));
     if (scal) {
-        if (poly) RET(add_in(S_SC, KMM_SCALAR));   // the scalar itself enters only the polymer's beta (itarget)
+        // the scalar itself enters only the polymer's beta of itarget = 1, 2
+        if (poly && (ctx->p.itarget != 0 || !lean)) RET(add_in(S_SC, KMM_SCALAR));
         if (derived) {
             RET(add_in_from(S_CX, KMM_SCALAR, 1));
             RET(add_in(S_CY, KMM_SCLY));
@@ -1395,10 +1416,17 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
         for (int m = 0; m < 3; ++m) RET(add_in(S_LU + m, KMM_LU + m));
     if (poly) {
         // c_ij and dc_ijk = d c_ij / d x_k; c21 = c12, c31 = c13, c32 = c23 (copied by the step)
+        // (those share one input; the pointwise terms read dc_ijk of the six distinct components only): 42 inputs
+        // with the scalar instead of 55, whose z inverse and x stage took 0.46 and 1.16 ms at 128 x 129 x 128
+        // (now 0.37 and 0.98)
         static const int uniq[9] = {0, 1, 2, 1, 4, 5, 2, 5, 8};
-        for (int m = 0; m < 9; ++m) RET(add_in(S_C11 + m, KMM_C11 + (derived ? uniq[m] : m)));
+        for (int m = 0; m < 9; ++m) {
+            if (derived && lean && uniq[m] != m) A.slot_of_in[S_C11 + m] = A.slot_of_in[S_C11 + uniq[m]];
+            else RET(add_in(S_C11 + m, KMM_C11 + (derived ? uniq[m] : m)));
+        }
         for (int m = 0; m < 27; ++m) {
             const int ij = m / 3, k = m % 3;
+            if (lean && uniq[ij] != ij) continue;
             if (!derived) RET(add_in(S_DC111 + m, KMM_DC111 + m));
             else if (k == 1) RET(add_in(S_DC111 + m, KMM_DC111 + 3 * uniq[ij] + 1));
             else RET(add_in_from(S_DC111 + m, KMM_C11 + uniq[ij], k == 0 ? 1 : 2));
@@ -1412,8 +1440,8 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     if (poly) {
         for (int m = 0; m < 6; ++m) RET(add_out(O_C11N + m, KMM_C11N + m));
         for (int m = 0; m < 6; ++m) RET(add_out(O_STR11N + m, KMM_STR11N + m));
-        static const int qq[6] = {KMM_QP11, KMM_QP12, KMM_QP13, KMM_QP22, KMM_QP23, KMM_QP33};
-        for (int m = 0; m < 6; ++m) RET(add_out(O_QP11 + m, qq[m]));
+        if (!qp_scaled)
+            for (int m = 0; m < 6; ++m) RET(add_out(O_QP11 + m, kQpOut[m]));
     }
     // x derivatives formed in the x stage (with polymer, derived inputs and a compiled x stage:
     // k_xphys2 or the two-pass k_xinv_big2): every input i kx f whose f is also an input moves
@@ -1425,11 +1453,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
                              !(ctx->force_xbig && ctx->p.precision == 0)) ||
                             mx == 576;
     if (derived && poly && x_compiled) {
-        int slot_at[MAXIO];
-        for (int i = 0; i < nin; ++i) slot_at[i] = -1;
-        for (int sl = 0; sl < S_NSLOT; ++sl)
-            if (A.slot_of_in[sl] >= 0) slot_at[A.slot_of_in[sl]] = sl;
-        int order[MAXIO], no = 0;
+        int order[MAXIO], at[MAXIO], no = 0;   // at: an input's new place
         bool used[MAXIO], odd_x[MAXIO];
         for (int i = 0; i < nin; ++i) used[i] = odd_x[i] = false;
         for (int d = 0; d < nin; ++d) {
@@ -1450,10 +1474,12 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
             const int old = order[pos];
             z2.base[pos] = zr.base[old];
             z2.mult[pos] = zr.mult[old];
-            if (slot_at[old] >= 0) A.slot_of_in[slot_at[old]] = pos;
+            at[old] = pos;
             xform[pos] = odd_x[pos];
         }
         zr = z2;
+        for (int sl = 0; sl < S_NSLOT; ++sl)
+            if (A.slot_of_in[sl] >= 0) A.slot_of_in[sl] = at[A.slot_of_in[sl]];
     }
     // the z inverse's outputs (the inputs not formed in the x stage, compacted) and the x stage's rows
     int nq = 0;
@@ -1797,6 +1823,17 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
                     ctx->pl_out, outp, ctx->py2, ctx->py2.tw, nyp, nz, nxh, ncols);
             CKL();
         }
+    }
+    if (qp_scaled) {
+        StrQp L;
+        for (int m = 0; m < 6; ++m) {
+            L.s[m] = SPEC(ctx, KMM_STR11N + m);
+            L.q[m] = SPEC(ctx, kQpOut[m]);
+            if (!L.s[m] || !L.q[m]) return KMM_ERR_NOMEM;
+        }
+        const double zb = (1.0 - A.qbeta) / (A.re * A.qbeta * A.tpoly);
+        k_qp_scale<<<dim3(kmm_blocks(ctx->nspec, 256), 6), 256, 0, ctx->stream>>>(L, ctx->nspec, zb);
+        CKL();
     }
     kmm_toc(ctx, KMM_STAGE_DCT_BWD);
 
