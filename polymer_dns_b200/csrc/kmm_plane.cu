@@ -27,7 +27,13 @@
 #define MAXIO 64
 
 struct FieldPtrs { const double2 *p[MAXIO]; };
-struct FieldPtrsW { double2 *p[MAXIO]; };
+// outputs of the y back transform; output twin0 + m, m < 6, is also stored times zb at twin[m]
+struct FieldPtrsW {
+    double2 *p[MAXIO];
+    double2 *twin[6];
+    unsigned twin0 = MAXIO;
+    double zb;
+};
 
 // Block FFT buffers.  At the compiled lengths each of the 8 warps owns NQ = NB / 8 consecutive
 // sequences, stored conflict-free (fpos<C>, kmm_fft.cuh) within the warp's region, and the warps'
@@ -1088,12 +1094,14 @@ __global__ void __launch_bounds__(256) k_dct_bwd(const C *__restrict__ pl, const
     __syncthreads();
     C *r = fft_block<C, -1, DCT_CB>(P, a, b, tw, L);
     double2 *dst = out.p[f] + (size_t)col0 * nyp;
+    double2 *twin = f - out.twin0 < 6 ? out.twin[f - out.twin0] + (size_t)col0 * nyp : NULL;
     for (int e = threadIdx.x; e < ncb * nyp; e += blockDim.x) {
         const int c = e / nyp, i = e - c * nyp;
         const C rv = r[fb_at<C, DCT_CB>(c, i, L, ct)];
         double2 v = make_double2((double)rv.x / (double)ny, (double)rv.y / (double)ny);
         if (i == 0 || i == ny) v = make_double2(v.x / 2.0, v.y / 2.0);
         dst[e] = v;
+        if (twin) twin[e] = cscale(v, out.zb);
     }
 }
 
@@ -1133,12 +1141,14 @@ __global__ void __launch_bounds__(256) k_dct_bwd_h(const C *__restrict__ pl, con
     if (c < ncb) dct1_half<C, N>(xs + c * NYP, a + c * (flen<C>(N) + FB_PAD), b + c * (flen<C>(N) + FB_PAD), tw);
     __syncthreads();
     double2 *dst = out.p[f] + (size_t)col0 * NYP;
+    double2 *twin = f - out.twin0 < 6 ? out.twin[f - out.twin0] + (size_t)col0 * NYP : NULL;
     for (int e = threadIdx.x; e < ncb * NYP; e += blockDim.x) {
         const C rv = xs[e];
         const int i = e % NYP;
         double2 v = make_double2((double)rv.x / (double)N, (double)rv.y / (double)N);
         if (i == 0 || i == N) v = make_double2(v.x / 2.0, v.y / 2.0);
         dst[e] = v;
+        if (twin) twin[e] = cscale(v, out.zb);
     }
 }
 
@@ -1190,18 +1200,6 @@ static int dct_h_bwd(kmm_ctx *ctx, int nf, const C *pl, const FieldPtrsW &out, c
     default: return KMM_ERR_UNSUPPORTED;
     }
 #undef DH
-}
-
-// qp = zb str for the six components (blockIdx.y)
-struct StrQp {
-    const double2 *s[6];
-    double2 *q[6];
-};
-__global__ void k_qp_scale(StrQp L, size_t n, double zb) {
-    const double2 *__restrict__ s = L.s[blockIdx.y];
-    double2 *__restrict__ q = L.q[blockIdx.y];
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-        q[e] = cscale(s[e], zb);
 }
 
 // ---------------------------------------------------------------------------
@@ -1345,8 +1343,8 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     // FP64 only: two fields share each transform along x, so that another set of fields changes the last bits of
     // all, which the mixed form's FP32 transforms amplify to the rounding floor of fn (4e-4 at 96 x 97 x 96)
     const bool lean = ctx->p.precision == 0;
-    // qp_ij = (1 - beta) / (re beta tpoly) str_ij with a constant beta (itarget = 0): formed from str_ij's
-    // coefficients at the end instead of being transformed
+    // qp_ij = (1 - beta) / (re beta tpoly) str_ij with a constant beta (itarget = 0): stored beside str_ij's
+    // coefficients by the y back transform instead of being transformed itself
     const bool qp_scaled = poly && lean && ctx->p.itarget == 0;
     static const int kQpOut[6] = {KMM_QP11, KMM_QP12, KMM_QP13, KMM_QP22, KMM_QP23, KMM_QP33};
     PhysArgs A;
@@ -1443,8 +1441,13 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     if (poly) {
         for (int m = 0; m < 6; ++m) RET(add_out(O_C11N + m, KMM_C11N + m));
         for (int m = 0; m < 6; ++m) RET(add_out(O_STR11N + m, KMM_STR11N + m));
-        if (!qp_scaled)
+        if (qp_scaled) {
+            outp.twin0 = (unsigned)A.slot_of_out[O_STR11N];
+            for (int m = 0; m < 6; ++m)
+                if (!(outp.twin[m] = SPEC(ctx, kQpOut[m]))) return KMM_ERR_NOMEM;
+        } else {
             for (int m = 0; m < 6; ++m) RET(add_out(O_QP11 + m, kQpOut[m]));
+        }
     }
     // x derivatives formed in the x stage (with polymer, derived inputs and a compiled x stage:
     // k_xphys2 or the two-pass k_xinv_big2): every input i kx f whose f is also an input moves
@@ -1522,6 +1525,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     A.ugain = ctx->ugain;
     A.zl2 = ctx->p.zlmax * ctx->p.zlmax;
     A.qbeta = ctx->p.qbeta;
+    if (qp_scaled) outp.zb = (1.0 - A.qbeta) / (ctx->re * A.qbeta * ctx->p.tpoly);
     A.alpha_poly = ctx->p.alpha_poly;
     A.re = ctx->re;
     A.tpoly = ctx->p.tpoly;
@@ -1826,17 +1830,6 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
                     ctx->pl_out, outp, ctx->py2, ctx->py2.tw, nyp, nz, nxh, ncols);
             CKL();
         }
-    }
-    if (qp_scaled) {
-        StrQp L;
-        for (int m = 0; m < 6; ++m) {
-            L.s[m] = SPEC(ctx, KMM_STR11N + m);
-            L.q[m] = SPEC(ctx, kQpOut[m]);
-            if (!L.s[m] || !L.q[m]) return KMM_ERR_NOMEM;
-        }
-        const double zb = (1.0 - A.qbeta) / (A.re * A.qbeta * A.tpoly);
-        k_qp_scale<<<dim3(kmm_blocks(ctx->nspec, 256), 6), 256, 0, ctx->stream>>>(L, ctx->nspec, zb);
-        CKL();
     }
     kmm_toc(ctx, KMM_STAGE_DCT_BWD);
 
