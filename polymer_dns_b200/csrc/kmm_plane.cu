@@ -1419,7 +1419,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
         // c_ij and dc_ijk = d c_ij / d x_k; c21 = c12, c31 = c13, c32 = c23 (copied by the step)
         // (those share one input; the pointwise terms read dc_ijk of the six distinct components only): 42 inputs
         // with the scalar instead of 55, whose z inverse and x stage took 0.46 and 1.16 ms at 128 x 129 x 128
-        // (now 0.37 and 0.98)
+        // (now 0.37 and 0.95)
         static const int uniq[9] = {0, 1, 2, 1, 4, 5, 2, 5, 8};
         for (int m = 0; m < 9; ++m) {
             if (derived && lean && uniq[m] != m) A.slot_of_in[S_C11 + m] = A.slot_of_in[S_C11 + uniq[m]];
