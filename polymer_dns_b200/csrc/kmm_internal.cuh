@@ -198,7 +198,7 @@ int kmm_internal_cderiv(kmm_ctx *ctx, const double2 *f, double2 *df);
 int kmm_internal_cderiv_many(kmm_ctx *ctx, const double2 *const *f, double2 *const *df, int n);
 int kmm_internal_norm(kmm_ctx *ctx, double2 *a);
 // norm of nf distinct fields, KMM_NORM_BATCH to a launch (the same values as one call per field)
-#define KMM_NORM_BATCH 32
+#define KMM_NORM_BATCH 36
 int kmm_internal_norm_many(kmm_ctx *ctx, double2 *const *a, int nf);
 int kmm_internal_wallderiv(kmm_ctx *ctx, const double2 *f, int order, int wall, double2 *out, int iy);
 int kmm_internal_solve(kmm_ctx *ctx, double2 *u, double g, int ib, const double2 *bct, const double2 *bcb);

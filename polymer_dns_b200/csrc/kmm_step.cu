@@ -164,6 +164,14 @@ static int poly_norm_c(kmm_ctx *ctx) { return norm_range(ctx, KMM_C11, 9); }
 
 static int poly_norm_dc(kmm_ctx *ctx) { return norm_range(ctx, KMM_DC111, 27); }
 
+// the norms of one place in the step as one launch (a launch of k_norm takes 3 us whatever its list; a polymer
+// step's 17 launches were 57 us; with 9 the step of 128 x 129 x 128 takes 3.30 ms instead of 3.33)
+struct NormIds {
+    int id[KMM_NORM_BATCH], n;
+    void add(int f) { id[n++] = f; }
+    void range(int f, int c) { for (int m = 0; m < c; ++m) add(f + m); }
+};
+
 static int poly_norm_out(kmm_ctx *ctx) {
     RET(poly_norm_c(ctx));
     RET(norm_range(ctx, KMM_C11N, 6));
@@ -456,14 +464,19 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     CKL();
     RET(kmm_copy(ctx, KMM_H1NM1, KMM_H1N));
     RET(kmm_copy(ctx, KMM_H3NM1, KMM_H3N));
-    { static const int l[2] = {KMM_V, KMM_OMY}; RET(norm_ids(ctx, l, 2)); }
+    // with derived inputs vcw3dp forms the x and z derivatives itself (in its z inverse): only the
+    // y derivatives are computed here, in one batched cderiv launch
+    const bool derived = kmm_derived_inputs(ctx);
+    {
+        NormIds l = {{KMM_V, KMM_OMY}, 2};
+        if (ctx->p.scalar_on) l.add(KMM_SCALAR);
+        if (ctx->p.polymer_on && derived) l.range(KMM_C11, 9);   // derivscji takes c_ij before its norm
+        RET(norm_ids(ctx, l.id, l.n));
+    }
     RET(kmm_veloc(ctx));
     { static const int l[2] = {KMM_U, KMM_W}; RET(norm_ids(ctx, l, 2)); }
     RET(kmm_vort(ctx));
     { static const int l[2] = {KMM_OMX, KMM_OMZ}; RET(norm_ids(ctx, l, 2)); }
-    // with derived inputs vcw3dp forms the x and z derivatives itself (in its z inverse): only the
-    // y derivatives are computed here, in one batched cderiv launch
-    const bool derived = kmm_derived_inputs(ctx);
     const double2 *dsrc[KMM_CDERIV_BATCH];
     double2 *ddst[KMM_CDERIV_BATCH];
     int nd = 0;
@@ -476,7 +489,6 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
         return KMM_OK;
     };
     if (ctx->p.scalar_on) {
-        RET(kmm_norm(ctx, KMM_SCALAR));
         if (derived) {
             RET(want_dy(KMM_SCALAR, KMM_SCLY));
         } else {
@@ -502,7 +514,6 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     }
     if (ctx->p.polymer_on) {
         if (derived) {
-            RET(poly_norm_c(ctx));
             static const int uq[6] = {0, 1, 2, 4, 5, 8};   // c11 c12 c13 c22 c23 c33
             for (int m = 0; m < 6; ++m) RET(want_dy(KMM_C11 + uq[m], KMM_DC111 + 3 * uq[m] + 1));
         } else {
@@ -521,10 +532,18 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     ctx->in_step = 0;
     if (st != KMM_OK) return st;
     kmm_tic(ctx);
-    { static const int l[5] = {KMM_V, KMM_OMY, KMM_FN, KMM_GN, KMM_OMZ}; RET(norm_ids(ctx, l, 5)); }
-    if (ctx->p.scalar_on) { static const int l[2] = {KMM_SCALAR, KMM_SCN}; RET(norm_ids(ctx, l, 2)); }
+    {
+        NormIds l = {{KMM_V, KMM_OMY, KMM_FN, KMM_GN, KMM_OMZ}, 5};
+        if (ctx->p.scalar_on) { l.add(KMM_SCALAR); l.add(KMM_SCN); }
+        if (ctx->p.polymer_on && it >= ctx->p.src_start - 1) {
+            l.range(KMM_C11, 9);
+            l.range(KMM_C11N, 6);
+            l.range(KMM_STR11N, 6);
+            for (int m = 0; m < 6; ++m) l.add(kQp[m]);
+        }
+        RET(norm_ids(ctx, l.id, l.n));
+    }
     if (ctx->p.polymer_on) {
-        if (it >= ctx->p.src_start - 1) RET(poly_norm_out(ctx));
         if (it >= ctx->p.src_start) {
             RET(kmm_polyforce(ctx));
             static const int l[3] = {KMM_T1, KMM_T2, KMM_T3};
@@ -538,8 +557,7 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     CKL();
     { static const int l[3] = {KMM_FN, KMM_GN, KMM_OMZ}; RET(norm_ids(ctx, l, 3)); }
     RET(kmm_nonlin(ctx));
-    { static const int l[2] = {KMM_FN, KMM_GN}; RET(norm_ids(ctx, l, 2)); }
-    if (ctx->p.scalar_on) RET(kmm_norm(ctx, KMM_SCN));
+    { static const int l[3] = {KMM_FN, KMM_GN, KMM_SCN}; RET(norm_ids(ctx, l, ctx->p.scalar_on ? 3 : 2)); }
     kmm_toc(ctx, KMM_STAGE_POST);
     return KMM_OK;
 }
