@@ -54,7 +54,7 @@ struct kmm_ctx {
     int device;
     cudaStream_t stream;
     cudaStream_t side;           // fused step: the tracers run here, overlapping the z-forward and back stages
-    cudaStream_t side2;          // fused step: with `side`, the scalar and omega_y column kernels beside v's
+    cudaStream_t side2;          // with `side`: fused step, the scalar and omega_y column kernels beside v's; routine step, u0 and w0
     cudaEvent_t fork_ev, join_ev, cfork_ev, cjoin_ev[2];
     // grid (grid_size.f90:1-47, run-time here)
     int nx, ny, nz, nyp, nym, nxh, nyh, nzh, nyhp, nyhm, mx, mz;

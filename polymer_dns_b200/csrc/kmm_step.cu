@@ -402,6 +402,16 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
             RET(kmm_copy(ctx, KMM_C32, KMM_C23));
         }
     }
+    // the u0 and w0 solves (each one block, a serial chain of 44 us at ny = 128) on the side streams, beside the
+    // column solves: they read and write only the mean profiles.  Behind those solves they added their length to
+    // the step (128 x 129 x 128 with polymer 3.30 ms, so 3.26)
+    CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+    CK(cudaStreamWaitEvent(ctx->side, ctx->fork_ev, 0));
+    CK(cudaStreamWaitEvent(ctx->side2, ctx->fork_ev, 0));
+    RET(kmm_internal_uzero(ctx, 3, ctx->side));
+    RET(kmm_internal_uzero(ctx, 1, ctx->side2));
+    CK(cudaEventRecord(ctx->cjoin_ev[0], ctx->side));
+    CK(cudaEventRecord(ctx->cjoin_ev[1], ctx->side2));
     // phirhs and its solves in one blocked kernel per field where compiled (every boundary value
     // is zero: phirhs zeroes bctop / bcbot, main_dns.f90:39, solvers.f90:670-671), else routine by
     // routine
@@ -452,14 +462,8 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     }
     RET(kmm_zero(ctx, KMM_BCTOP));   // as phirhs leaves them
     RET(kmm_zero(ctx, KMM_BCBOT));
-    // the u0 and w0 solves (each one block) side by side: w0's on the side stream
-    CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
-    CK(cudaStreamWaitEvent(ctx->side, ctx->fork_ev, 0));
-    RET(kmm_internal_uzero(ctx, 3, ctx->side));
-    RET(kmm_internal_uzero(ctx, 1, ctx->stream));
+    for (int e = 0; e < 2; ++e) CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[e], 0));   // u0, w0
     RET(kmm_flowrate_apply(ctx, ctx->stream));
-    CK(cudaEventRecord(ctx->join_ev, ctx->side));
-    CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
     k_zero_mean<<<1, 256, 0, ctx->stream>>>(SPEC(ctx, KMM_OMY), ctx->nyp);
     CKL();
     RET(kmm_copy(ctx, KMM_H1NM1, KMM_H1N));
