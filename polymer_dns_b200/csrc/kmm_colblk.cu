@@ -167,13 +167,14 @@ __device__ __forceinline__ bool bpair(BPair &P, int nz, int nzh, int nxh, const 
     return true;
 }
 
+// KEEP: dc/dy, c1, c2, u, w and omega_x go to their mirrors too (kmm_keeps_mirrors).
 // The forward column stage as four kernels, in this order (each reads only what the previous
 // ones have finished): scalar; omega_y (with the mean modes); v; u, w and the y-physical
 // outputs of the velocity.  Splitting keeps each kernel's registers and code small; the price
 // is one extra read of v and omega_y.
 
 // passive scalar (main_dns.f90:325-359): CN/AB2 right-hand side, Robin solve, norm, store; y-physical c, dc/dy
-template <int K, typename C>
+template <int K, typename C, bool KEEP>
 __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_scl(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                             const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_scl(C
     // one column variable live through each transform (the register-resident FFT needs the rest)
     bdct_store<K, C>(s, fa, fb, tw, (C *)A.yp + 6 * fstride + yoff);
     bcderiv<K>(d1, s, A.dyde, FULL);
+    if (KEEP) bstore_s<K>(A.kscly + P.off, d1, wsm);
     bdct_store<K, C>(d1, fa, fb, tw, (C *)A.yp + 7 * fstride + yoff);
 }
 
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::omy) k_bcol_omy(C
 
 // wall-normal velocity (main_dns.f90:363-407, 426-466, 489-502, 520): phi, phirhs, Helmholtz and
 // Poisson solves, influence-matrix correction, norm, store; y-physical v
-template <int K, typename C>
+template <int K, typename C, bool KEEP>
 __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::v) k_bcol_v(ColFwdArgs A, FusedTabs T, const double *__restrict__ rj,
                                                           const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
@@ -318,6 +320,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::v) k_bcol_v(ColFw
         }
         const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[P.col]), cmul(wt, A.dnv2b[P.col])), A.denom[P.col]);
         const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[P.col]), cmul(wb, A.dnv1t[P.col])), A.denom[P.col]);
+        if (KEEP && bl_t() == 0) { A.kc1[P.col] = c1; A.kc2[P.col] = c2; }
         BCol<K> gfa;
         bload_s<K>(gfa, A.gf1 + P.off, wsm);
 #pragma unroll
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::v) k_bcol_v(ColFw
 }
 
 // veloc (solvers.f90:1576-1659) from the new v and omega_y; y-physical u, du/dy, w, dw/dy
-template <int K, typename C>
+template <int K, typename C, bool KEEP>
 __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_uw(ColFwdArgs A, const C *__restrict__ tw) {
     constexpr int NY = 16 * K, NYP = NY + 1;
     constexpr unsigned FULL = 0xffffffffu;
@@ -389,9 +392,16 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::fwd) k_bcol_uw(Co
 #pragma unroll
             for (int m = 0; m <= K; ++m) x.v[m] = zero;
         }
+        if (KEEP) bstore_s<K>((which == 0 ? A.ku : A.kw) + P.off, x, wsm);
         bdct_store<K, C>(x, fa, fb, tw, (C *)A.yp + (which == 0 ? 0 : 2) * fstride + yoff);
         BCol<K> d1;
         bcderiv<K>(d1, x, A.dyde, FULL);
+        if (KEEP && which == 1) {   // omega_x = dw/dy - i kz v (vort, solvers.f90:1663-1722)
+            bload_s<K>(x, A.v + P.off, wsm);
+#pragma unroll
+            for (int m = 0; m <= K; ++m) x.v[m] = csub(d1.v[m], cimul(x.v[m], kzv));
+            bstore_s<K>(A.komx + P.off, x, wsm);
+        }
         bdct_store<K, C>(d1, fa, fb, tw, (C *)A.yp + (which == 0 ? 4 : 5) * fstride + yoff);
     }
 }
@@ -567,13 +577,13 @@ int kmm_colblk_fwd(kmm_ctx *ctx, const ColFwdArgs &A, const FusedTabs &T, const 
     CK(cudaEventRecord(ctx->cfork_ev, ctx->stream));
     CK(cudaStreamWaitEvent(s_omy, ctx->cfork_ev, 0));
     if (A.scalar) CK(cudaStreamWaitEvent(s_scl, ctx->cfork_ev, 0));
-#define BF(KK, CC)                                                                                    \
+#define BF(KK, CC, KP)                                                                                    \
     do {                                                                                              \
         const CC *twc = (const CC *)tw;                                                               \
         const size_t smem = (size_t)CB_WARPS * CbSmem<KK, CC>::warp_bytes;                            \
         if (A.scalar) {                                                                               \
-            RET(kmm_smem_attr(ctx, (const void *)k_bcol_scl<KK, CC>, smem));                          \
-            k_bcol_scl<KK, CC><<<nblk, CB_WARPS * 32, smem, s_scl>>>(A, T, rj, twc);                   \
+            RET(kmm_smem_attr(ctx, (const void *)k_bcol_scl<KK, CC, KP>, smem));                          \
+            k_bcol_scl<KK, CC, KP><<<nblk, CB_WARPS * 32, smem, s_scl>>>(A, T, rj, twc);                   \
             CKL();                                                                                    \
             CK(cudaEventRecord(ctx->cjoin_ev[0], s_scl));                                             \
         }                                                                                             \
@@ -582,30 +592,39 @@ int kmm_colblk_fwd(kmm_ctx *ctx, const ColFwdArgs &A, const FusedTabs &T, const 
         CKL();                                                                                        \
         RET(kmm_flowrate_apply(ctx, s_omy));   /* u0 comes from this kernel's mean pair */              \
         CK(cudaEventRecord(ctx->cjoin_ev[1], s_omy));                                                 \
-        RET(kmm_smem_attr(ctx, (const void *)k_bcol_v<KK, CC>, smem));                                \
-        k_bcol_v<KK, CC><<<nblk, CB_WARPS * 32, smem, ctx->stream>>>(A, T, rj, twc);                   \
+        RET(kmm_smem_attr(ctx, (const void *)k_bcol_v<KK, CC, KP>, smem));                                \
+        k_bcol_v<KK, CC, KP><<<nblk, CB_WARPS * 32, smem, ctx->stream>>>(A, T, rj, twc);                   \
         CKL();                                                                                        \
         if (A.scalar) CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[0], 0));                      \
         CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[1], 0));                                    \
-        RET(kmm_smem_attr(ctx, (const void *)k_bcol_uw<KK, CC>, smem));                               \
-        k_bcol_uw<KK, CC><<<dim3(nblk, 2), CB_WARPS * 32, smem, ctx->stream>>>(A, twc);                \
+        RET(kmm_smem_attr(ctx, (const void *)k_bcol_uw<KK, CC, KP>, smem));                               \
+        k_bcol_uw<KK, CC, KP><<<dim3(nblk, 2), CB_WARPS * 32, smem, ctx->stream>>>(A, twc);                \
         CKL();                                                                                        \
         return KMM_OK;                                                                                \
     } while (0)
     if (fp32) {
         switch (K) {
-        case 2: BF(2, float2);
-        case 4: BF(4, float2);
-        case 6: BF(6, float2);
-        case 8: BF(8, float2);
+        case 2: BF(2, float2, false);
+        case 4: BF(4, float2, false);
+        case 6: BF(6, float2, false);
+        case 8: BF(8, float2, false);
+        default: return KMM_ERR_UNSUPPORTED;
+        }
+    }
+    if (A.ku) {   // a run-time length in x: the mirrors too
+        switch (K) {
+        case 2: BF(2, double2, true);
+        case 4: BF(4, double2, true);
+        case 6: BF(6, double2, true);
+        case 8: BF(8, double2, true);
         default: return KMM_ERR_UNSUPPORTED;
         }
     }
     switch (K) {
-    case 2: BF(2, double2);
-    case 4: BF(4, double2);
-    case 6: BF(6, double2);
-    case 8: BF(8, double2);
+    case 2: BF(2, double2, false);
+    case 4: BF(4, double2, false);
+    case 6: BF(6, double2, false);
+    case 8: BF(8, double2, false);
     default: return KMM_ERR_UNSUPPORTED;
     }
 #undef BF

@@ -614,6 +614,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         col_norm<E>(s, xbuf, kx, j, A.nzh);
         col_store<E>(A.scal + off, s, nyp);
         col_cderiv<E>(n1, s, nyp, A.dyde);
+        if (A.kscly) col_store<E>(A.kscly + off, n1, nyp);
         col_dct<E, L0>(s, fa, fb, P, nyp, true);
         col_store<E>(A.yp + 6 * ncols * nyp + off, s, nyp);
         col_dct<E, L0>(n1, fa, fb, P, nyp, true);
@@ -659,6 +660,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         }
 #pragma unroll
         for (int e = 0; e < E; ++e) v.v[e] = om.v[e] = make_double2(0.0, 0.0);
+        if (A.kc1 && lane == 0) A.kc1[col] = A.kc2[col] = make_double2(0.0, 0.0);
         __syncthreads();   // warp 0 reads w0 below
     } else {
         // ---- wall-normal velocity: phi, phirhs, Helmholtz + Poisson (main_dns.f90:363-407)
@@ -704,6 +706,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
             }
             const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[col]), cmul(wt, A.dnv2b[col])), A.denom[col]);
             const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[col]), cmul(wb, A.dnv1t[col])), A.denom[col]);
+            if (A.kc1 && lane == 0) { A.kc1[col] = c1; A.kc2[col] = c2; }
             Col<E> gfa;
             col_load<E>(gfa, A.gf1 + off, nyp);
 #pragma unroll
@@ -765,6 +768,10 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
     }
     col_store<E>(A.v + off, v, nyp);
     col_store<E>(A.omy + off, om, nyp);
+    if (A.ku) {
+        col_store<E>(A.ku + off, u, nyp);
+        col_store<E>(A.kw + off, w, nyp);
+    }
     // ---- y-physical outputs: u, v, w, omega_y, du/dy, dw/dy [, c, dc/dy]
     double2 *yp = A.yp;
     col_dct<E, L0>(v, fa, fb, P, nyp, true);
@@ -777,6 +784,13 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
     col_dct<E, L0>(d1, fa, fb, P, nyp, true);
     col_store<E>(yp + 4 * ncols * nyp + off, d1, nyp);
     col_cderiv<E>(d1, w, nyp, A.dyde);
+    if (A.komx) {   // omega_x = dw/dy - i kz v (vort, solvers.f90:1663-1722)
+        Col<E> ox;
+        col_load<E>(ox, A.v + off, nyp);
+#pragma unroll
+        for (int e = 0; e < E; ++e) ox.v[e] = csub(d1.v[e], cimul(ox.v[e], kzv));
+        col_store<E>(A.komx + off, ox, nyp);
+    }
     col_dct<E, L0>(w, fa, fb, P, nyp, true);
     col_store<E>(yp + 2 * ncols * nyp + off, w, nyp);
     col_dct<E, L0>(d1, fa, fb, P, nyp, true);
@@ -1332,7 +1346,6 @@ static int fused_launch(kmm_ctx *ctx) {
         kmm_set_error(ctx, "mixed precision needs nx, ny, nz in {32, 64, 96, 128} and the blocked column kernels");
         return KMM_ERR_UNSUPPORTED;
     }
-    ctx->it += 1;
 
     // history copies fnm1 = fn, gnm1 = gn, scnm1 = scn become pointer swaps: the kernels read the
     // old n / n-1 fields and the new n fields are written into the swapped-out buffers
@@ -1348,12 +1361,19 @@ static int fused_launch(kmm_ctx *ctx) {
     F.dnv1b = SPEC(ctx, KMM_DNV1B); F.dnv1t = SPEC(ctx, KMM_DNV1T); F.dnv2b = SPEC(ctx, KMM_DNV2B);
     F.dnv2t = SPEC(ctx, KMM_DNV2T); F.denom = SPEC(ctx, KMM_DENOM);
     F.u0 = REAL(ctx, KMM_U0); F.w0 = REAL(ctx, KMM_W0); F.h1n = REAL(ctx, KMM_H1N); F.h1nm1 = REAL(ctx, KMM_H1NM1);
-    F.h3n = REAL(ctx, KMM_H3N); F.h3nm1 = REAL(ctx, KMM_H3NM1); F.scratch = ctx->d_scratch;
+    F.h3n = REAL(ctx, KMM_H3N); F.h3nm1 = REAL(ctx, KMM_H3NM1);
+    if (kmm_keeps_mirrors(ctx)) {
+        F.ku = SPEC(ctx, KMM_U); F.kw = SPEC(ctx, KMM_W); F.komx = SPEC(ctx, KMM_OMX);
+        F.kc1 = SPEC(ctx, KMM_C1); F.kc2 = SPEC(ctx, KMM_C2);
+        F.kscly = scalar ? SPEC(ctx, KMM_SCLY) : NULL;
+        if (!F.ku || !F.kw || !F.komx || !F.kc1 || !F.kc2 || (scalar && !F.kscly)) return KMM_ERR_NOMEM;
+    }
     F.yp = g_yp; F.wavx = ctx->d_wavx; F.wavz = ctx->d_wavz;
     F.nz = nz; F.nxh = nxh; F.nyp = nyp; F.nzh = ctx->nzh; F.scalar = scalar; F.nb = ctx->nb; F.nt = ctx->nt;
     F.re = ctx->re; F.dt = ctx->dt; F.th = ctx->theta; F.dyde = ctx->dyde; F.diff = ctx->p.diff; F.c0 = ctx->h_c[0];
     F.atu = ctx->atu; F.btu = ctx->btu; F.gtu = ctx->gtu; F.abu = ctx->abu; F.bbu = ctx->bbu; F.gbu = ctx->gbu;
     F.atw = ctx->atw; F.gtw = ctx->gtw; F.abw = ctx->abw; F.bbw = ctx->bbw; F.gbw = ctx->gbw;
+    ctx->it += 1;
     const int E = (nyp + 31) / 32;
     const size_t smc = sizeof(double2) * (64 * (size_t)E + 2 * 2 * 2 * (size_t)ctx->ny);
     const int nblk = (int)(ncols / 2);
@@ -1435,12 +1455,14 @@ static int fused_launch(kmm_ctx *ctx) {
     kmm_toc(ctx, KMM_STAGE_ZFFT_BWD);
     // x transforms + products
     double *up3 = NULL, *vp3 = NULL, *wp3 = NULL;
-    if (ctx->p.npart > 0) { up3 = REAL(ctx, KMM_UP3D); vp3 = REAL(ctx, KMM_VP3D); wp3 = REAL(ctx, KMM_WP3D); }
+    const bool save = ctx->p.npart > 0 || !kmm_compiled_mx(ctx);
+    if (save) { up3 = REAL(ctx, KMM_UP3D); vp3 = REAL(ctx, KMM_VP3D); wp3 = REAL(ctx, KMM_WP3D); }
+    if (save && (!up3 || !vp3 || !wp3)) return KMM_ERR_NOMEM;
     kmm_tic(ctx);
     {
         const int xst = kmm_fast_x2(ctx, g_q, g_r, f32 ? (const void *)FU->twf_mx : (const void *)ctx->wmx.tw, f32,
-                                    scalar ? 6 : -1, nout, ctx->p.npart > 0, up3, vp3, wp3);
-        if (xst == KMM_ERR_UNSUPPORTED) RET(kmm_fast_x(ctx, g_q, g_r, scalar ? 6 : -1, nout, ctx->p.npart > 0, up3, vp3, wp3));
+                                    scalar ? 6 : -1, nout, save, up3, vp3, wp3);
+        if (xst == KMM_ERR_UNSUPPORTED) RET(kmm_fast_x(ctx, g_q, g_r, scalar ? 6 : -1, nout, save, up3, vp3, wp3));
         else RET(xst);
     }
     kmm_toc(ctx, KMM_STAGE_XPHYS);

@@ -45,8 +45,10 @@ static __device__ __forceinline__ TauTab tab_at(const FusedTabs &T, int c, int c
 struct ColFwdArgs {
     double2 *v, *omy, *fn, *fnm1, *gn, *gnm1, *scal, *scn, *scnm1;
     const double2 *gf1, *gf2, *dnv1b, *dnv1t, *dnv2b, *dnv2t, *denom;
-    double *u0, *w0, *h1n, *h1nm1, *h3n, *h3nm1, *scratch;
+    double *u0, *w0, *h1n, *h1nm1, *h3n, *h3nm1;
     double2 *yp;      // y-physical outputs [8][ncols][nyp]
+    // mirrors the step also leaves current (kmm_keeps_mirrors; all NULL elsewhere): u, w, omega_x, dc/dy, c1, c2
+    double2 *ku, *kw, *komx, *kscly, *kc1, *kc2;
     const double *wavx, *wavz;
     int nz, nxh, nyp, nzh, scalar, nb, nt;
     double re, dt, th, dyde, diff, c0;

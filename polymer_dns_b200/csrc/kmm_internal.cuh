@@ -164,6 +164,15 @@ void kmm_fused_replayed(kmm_ctx *ctx, int parity);
 int kmm_fused_enqueue(kmm_ctx *ctx);
 void kmm_graph_release(kmm_ctx *ctx);
 bool kmm_fused_applicable(const kmm_ctx *ctx);
+// The grids on which the fused step leaves u, w, omega_x, dc/dy, c1, c2 and the 3/2-grid velocities in their
+// mirrors as the routine step does: those with a run-time length in y or x.  At the compiled lengths of both
+// it writes only what the next step reads (the mirrors would be 2 % of a step's traffic there).
+static inline bool kmm_compiled_mx(const kmm_ctx *ctx) {
+    return ctx->mx == 48 || ctx->mx == 96 || ctx->mx == 144 || ctx->mx == 192;
+}
+static inline bool kmm_keeps_mirrors(const kmm_ctx *ctx) {
+    return !(kmm_compiled_mx(ctx) && (ctx->ny == 32 || ctx->ny == 64 || ctx->ny == 96 || ctx->ny == 128));
+}
 // TMA forms of the z transforms, FP64 and FP32 (kmm_ztma.cu)
 bool kmm_ztma_supported(const kmm_ctx *ctx);
 int kmm_zb_tma(kmm_ctx *ctx, const double2 *yp, double2 *q, int nbase, int nq, const double2 *tw);

@@ -1668,7 +1668,7 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     bool fast_done = false, xstat = false;
     if (fast_x) {
         kmm_tic(ctx);
-        const bool save = ctx->p.npart > 0 || !ctx->in_step;
+        const bool save = ctx->p.npart > 0 || !ctx->in_step || !kmm_compiled_mx(ctx);
         const int fst = kmm_fast_x(ctx, ctx->q_in, ctx->q_out, scal ? A.slot_of_in[S_CX] : -1, nout, save, up3, vp3, wp3);
         if (fst == KMM_OK) fast_done = true;
         else if (fst != KMM_ERR_UNSUPPORTED) return fst;
