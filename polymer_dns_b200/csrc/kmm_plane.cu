@@ -1393,8 +1393,9 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     static const int fl[6] = {KMM_U, KMM_V, KMM_W, KMM_OMX, KMM_OMY, KMM_OMZ};
     for (int m = 0; m < 6; ++m) RET(add_in(S_U + m, fl[m]));
     if (scal) {
-        // the scalar itself enters only the polymer's beta of itarget = 1, 2
-        if (poly && (ctx->p.itarget != 0 || !lean)) RET(add_in(S_SC, KMM_SCALAR));
+        // the scalar itself enters only the polymer's beta of itarget = 1, 2 (a mixed context keeps its place
+        // in the pairs, as above)
+        if (!lean || (poly && ctx->p.itarget != 0)) RET(add_in(S_SC, KMM_SCALAR));
         if (derived) {
             RET(add_in_from(S_CX, KMM_SCALAR, 1));
             RET(add_in(S_CY, KMM_SCLY));
@@ -1593,9 +1594,11 @@ extern "C" int kmm_vcw3dp(kmm_ctx *ctx) {
     const bool xbig = (!mx_compiled && (sm_x + 1024 > 227 * 1024 || mx == 576)) ||
                       (ctx->force_xbig && ctx->p.precision == 0);
     // the fused x stage (kmm_fast_x): no polymer, no immersed boundary, no inertial particles, no particle
-    // or targeted scalar source, FP64
+    // or targeted scalar source, FP64 (at mx = 576 in FP64 contexts only: k_fx_row rounds the scalar term otherwise
+    // than the two-pass form, from which a mixed context's initial state keeps its bits)
     const bool f32 = ctx->p.precision == 1 && ctx->in_step;
-    const bool fast_x = !poly && !ib_any && !inertial && !(scal && ctx->p.scl_flag >= 2) && !f32;
+    const bool fast_x = !poly && !ib_any && !inertial && !(scal && ctx->p.scl_flag >= 2) && !f32 &&
+                        !(mx == 576 && ctx->p.precision == 1);
     if (xbig && fast_x && mx == 576) {
         // k_fx_row needs no buffer of the physical inputs
     } else if (xbig) {
