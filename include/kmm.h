@@ -371,6 +371,15 @@ int  kmm_set_option(kmm_ctx *ctx, int option, int value);
  * The context stays usable afterwards.                                                    */
 int  kmm_wait_selftest(kmm_ctx *ctx, double limit_ms);
 
+/* ---- failures injected on the host (no counterpart in the reference) --------------------
+ * For tests of the error paths; nothing fails on the device.  KMM_INJECT_NOMEM: the `value`-th
+ * allocation from now on among those made on first use by the fused step (tables, buffers) and by
+ * kmm_solve / kmm_penta / kmm_phirhs (tables) reports out of memory, as if the device were full
+ * (0: none).  Those paths then run their forms that need no such memory: the routine step (until
+ * KMM_OPT_FUSED is set again or kmm_initial is called) and the table-free solves.            */
+enum kmm_injection { KMM_INJECT_NOMEM = 1 };
+int  kmm_inject(kmm_ctx *ctx, int what, int value);
+
 /* ---- transform without device allocation --------------------------------------
  * kmm_xyzfft_noalloc has no counterpart in the reference.  It is kmm_xyzfft (the physical ->
  * spectral transform of an initial field, helpers.f90:6-87) for callers that cannot allocate

@@ -53,6 +53,23 @@ void *kmm_field_ptr(kmm_ctx *ctx, int f) {
     return p;
 }
 
+int kmm_dalloc(kmm_ctx *ctx, void **p, size_t bytes) {
+    *p = NULL;
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (!(ctx->inject_nomem > 0 && --ctx->inject_nomem == 0)) e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) return KMM_OK;
+    *p = NULL;
+    cudaGetLastError();
+    kmm_set_error(ctx, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
+    return e == cudaErrorMemoryAllocation ? KMM_ERR_NOMEM : KMM_ERR_CUDA;
+}
+
+extern "C" int kmm_inject(kmm_ctx *ctx, int what, int value) {
+    if (!ctx || what != KMM_INJECT_NOMEM || value < 0) return KMM_ERR_ARG;
+    ctx->inject_nomem = value;
+    return KMM_OK;
+}
+
 extern "C" int kmm_field_size(const kmm_ctx *ctx, int field, size_t *nelem, int *elem_bytes) {
     if (!ctx) return KMM_ERR_ARG;
     return kmm_field_info(ctx, field, nelem, elem_bytes);
@@ -479,10 +496,10 @@ int kmm_smem_attr(kmm_ctx *ctx, const void *func, size_t bytes) {
 extern "C" int kmm_set_option(kmm_ctx *ctx, int option, int value) {
     if (!ctx) return KMM_ERR_ARG;
     switch (option) {
-    case KMM_OPT_FUSED: ctx->use_fused = value ? 1 : 0; kmm_graph_release(ctx); return KMM_OK;
-    case KMM_OPT_COLUMN_BLOCKED: ctx->use_colblk = value ? 1 : 0; kmm_graph_release(ctx); return KMM_OK;
+    case KMM_OPT_FUSED: ctx->use_fused = value ? 1 : 0; ctx->fused_nomem = 0; ctx->fused_ran = 0; kmm_graph_release(ctx); return KMM_OK;
+    case KMM_OPT_COLUMN_BLOCKED: ctx->use_colblk = value ? 1 : 0; ctx->fused_ran = 0; kmm_graph_release(ctx); return KMM_OK;
     case KMM_OPT_GRAPH: ctx->use_graph = value ? 1 : 0; kmm_graph_release(ctx); return KMM_OK;
-    case KMM_OPT_ZTMA: ctx->use_ztma = value ? 1 : 0; kmm_graph_release(ctx); return KMM_OK;
+    case KMM_OPT_ZTMA: ctx->use_ztma = value ? 1 : 0; ctx->fused_ran = 0; kmm_graph_release(ctx); return KMM_OK;
     case KMM_OPT_XBIG: ctx->force_xbig = value ? 1 : 0; return KMM_OK;
     case KMM_OPT_TC_DCT: ctx->use_tcdct = value ? 1 : 0; return KMM_OK;
     case KMM_OPT_DERIVED_INPUTS: ctx->use_derived = value ? 1 : 0; return KMM_OK;

@@ -125,8 +125,9 @@ static int block_tables(kmm_ctx *ctx, const double *const src[4], double *dst[4]
     const int K = kmm_blocked_ny(ctx->ny) ? ctx->ny / 16 : 0;
     const size_t n = (size_t)ncols * ctx->nyp;
     const int nb = (int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-    for (int a = 0; a < 4; ++a) {
-        CK(cudaMalloc(&dst[a], sizeof(double) * n));
+    for (int a = 0; a < 4; ++a) dst[a] = NULL;
+    for (int a = 0; a < 4; ++a) {   // (the caller frees dst on failure)
+        RET(kmm_dalloc(ctx, (void **)&dst[a], sizeof(double) * n));
         k_tab_block<<<nb, 256, 0, ctx->stream>>>(src[a], dst[a], ncols, ctx->nyp, K, a == 0);
         CKL();
     }
@@ -150,9 +151,10 @@ static int upload_rj(kmm_ctx *ctx, double **out, bool blocked) {
     double *h = (double *)calloc(3 * (size_t)nyp, sizeof(double));
     if (!h) return KMM_ERR_NOMEM;
     rj_rows(h, nyp, blocked);
-    cudaError_t e = cudaMalloc(out, sizeof(double) * 3 * nyp);
-    if (e == cudaSuccess) e = cudaMemcpy(*out, h, sizeof(double) * 3 * nyp, cudaMemcpyHostToDevice);
+    const int st = kmm_dalloc(ctx, (void **)out, sizeof(double) * 3 * nyp);
+    const cudaError_t e = st == KMM_OK ? cudaMemcpy(*out, h, sizeof(double) * 3 * nyp, cudaMemcpyHostToDevice) : cudaSuccess;
     free(h);
+    RET(st);
     CK(e);
     return KMM_OK;
 }
@@ -161,22 +163,21 @@ static int upload_rj(kmm_ctx *ctx, double **out, bool blocked) {
 static int make_twf(kmm_ctx *ctx, int n, float2 **out) {
     const size_t nt = (size_t)kct::tw_total(n);
     float2 *h = (float2 *)malloc(sizeof(float2) * nt);
+    if (!h) return KMM_ERR_NOMEM;
     for (int k = 0; k < n; ++k) {
         const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
         h[k] = make_float2((float)cosl(a), -(float)sinl(a));
     }
     tw_pack(h, n);
-    cudaError_t e = cudaMalloc(out, sizeof(float2) * nt);
-    if (e == cudaSuccess) e = cudaMemcpy(*out, h, sizeof(float2) * nt, cudaMemcpyHostToDevice);
+    const int st = kmm_dalloc(ctx, (void **)out, sizeof(float2) * nt);
+    const cudaError_t e = st == KMM_OK ? cudaMemcpy(*out, h, sizeof(float2) * nt, cudaMemcpyHostToDevice) : cudaSuccess;
     free(h);
+    RET(st);
     CK(e);
     return KMM_OK;
 }
 
-static int build_tables(kmm_ctx *ctx) {
-    if (ctx->fused) return KMM_OK;
-    KmmFused *F = (KmmFused *)calloc(1, sizeof(KmmFused));
-    ctx->fused = F;
+static int fill_tables(kmm_ctx *ctx, KmmFused *F) {
     const int ncols = ctx->nz * ctx->nxh;
     const double g1 = ctx->re / (ctx->dt * ctx->theta);
     const double gs = ctx->re * ctx->p.diff / (ctx->dt * ctx->theta);
@@ -193,11 +194,9 @@ static int build_tables(kmm_ctx *ctx) {
     for (int c = 0; c < TB_N; ++c) {
         const int nc = (c == TB_U0 || c == TB_W0) ? 1 : ncols;   // the mean modes use column (0,0) only
         const size_t n = (size_t)nc * ctx->nyp;
-        CK(cudaMalloc(&T.td[c], sizeof(double) * n));
-        CK(cudaMalloc(&T.te[c], sizeof(double) * n));
-        CK(cudaMalloc(&T.tb1[c], sizeof(double) * n));
-        CK(cudaMalloc(&T.tb2[c], sizeof(double) * n));
-        CK(cudaMalloc(&T.tf[c], sizeof(double) * 4 * nc));
+        double **const tab[4] = {&T.td[c], &T.te[c], &T.tb1[c], &T.tb2[c]};
+        for (int a = 0; a < 4; ++a) RET(kmm_dalloc(ctx, (void **)tab[a], sizeof(double) * n));
+        RET(kmm_dalloc(ctx, (void **)&T.tf[c], sizeof(double) * 4 * nc));
         T.g[c] = cfg[c].g;
         k_tau_tables<<<(nc + 127) / 128, 128, 0, ctx->stream>>>(T.td[c], T.te[c], T.tb1[c], T.tb2[c], T.tf[c], cfg[c],
                                                                ctx->d_wavx, ctx->d_wavz, nc, ctx->nz, ctx->nyp,
@@ -211,8 +210,9 @@ static int build_tables(kmm_ctx *ctx) {
             const int nc = (c == TB_U0 || c == TB_W0) ? 1 : ncols;
             const double *src[4] = {T.td[c], T.te[c], T.tb1[c], T.tb2[c]};
             double *dst[4];
-            RET(block_tables(ctx, src, dst, nc));
+            const int st = block_tables(ctx, src, dst, nc);
             F->btabs.td[c] = dst[0]; F->btabs.te[c] = dst[1]; F->btabs.tb1[c] = dst[2]; F->btabs.tb2[c] = dst[3];
+            RET(st);
             F->btabs.tf[c] = T.tf[c];
             F->btabs.g[c] = T.g[c];
         }
@@ -221,23 +221,58 @@ static int build_tables(kmm_ctx *ctx) {
     for (int c = 0; c < TB_N; ++c) {   // the canonical pivots become 1 / d too (K = 0: positions kept)
         const size_t n = (size_t)((c == TB_U0 || c == TB_W0) ? 1 : ncols) * ctx->nyp;
         double *r = NULL;
-        CK(cudaMalloc(&r, sizeof(double) * n));
+        RET(kmm_dalloc(ctx, (void **)&r, sizeof(double) * n));
         k_tab_block<<<(int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184), 256, 0, ctx->stream>>>(T.td[c], r, (int)(n / ctx->nyp),
                                                                                                  ctx->nyp, 0, 1);
-        CKL();
-        CK(cudaFree(T.td[c]));
+        cudaFree(T.td[c]);
         T.td[c] = r;
+        CKL();
     }
     RET(make_twf(ctx, 2 * ctx->ny, &F->twf_y2));
     RET(make_twf(ctx, ctx->mz, &F->twf_mz));
     RET(make_twf(ctx, ctx->mx, &F->twf_mx));
     const size_t ncp = (size_t)ncols * ctx->nyp, nq = (size_t)ctx->nyp * ctx->mz * ctx->nxh;
-    CK(cudaMalloc(&F->yp, sizeof(double2) * ncp * 8));
-    CK(cudaMalloc(&F->q, sizeof(double2) * nq * 10));
-    CK(cudaMalloc(&F->r, sizeof(double2) * nq * 4));
-    CK(cudaMalloc(&F->yo, sizeof(double2) * ncp * 4));
-    CK(cudaMalloc(&F->acc, sizeof(double) * (2 * (size_t)ctx->nyp + 1)));
+    RET(kmm_dalloc(ctx, (void **)&F->yp, sizeof(double2) * ncp * 8));
+    RET(kmm_dalloc(ctx, (void **)&F->q, sizeof(double2) * nq * 10));
+    RET(kmm_dalloc(ctx, (void **)&F->r, sizeof(double2) * nq * 4));
+    RET(kmm_dalloc(ctx, (void **)&F->yo, sizeof(double2) * ncp * 4));
+    RET(kmm_dalloc(ctx, (void **)&F->acc, sizeof(double) * (2 * (size_t)ctx->nyp + 1)));
     CK(cudaMemsetAsync(F->acc, 0, sizeof(double) * (2 * (size_t)ctx->nyp + 1), ctx->stream));
+    return KMM_OK;
+}
+
+static void fused_free(KmmFused *F) {
+    for (int c = 0; c < TB_N; ++c) {
+        cudaFree(F->tabs.td[c]); cudaFree(F->tabs.te[c]); cudaFree(F->tabs.tb1[c]); cudaFree(F->tabs.tb2[c]);
+        cudaFree(F->tabs.tf[c]);
+        cudaFree(F->btabs.td[c]); cudaFree(F->btabs.te[c]); cudaFree(F->btabs.tb1[c]); cudaFree(F->btabs.tb2[c]);
+    }
+    cudaFree(F->yp); cudaFree(F->q); cudaFree(F->r); cudaFree(F->yo); cudaFree(F->acc); cudaFree(F->rj); cudaFree(F->brj);
+    cudaFree(F->twf_y2); cudaFree(F->twf_mz); cudaFree(F->twf_mx);
+    free(F);
+}
+
+// the tables and buffers belong to the context once they are complete: a build that fails leaves none behind
+static int build_tables(kmm_ctx *ctx) {
+    if (ctx->fused) return KMM_OK;
+    KmmFused *F = (KmmFused *)calloc(1, sizeof(KmmFused));
+    if (!F) return KMM_ERR_NOMEM;
+    const int st = fill_tables(ctx, F);
+    if (st != KMM_OK) {
+        fused_free(F);
+        return st;
+    }
+    ctx->fused = F;
+    return KMM_OK;
+}
+
+int kmm_fused_select(kmm_ctx *ctx, bool *fused) {
+    *fused = ctx->use_fused && kmm_fused_applicable(ctx);
+    if (!*fused || ctx->fused) return KMM_OK;
+    const int st = build_tables(ctx);
+    if (st != KMM_ERR_NOMEM) return st;
+    ctx->fused_nomem = 1;   // until KMM_OPT_FUSED is set again or kmm_initial starts another run
+    *fused = false;
     return KMM_OK;
 }
 
@@ -327,17 +362,9 @@ void kmm_tau_release(kmm_ctx *ctx) {
 }
 
 void kmm_fused_release(kmm_ctx *ctx) {
-    KmmFused *F = ctx->fused;
-    if (!F) return;
-    for (int c = 0; c < TB_N; ++c) {
-        cudaFree(F->tabs.td[c]); cudaFree(F->tabs.te[c]); cudaFree(F->tabs.tb1[c]); cudaFree(F->tabs.tb2[c]);
-        cudaFree(F->tabs.tf[c]);
-        cudaFree(F->btabs.td[c]); cudaFree(F->btabs.te[c]); cudaFree(F->btabs.tb1[c]); cudaFree(F->btabs.tb2[c]);
-    }
-    cudaFree(F->yp); cudaFree(F->q); cudaFree(F->r); cudaFree(F->yo); cudaFree(F->acc); cudaFree(F->rj); cudaFree(F->brj);
-    cudaFree(F->twf_y2); cudaFree(F->twf_mz); cudaFree(F->twf_mx);
-    free(F);
+    if (ctx->fused) fused_free(ctx->fused);
     ctx->fused = NULL;
+    ctx->fused_ran = 0;
 }
 
 
@@ -1139,7 +1166,7 @@ int kmm_tracers(kmm_ctx *ctx);
 // the fused path applies when: no polymer, no immersed boundary, Dirichlet-type velocity walls
 // (nb = nt = 1 or 2), nyp in the compiled register layouts, and the x transform instance exists
 bool kmm_fused_applicable(const kmm_ctx *ctx) {
-    if (ctx->p.polymer_on || ctx->f[KMM_IMATRIX] != NULL) return false;
+    if (ctx->p.polymer_on || ctx->f[KMM_IMATRIX] != NULL || ctx->fused_nomem) return false;
     // the flow-rate correction sits between the v and the u, w column kernels, which only the
     // blocked kernels (ny = 32, 64, 96, 128) launch separately
     const bool blocked = ctx->use_colblk && (ctx->ny == 32 || ctx->ny == 64 || ctx->ny == 96 || ctx->ny == 128);
@@ -1279,7 +1306,7 @@ static int capture_graphs(kmm_ctx *ctx) {
 // when the step is not replayed from a graph; *parity receives the arrangement
 int kmm_fused_graph_for_step(kmm_ctx *ctx, int *parity) {
     const bool graphable = ctx->use_fused && kmm_fused_applicable(ctx) && ctx->use_graph && !ctx->timing_on &&
-                           ctx->fused != NULL && ctx->it >= ctx->p.irstrt;
+                           ctx->fused_ran && ctx->it >= ctx->p.irstrt;
     if (!graphable) return -1;
     if (!ctx->graph_ready) RET(capture_graphs(ctx));
     *parity = ctx->f[KMM_FN] == ctx->g_fn0 ? 0 : 1;
@@ -1294,11 +1321,13 @@ void kmm_fused_replayed(kmm_ctx *ctx, int parity) {
 }
 
 int kmm_fused_enqueue(kmm_ctx *ctx) {
-    // graphs only after the step that initialises the tracers (it == irstrt) and the tau tables
-    const bool graphable = ctx->use_graph && !ctx->timing_on && ctx->fused != NULL && ctx->it >= ctx->p.irstrt;
+    // graphs only after the step that initialises the tracers (it == irstrt) and a step launched kernel by kernel
+    const bool graphable = ctx->use_graph && !ctx->timing_on && ctx->fused_ran && ctx->it >= ctx->p.irstrt;
     if (!graphable) {
         kmm_report_arm(ctx);
-        return kmm_fused_launch(ctx);
+        RET(kmm_fused_launch(ctx));
+        ctx->fused_ran = 1;
+        return KMM_OK;
     }
     if (!ctx->graph_ready) RET(capture_graphs(ctx));
     const int parity = ctx->f[KMM_FN] == ctx->g_fn0 ? 0 : 1;

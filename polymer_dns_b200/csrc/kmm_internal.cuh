@@ -138,11 +138,20 @@ struct kmm_ctx {
     float2 *rtw32[3]; // FP32 twiddles of 2 ny, mz, mx for the routine path's mixed form (kmm_fused.cu)
     double *d_frate;  // constant flow rate: W, G, the last correction, scratch (kmm_column.cu)
     int frate_ready;
+    int fused_ran;            // a fused step has run since its kernels were chosen (attributes and fields are set: capturable)
+    int fused_nomem;          // the fused step's tables or buffers did not fit: the routine step runs
+    int inject_nomem;         // KMM_INJECT_NOMEM: the allocation that is to fail (counted down), 0: none
     void *hoststate;  // host arrays bound by kmm_bind_host, their copy streams and events (kmm_hoststate.cu)
 };
 
 void kmm_hoststate_release(kmm_ctx *ctx);
 void kmm_fused_release(kmm_ctx *ctx);
+// whether this step is the fused one: KMM_OPT_FUSED, kmm_fused_applicable and its tables and buffers (built here
+// on first use; where memory does not allow them the routine step runs, as on a grid the kernels cannot hold)
+int kmm_fused_select(kmm_ctx *ctx, bool *fused);
+// cudaMalloc for tables and workspaces built on first use: KMM_ERR_NOMEM (and *p = NULL, the CUDA error cleared)
+// where memory is short
+int kmm_dalloc(kmm_ctx *ctx, void **p, size_t bytes);
 int kmm_fused_step(kmm_ctx *ctx);
 // the fused step in two halves: enqueue every kernel, then wait and evaluate the CFL number and the
 // status (kmm_fused_step = launch + finish; the ensemble launches all members first).

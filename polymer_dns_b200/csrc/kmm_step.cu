@@ -233,6 +233,7 @@ static int initial_restart(kmm_ctx *ctx) {
 extern "C" int kmm_initial(kmm_ctx *ctx) {
     if (!ctx) return KMM_ERR_ARG;
     kmm_graph_release(ctx);
+    ctx->fused_nomem = 0;
     const size_t n = ctx->nspec;
     RET(kmm_gfcn(ctx));
     RET(kmm_flowrate_setup(ctx));
@@ -339,7 +340,9 @@ static int swap_fields(kmm_ctx *ctx, int nm1, int n) {
 // ---------------------------------------------------------------------------
 extern "C" int kmm_step(kmm_ctx *ctx) {
     if (!ctx) return KMM_ERR_ARG;
-    if (ctx->use_fused && kmm_fused_applicable(ctx)) return kmm_fused_step(ctx);
+    bool fused;
+    RET(kmm_fused_select(ctx, &fused));
+    if (fused) return kmm_fused_step(ctx);
     if (ctx->p.precision == 1) {
         // the routine path's mixed form runs its transforms at the compiled lengths only; never fall
         // back silently to FP64
@@ -567,7 +570,9 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
 }
 
 int kmm_step_reported(kmm_ctx *ctx, bool *pending) {
-    if (!(ctx->use_fused && kmm_fused_applicable(ctx))) return kmm_step(ctx);
+    bool fused;
+    RET(kmm_fused_select(ctx, &fused));
+    if (!fused) return kmm_step(ctx);
     RET(kmm_fused_enqueue(ctx));
     *pending = true;
     return kmm_fused_report(ctx);
@@ -761,7 +766,10 @@ static int ensemble_step_all(kmm_ctx **ctxs, int n, int *status) {
             status[m] = KMM_ERR_CUDA;
             continue;
         }
-        if (c->use_fused && kmm_fused_applicable(c)) {
+        bool fused = false;
+        status[m] = kmm_fused_select(c, &fused);
+        if (status[m] != KMM_OK) continue;
+        if (fused) {
             status[m] = kmm_fused_enqueue(c);
             launched[m] = status[m] == KMM_OK;
         } else {

@@ -1,0 +1,43 @@
+"""Device memory that runs out while tables and buffers are built on first use (reported by the host-side injection,
+nothing is really exhausted): the forms that need no such memory run, and the next build starts afresh."""
+import numpy as np
+import pytest
+
+from polymer_dns_b200 import abi, runtime
+from tests.kmm_cases import cfg_small, initial_fields, load_initial, rel_err
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("V", "OMY", "FN", "GN", "U0", "W0")
+
+
+def _run(grid, fail, fused=1, how="run", **kw):
+    p = cfg_small(*grid, dt=0.002, **kw)
+    with runtime.KmmContext(p) as c:
+        c.call("set_option", abi.OPT_FUSED, fused)
+        fields = initial_fields(p, kmax=3)
+        load_initial(c, p, fields)
+        c.initial()
+        c.call("inject", abi.INJECT_NOMEM, fail)
+        if how == "ensemble":
+            assert runtime.ensemble_run([c], 2) == [abi.OK]
+        else:
+            c.run(2)
+        first = {k: c.download(k) for k in NAMES}
+        c.call("inject", abi.INJECT_NOMEM, 0)
+        c.call("set_option", abi.OPT_FUSED, 1)
+        c.run(1)
+        return first, {k: c.download(k) for k in NAMES}
+
+
+# the first, a middle and (at the blocked ny: among) the last of the fused step's allocations
+@pytest.mark.parametrize("grid", [(32, 32, 32), (40, 24, 12)])
+@pytest.mark.parametrize("fail", [1, 17, 35])
+def test_fused_step_without_memory_is_the_routine_step(grid, fail):
+    want, _ = _run(grid, 0, fused=0)
+    _, after = _run(grid, 0)
+    for how in ("run", "ensemble"):
+        got, got_after = _run(grid, fail, how=how)
+        for k in NAMES:
+            assert np.array_equal(got[k], want[k]), (how, k)
+            assert rel_err(got_after[k], after[k]) < 1e-9, (how, k)   # the two paths' FP64 rounding over 3 steps
