@@ -294,8 +294,13 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
     if (!C) {
         C = (TauCache *)calloc(1, sizeof(TauCache));
         if (!C) return KMM_ERR_NOMEM;
+        const int st = upload_rj(ctx, &C->rj, kmm_blocked_ny(ctx->ny));
+        if (st != KMM_OK) {
+            cudaFree(C->rj);
+            free(C);
+            return st == KMM_ERR_NOMEM ? KMM_ERR_UNSUPPORTED : st;
+        }
         ctx->tauc = C;
-        RET(upload_rj(ctx, &C->rj, kmm_blocked_ny(ctx->ny)));
     }
     const TabCfg want = {g, robin, robin ? at : 0.0, robin ? bt : 0.0, robin ? ab : 0.0, robin ? bb : 0.0, 1.0};
     int s = -1;
@@ -310,25 +315,27 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
         s = C->n;
         const int ncols = ctx->nz * ctx->nxh;
         const size_t n = (size_t)ncols * ctx->nyp;
-        double *canon[4] = {NULL, NULL, NULL, NULL};
-        cudaError_t me = cudaMalloc(&C->tabs[s][4], sizeof(double) * 4 * ncols);
-        for (int a = 0; a < 4 && me == cudaSuccess; ++a) me = cudaMalloc(&canon[a], sizeof(double) * n);
-        if (me != cudaSuccess) {   // no room for tables: the caller keeps the table-free kernels
-            for (int a = 0; a < 4; ++a) cudaFree(canon[a]);
-            cudaFree(C->tabs[s][4]);
-            C->tabs[s][4] = NULL;
-            cudaGetLastError();
-            return KMM_ERR_UNSUPPORTED;
+        double *canon[4] = {NULL, NULL, NULL, NULL}, **tab = C->tabs[s];
+        for (int a = 0; a < 5; ++a) tab[a] = NULL;
+        int st = kmm_dalloc(ctx, (void **)&tab[4], sizeof(double) * 4 * ncols);
+        for (int a = 0; a < 4 && st == KMM_OK; ++a) st = kmm_dalloc(ctx, (void **)&canon[a], sizeof(double) * n);
+        if (st == KMM_OK) {
+            k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(canon[0], canon[1], canon[2], canon[3], tab[4], want,
+                                                                      ctx->d_wavx, ctx->d_wavz, ncols, ctx->nz, ctx->nyp,
+                                                                      ctx->dyde);
+            CKL();
+            const double *src[4] = {canon[0], canon[1], canon[2], canon[3]};
+            st = block_tables(ctx, src, tab, ncols);
+            CK(cudaStreamSynchronize(ctx->stream));   // once per configuration, before the canonical copies go
         }
-        k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(canon[0], canon[1], canon[2], canon[3],
-                                                                  C->tabs[s][4], want, ctx->d_wavx, ctx->d_wavz,
-                                                                  ncols, ctx->nz, ctx->nyp, ctx->dyde);
-        CKL();
-        const double *src[4] = {canon[0], canon[1], canon[2], canon[3]};
-        const int bst = block_tables(ctx, src, C->tabs[s], ncols);
-        CK(cudaStreamSynchronize(ctx->stream));   // once per configuration, before the canonical copies go
         for (int a = 0; a < 4; ++a) cudaFree(canon[a]);
-        RET(bst);
+        if (st != KMM_OK) {   // no room for tables: the caller keeps the table-free kernels
+            for (int a = 0; a < 5; ++a) {
+                cudaFree(tab[a]);
+                tab[a] = NULL;
+            }
+            return st == KMM_ERR_NOMEM ? KMM_ERR_UNSUPPORTED : st;
+        }
         C->cfg[s] = want;
         C->n = s + 1;
     }

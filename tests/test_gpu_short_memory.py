@@ -41,3 +41,28 @@ def test_fused_step_without_memory_is_the_routine_step(grid, fail):
         for k in NAMES:
             assert np.array_equal(got[k], want[k]), (how, k)
             assert rel_err(got_after[k], after[k]) < 1e-9, (how, k)   # the two paths' FP64 rounding over 3 steps
+
+
+# the rj rows, the corner factors, a canonical table and the tables kept
+@pytest.mark.parametrize("ny", [32, 36])
+@pytest.mark.parametrize("fail", [1, 2, 4, 8, 10])
+def test_solves_without_memory_for_tables(ny, fail):
+    p = cfg_small(24, ny, 12)
+    rng = np.random.default_rng(7)
+    x = rng.standard_normal((ny + 1, 12, 12)) + 1j * rng.standard_normal((ny + 1, 12, 12))
+    got = []
+    for n in (0, fail):
+        with runtime.KmmContext(p) as c:
+            c.call("inject", abi.INJECT_NOMEM, n)
+            out = []
+            for _ in range(4):   # the failing call, and calls that may build again
+                c.upload("V", x)
+                c.call("solve", "V", 50.0, 0)
+                out.append(c.download("V"))
+                c.upload("OMY", x)
+                c.call("penta", "OMY", 50.0, 0, 1.0, 0.0, 1.0, 0.0)
+                out.append(c.download("OMY"))
+            got.append(out)
+    for a, b in zip(*got):
+        assert np.abs(a).max() > 0.0
+        assert rel_err(b, a) < 1e-10   # tabled and table-free solves of one tau system
