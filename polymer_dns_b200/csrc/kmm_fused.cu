@@ -119,6 +119,10 @@ __global__ void k_tab_block(const double *__restrict__ src, double *__restrict__
     }
 }
 
+__global__ void k_recip(double *x, size_t n) {
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) x[e] = 1.0 / x[e];
+}
+
 // copies of one configuration's td (as 1 / d), te, tb1, tb2 (tf is per column, unchanged), lane-blocked
 // for the ny of the blocked kernels, else (K = 0) in the canonical order
 static int block_tables(kmm_ctx *ctx, const double *const src[4], double *dst[4], int ncols) {
@@ -281,12 +285,32 @@ int kmm_fused_select(kmm_ctx *ctx, bool *fused) {
 // for the context's lifetime (a run meets a handful: v's two solves, omega_y, the scalar and the
 // polymer components)
 #define KMM_TAU_SETS 12
+#define KMM_TAU_AFTER 3
 struct TauCache {
     int n;
+    TabCfg seen[KMM_TAU_SETS];       // ny without blocked kernels: the last configurations asked for, and how often
+    int asked[KMM_TAU_SETS], next;
     TabCfg cfg[KMM_TAU_SETS];
     double *tabs[KMM_TAU_SETS][5];   // td (as 1 / d), te, tb1, tb2 (lane-blocked for the blocked ny); tf
     double *rj;                      // rj rows in the same order
 };
+
+static bool same_cfg(const TabCfg &a, const TabCfg &b) {
+    return a.g == b.g && a.robin == b.robin && a.at == b.at && a.bt == b.bt && a.ab == b.ab && a.bb == b.bb;
+}
+
+// The ny without blocked kernels have table-free solves (140 us a field at 80 x 61 x 60) and tabled ones (16); a set
+// takes 1.3 ms to build.  It is built when its configuration is asked for the third time, so that a
+// program whose g changes from call to call (a varying time step) neither waits for sets it uses once nor keeps them.
+// (The blocked ny build at once, as their fused phirhs and solves need the tables.)
+static bool worth_tables(TauCache *C, const TabCfg &want) {
+    for (int i = 0; i < KMM_TAU_SETS; ++i)
+        if (C->asked[i] && same_cfg(C->seen[i], want)) return ++C->asked[i] >= KMM_TAU_AFTER;
+    C->seen[C->next] = want;
+    C->asked[C->next] = 1;
+    C->next = (C->next + 1) % KMM_TAU_SETS;
+    return false;
+}
 
 int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, double ab, double bb, const double **tabs,
                    const double **rj) {
@@ -294,39 +318,37 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
     if (!C) {
         C = (TauCache *)calloc(1, sizeof(TauCache));
         if (!C) return KMM_ERR_NOMEM;
-        const int st = upload_rj(ctx, &C->rj, kmm_blocked_ny(ctx->ny));
-        if (st != KMM_OK) {
-            cudaFree(C->rj);
-            free(C);
-            return st == KMM_ERR_NOMEM ? KMM_ERR_UNSUPPORTED : st;
-        }
         ctx->tauc = C;
     }
     const TabCfg want = {g, robin, robin ? at : 0.0, robin ? bt : 0.0, robin ? ab : 0.0, robin ? bb : 0.0, 1.0};
     int s = -1;
     for (int i = 0; i < C->n && s < 0; ++i) {
-        const TabCfg &c = C->cfg[i];
-        if (c.g == want.g && c.robin == want.robin && c.at == want.at && c.bt == want.bt && c.ab == want.ab &&
-            c.bb == want.bb)
-            s = i;
+        if (same_cfg(C->cfg[i], want)) s = i;
     }
     if (s < 0) {
         if (C->n == KMM_TAU_SETS) return KMM_ERR_UNSUPPORTED;   // the caller keeps the table-free kernels
+        const bool blocked = kmm_blocked_ny(ctx->ny);
+        if (!blocked && !worth_tables(C, want)) return KMM_ERR_UNSUPPORTED;
         s = C->n;
         const int ncols = ctx->nz * ctx->nxh;
         const size_t n = (size_t)ncols * ctx->nyp;
-        double *canon[4] = {NULL, NULL, NULL, NULL}, **tab = C->tabs[s];
+        double *canon[4] = {NULL, NULL, NULL, NULL}, **tab = C->tabs[s], **cn = blocked ? canon : tab;
         for (int a = 0; a < 5; ++a) tab[a] = NULL;
-        int st = kmm_dalloc(ctx, (void **)&tab[4], sizeof(double) * 4 * ncols);
-        for (int a = 0; a < 4 && st == KMM_OK; ++a) st = kmm_dalloc(ctx, (void **)&canon[a], sizeof(double) * n);
+        int st = C->rj ? KMM_OK : upload_rj(ctx, &C->rj, blocked);
+        if (st == KMM_OK) st = kmm_dalloc(ctx, (void **)&tab[4], sizeof(double) * 4 * ncols);
+        for (int a = 0; a < 4 && st == KMM_OK; ++a) st = kmm_dalloc(ctx, (void **)&cn[a], sizeof(double) * n);
         if (st == KMM_OK) {
-            k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(canon[0], canon[1], canon[2], canon[3], tab[4], want,
-                                                                      ctx->d_wavx, ctx->d_wavz, ncols, ctx->nz, ctx->nyp,
-                                                                      ctx->dyde);
+            k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(cn[0], cn[1], cn[2], cn[3], tab[4], want, ctx->d_wavx,
+                                                                      ctx->d_wavz, ncols, ctx->nz, ctx->nyp, ctx->dyde);
             CKL();
-            const double *src[4] = {canon[0], canon[1], canon[2], canon[3]};
-            st = block_tables(ctx, src, tab, ncols);
-            CK(cudaStreamSynchronize(ctx->stream));   // once per configuration, before the canonical copies go
+            if (blocked) {
+                const double *src[4] = {canon[0], canon[1], canon[2], canon[3]};
+                st = block_tables(ctx, src, tab, ncols);
+                CK(cudaStreamSynchronize(ctx->stream));   // once per configuration, before the canonical copies go
+            } else {
+                k_recip<<<kmm_blocks(n, 256), 256, 0, ctx->stream>>>(tab[0], n);
+                CKL();
+            }
         }
         for (int a = 0; a < 4; ++a) cudaFree(canon[a]);
         if (st != KMM_OK) {   // no room for tables: the caller keeps the table-free kernels
@@ -532,8 +554,8 @@ int kmm_warpcol_phirhs_solve(kmm_ctx *ctx, double2 *const *x, const double2 *con
     WarpColCfg S[2];
     memset(S, 0, sizeof(S));
     const double *rj = NULL;
-    for (int k = 0; k < (nsolve ? 2 : 0); ++k) {
-        const KmmSolveSpec &q = spec[k < nsolve ? k : 0];
+    for (int k = 0; k < nsolve; ++k) {
+        const KmmSolveSpec &q = spec[k];
         RET(kmm_tau_tabset(ctx, q.g, q.robin, q.at, q.bt, q.ab, q.bb, S[k].tab, &rj));
         S[k].g = q.g;
         S[k].robin = q.robin;

@@ -66,3 +66,22 @@ def test_solves_without_memory_for_tables(ny, fail):
     for a, b in zip(*got):
         assert np.abs(a).max() > 0.0
         assert rel_err(b, a) < 1e-10   # tabled and table-free solves of one tau system
+
+
+def test_tables_only_for_configurations_that_come_back():
+    """ny without blocked kernels: a solve builds its tau tables at the third call with one g, and a changing g none."""
+    p = cfg_small(24, 36, 12)
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal((37, 12, 12)) + 1j * rng.standard_normal((37, 12, 12))
+    with runtime.KmmContext(p) as c:
+        def solve(g):
+            c.upload("V", x)
+            n = c.launch_count()
+            c.call("solve", "V", g, 0)
+            return c.launch_count() - n, c.download("V")
+
+        assert [solve(10.0 + m)[0] for m in range(20)] == [1] * 20
+        same = [solve(5.0) for _ in range(4)]
+        assert [n for n, _ in same] == [1, 1, 3, 1]   # tables, their reciprocals, the solve
+        assert np.array_equal(same[0][1], same[1][1]) and np.array_equal(same[2][1], same[3][1])
+        assert rel_err(same[2][1], same[0][1]) < 1e-10
