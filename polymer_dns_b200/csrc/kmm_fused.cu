@@ -54,12 +54,22 @@ __device__ __forceinline__ void tab_row(int i, int par, double wn, double dyde, 
     }
 }
 
+// the configurations of one launch: their arrays and numbers of columns
+struct TabJobs {
+    double *td[TB_N], *te[TB_N], *tb1[TB_N], *tb2[TB_N], *tf[TB_N];
+    TabCfg cfg[TB_N];
+    int nc[TB_N];
+};
+
 // one thread per column: d(i) chain (eqsolve / pntsolve), forward multipliers, border weights and
-// final f values for one configuration
-__global__ void k_tau_tables(double *td, double *te, double *tb1, double *tb2, double *tf, TabCfg C,
-                             const double *wavx, const double *wavz, int ncols, int nz, int nyp, double dyde) {
+// final f values; blockIdx.y picks the configuration (each is a serial chain of divisions that leaves most of the
+// chip idle, so they run side by side)
+__global__ void k_tau_tables(TabJobs J, const double *wavx, const double *wavz, int nz, int nyp, double dyde) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncols) return;
+    if (col >= J.nc[blockIdx.y]) return;
+    const TabCfg C = J.cfg[blockIdx.y];
+    double *td = J.td[blockIdx.y], *te = J.te[blockIdx.y], *tb1 = J.tb1[blockIdx.y], *tb2 = J.tb2[blockIdx.y],
+           *tf = J.tf[blockIdx.y];
     const int ny = nyp - 1, nyh = ny / 2, nyhm = nyh - 1, nyhp = nyh + 1;
     const int j = col % nz, k = col / nz;
     const double wn = wavz[j] * wavz[j] + wavx[k] * wavx[k] + C.g;
@@ -123,20 +133,28 @@ __global__ void k_recip(double *x, size_t n) {
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) x[e] = 1.0 / x[e];
 }
 
-// copies of one configuration's td (as 1 / d), te, tb1, tb2 (tf is per column, unchanged), lane-blocked
-// for the ny of the blocked kernels, else (K = 0) in the canonical order
-static int block_tables(kmm_ctx *ctx, const double *const src[4], double *dst[4], int ncols) {
-    const int K = kmm_blocked_ny(ctx->ny) ? ctx->ny / 16 : 0;
+// lane-blocked copies of one configuration's td (as 1 / d), te, tb1, tb2 (tf is per column, unchanged)
+static int block_tables(kmm_ctx *ctx, const double *const src[4], double *const dst[4], int ncols) {
     const size_t n = (size_t)ncols * ctx->nyp;
     const int nb = (int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-    for (int a = 0; a < 4; ++a) dst[a] = NULL;
-    for (int a = 0; a < 4; ++a) {   // (the caller frees dst on failure)
-        RET(kmm_dalloc(ctx, (void **)&dst[a], sizeof(double) * n));
-        k_tab_block<<<nb, 256, 0, ctx->stream>>>(src[a], dst[a], ncols, ctx->nyp, K, a == 0);
+    for (int a = 0; a < 4; ++a) {
+        k_tab_block<<<nb, 256, 0, ctx->stream>>>(src[a], dst[a], ncols, ctx->nyp, ctx->ny / 16, a == 0);
         CKL();
     }
     return KMM_OK;
 }
+
+// pieces of one allocation, each on a 256-byte boundary (an allocation on this path takes 0.2 ms: with one for
+// every array, 70 of them, the first step of a context took 14 to 16 ms at 64 x 65 x 64 and 128 x 129 x 128; it takes 0.65
+// and 1.6)
+struct Carver {
+    size_t end = 0;
+    size_t take(size_t bytes) {
+        const size_t o = end;
+        end += (bytes + 255) & ~(size_t)255;
+        return o;
+    }
+};
 
 // the three rj rows (1/(4j(j-1)), 1/(2(j^2-1)), 1/(4j(j+1))) on the host, in natural or lane-blocked order
 static void rj_rows(double *h, int nyp, bool blocked) {
@@ -150,15 +168,13 @@ static void rj_rows(double *h, int nyp, bool blocked) {
     }
 }
 
-static int upload_rj(kmm_ctx *ctx, double **out, bool blocked) {
+static int fill_rj(kmm_ctx *ctx, double *dev, bool blocked) {
     const int nyp = ctx->nyp;
     double *h = (double *)calloc(3 * (size_t)nyp, sizeof(double));
     if (!h) return KMM_ERR_NOMEM;
     rj_rows(h, nyp, blocked);
-    const int st = kmm_dalloc(ctx, (void **)out, sizeof(double) * 3 * nyp);
-    const cudaError_t e = st == KMM_OK ? cudaMemcpy(*out, h, sizeof(double) * 3 * nyp, cudaMemcpyHostToDevice) : cudaSuccess;
+    const cudaError_t e = cudaMemcpy(dev, h, sizeof(double) * 3 * nyp, cudaMemcpyHostToDevice);
     free(h);
-    RET(st);
     CK(e);
     return KMM_OK;
 }
@@ -194,64 +210,76 @@ static int fill_tables(kmm_ctx *ctx, KmmFused *F) {
     // mean modes (uzero -> psolve1d, solvers.f90:1065-1245): only the (0,0) column; w0 passes btu
     cfg[TB_U0] = {g1, 1, ctx->atu, ctx->btu, ctx->abu, ctx->bbu, -1.0};
     cfg[TB_W0] = {g1, 1, ctx->atw, ctx->btu, ctx->abw, ctx->bbw, -1.0};
-    FusedTabs &T = F->tabs;
+    // everything in one allocation; each of the four table arrays holds the configurations one after another
+    const bool blocked = kmm_blocked_ny(ctx->ny);
+    const int nyp = ctx->nyp;
+    TabJobs J;
+    size_t nall = 0, at[TB_N], fat[TB_N], ntf = 0;
     for (int c = 0; c < TB_N; ++c) {
-        const int nc = (c == TB_U0 || c == TB_W0) ? 1 : ncols;   // the mean modes use column (0,0) only
-        const size_t n = (size_t)nc * ctx->nyp;
-        double **const tab[4] = {&T.td[c], &T.te[c], &T.tb1[c], &T.tb2[c]};
-        for (int a = 0; a < 4; ++a) RET(kmm_dalloc(ctx, (void **)tab[a], sizeof(double) * n));
-        RET(kmm_dalloc(ctx, (void **)&T.tf[c], sizeof(double) * 4 * nc));
+        J.cfg[c] = cfg[c];
+        J.nc[c] = (c == TB_U0 || c == TB_W0) ? 1 : ncols;   // the mean modes use column (0,0) only
+        at[c] = nall;
+        fat[c] = ntf;
+        nall += (size_t)J.nc[c] * nyp;
+        ntf += 4 * (size_t)J.nc[c];
+    }
+    const size_t ncp = (size_t)ncols * nyp, nq = (size_t)nyp * ctx->mz * ctx->nxh;
+    Carver V;
+    size_t ot[4], ob[4];
+    for (int a = 0; a < 4; ++a) ot[a] = V.take(sizeof(double) * nall);
+    const size_t of = V.take(sizeof(double) * ntf), orj = V.take(sizeof(double) * 3 * nyp);
+    if (blocked)
+        for (int a = 0; a < 4; ++a) ob[a] = V.take(sizeof(double) * nall);
+    const size_t obrj = blocked ? V.take(sizeof(double) * 3 * nyp) : 0;
+    const size_t oyp = V.take(sizeof(double2) * ncp * 8), oq = V.take(sizeof(double2) * nq * 10);
+    const size_t orr = V.take(sizeof(double2) * nq * 4), oyo = V.take(sizeof(double2) * ncp * 4);
+    const size_t nacc = sizeof(double) * (2 * (size_t)nyp + 1), oacc = V.take(nacc);
+    RET(kmm_dalloc(ctx, (void **)&F->block, V.end));
+    char *const B = F->block;
+    auto dbl = [&](size_t o, size_t e) { return reinterpret_cast<double *>(B + o) + e; };
+    FusedTabs &T = F->tabs, &TB = F->btabs;
+    for (int c = 0; c < TB_N; ++c) {
+        J.td[c] = T.td[c] = dbl(ot[0], at[c]); J.te[c] = T.te[c] = dbl(ot[1], at[c]);
+        J.tb1[c] = T.tb1[c] = dbl(ot[2], at[c]); J.tb2[c] = T.tb2[c] = dbl(ot[3], at[c]);
+        J.tf[c] = T.tf[c] = dbl(of, fat[c]);
         T.g[c] = cfg[c].g;
-        k_tau_tables<<<(nc + 127) / 128, 128, 0, ctx->stream>>>(T.td[c], T.te[c], T.tb1[c], T.tb2[c], T.tf[c], cfg[c],
-                                                               ctx->d_wavx, ctx->d_wavz, nc, ctx->nz, ctx->nyp,
-                                                               ctx->dyde);
-        CKL();
     }
+    k_tau_tables<<<dim3((ncols + 127) / 128, TB_N), 128, 0, ctx->stream>>>(J, ctx->d_wavx, ctx->d_wavz, ctx->nz, nyp, ctx->dyde);
+    CKL();
     // reciprocals of the tau row coefficients (the same divisions as the device's tau_rhs)
-    RET(upload_rj(ctx, &F->rj, false));
-    if (kmm_blocked_ny(ctx->ny)) {   // the blocked column kernels' copies
+    F->rj = dbl(orj, 0);
+    RET(fill_rj(ctx, F->rj, false));
+    if (blocked) {   // the blocked column kernels' copies
         for (int c = 0; c < TB_N; ++c) {
-            const int nc = (c == TB_U0 || c == TB_W0) ? 1 : ncols;
+            TB.td[c] = dbl(ob[0], at[c]); TB.te[c] = dbl(ob[1], at[c]);
+            TB.tb1[c] = dbl(ob[2], at[c]); TB.tb2[c] = dbl(ob[3], at[c]);
+            TB.tf[c] = T.tf[c];
+            TB.g[c] = T.g[c];
             const double *src[4] = {T.td[c], T.te[c], T.tb1[c], T.tb2[c]};
-            double *dst[4];
-            const int st = block_tables(ctx, src, dst, nc);
-            F->btabs.td[c] = dst[0]; F->btabs.te[c] = dst[1]; F->btabs.tb1[c] = dst[2]; F->btabs.tb2[c] = dst[3];
-            RET(st);
-            F->btabs.tf[c] = T.tf[c];
-            F->btabs.g[c] = T.g[c];
+            double *const dst[4] = {TB.td[c], TB.te[c], TB.tb1[c], TB.tb2[c]};
+            RET(block_tables(ctx, src, dst, J.nc[c]));
         }
-        RET(upload_rj(ctx, &F->brj, true));
+        F->brj = dbl(obrj, 0);
+        RET(fill_rj(ctx, F->brj, true));
     }
-    for (int c = 0; c < TB_N; ++c) {   // the canonical pivots become 1 / d too (K = 0: positions kept)
-        const size_t n = (size_t)((c == TB_U0 || c == TB_W0) ? 1 : ncols) * ctx->nyp;
-        double *r = NULL;
-        RET(kmm_dalloc(ctx, (void **)&r, sizeof(double) * n));
-        k_tab_block<<<(int)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184), 256, 0, ctx->stream>>>(T.td[c], r, (int)(n / ctx->nyp),
-                                                                                                 ctx->nyp, 0, 1);
-        cudaFree(T.td[c]);
-        T.td[c] = r;
-        CKL();
+    k_recip<<<kmm_blocks(nall, 256), 256, 0, ctx->stream>>>(dbl(ot[0], 0), nall);   // the canonical pivots become 1 / d too
+    CKL();
+    if (ctx->p.precision == 1) {
+        RET(make_twf(ctx, 2 * ctx->ny, &F->twf_y2));
+        RET(make_twf(ctx, ctx->mz, &F->twf_mz));
+        RET(make_twf(ctx, ctx->mx, &F->twf_mx));
     }
-    RET(make_twf(ctx, 2 * ctx->ny, &F->twf_y2));
-    RET(make_twf(ctx, ctx->mz, &F->twf_mz));
-    RET(make_twf(ctx, ctx->mx, &F->twf_mx));
-    const size_t ncp = (size_t)ncols * ctx->nyp, nq = (size_t)ctx->nyp * ctx->mz * ctx->nxh;
-    RET(kmm_dalloc(ctx, (void **)&F->yp, sizeof(double2) * ncp * 8));
-    RET(kmm_dalloc(ctx, (void **)&F->q, sizeof(double2) * nq * 10));
-    RET(kmm_dalloc(ctx, (void **)&F->r, sizeof(double2) * nq * 4));
-    RET(kmm_dalloc(ctx, (void **)&F->yo, sizeof(double2) * ncp * 4));
-    RET(kmm_dalloc(ctx, (void **)&F->acc, sizeof(double) * (2 * (size_t)ctx->nyp + 1)));
-    CK(cudaMemsetAsync(F->acc, 0, sizeof(double) * (2 * (size_t)ctx->nyp + 1), ctx->stream));
+    F->yp = reinterpret_cast<double2 *>(B + oyp);
+    F->q = reinterpret_cast<double2 *>(B + oq);
+    F->r = reinterpret_cast<double2 *>(B + orr);
+    F->yo = reinterpret_cast<double2 *>(B + oyo);
+    F->acc = dbl(oacc, 0);
+    CK(cudaMemsetAsync(F->acc, 0, nacc, ctx->stream));
     return KMM_OK;
 }
 
 static void fused_free(KmmFused *F) {
-    for (int c = 0; c < TB_N; ++c) {
-        cudaFree(F->tabs.td[c]); cudaFree(F->tabs.te[c]); cudaFree(F->tabs.tb1[c]); cudaFree(F->tabs.tb2[c]);
-        cudaFree(F->tabs.tf[c]);
-        cudaFree(F->btabs.td[c]); cudaFree(F->btabs.te[c]); cudaFree(F->btabs.tb1[c]); cudaFree(F->btabs.tb2[c]);
-    }
-    cudaFree(F->yp); cudaFree(F->q); cudaFree(F->r); cudaFree(F->yo); cudaFree(F->acc); cudaFree(F->rj); cudaFree(F->brj);
+    cudaFree(F->block);
     cudaFree(F->twf_y2); cudaFree(F->twf_mz); cudaFree(F->twf_mx);
     free(F);
 }
@@ -300,7 +328,7 @@ static bool same_cfg(const TabCfg &a, const TabCfg &b) {
 }
 
 // The ny without blocked kernels have table-free solves (140 us a field at 80 x 61 x 60) and tabled ones (16); a set
-// takes 1.3 ms to build.  It is built when its configuration is asked for the third time, so that a
+// takes 0.4 ms to build.  It is built when its configuration is asked for the third time, so that a
 // program whose g changes from call to call (a varying time step) neither waits for sets it uses once nor keeps them.
 // (The blocked ny build at once, as their fused phirhs and solves need the tables.)
 static bool worth_tables(TauCache *C, const TabCfg &want) {
@@ -332,17 +360,34 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
         s = C->n;
         const int ncols = ctx->nz * ctx->nxh;
         const size_t n = (size_t)ncols * ctx->nyp;
-        double *canon[4] = {NULL, NULL, NULL, NULL}, **tab = C->tabs[s], **cn = blocked ? canon : tab;
-        for (int a = 0; a < 5; ++a) tab[a] = NULL;
-        int st = C->rj ? KMM_OK : upload_rj(ctx, &C->rj, blocked);
-        if (st == KMM_OK) st = kmm_dalloc(ctx, (void **)&tab[4], sizeof(double) * 4 * ncols);
-        for (int a = 0; a < 4 && st == KMM_OK; ++a) st = kmm_dalloc(ctx, (void **)&cn[a], sizeof(double) * n);
+        // a set is one allocation; the blocked ny's canonical arrays another, freed once the copies are made
+        Carver V, W;
+        const size_t of = V.take(sizeof(double) * 4 * ncols);
+        size_t ot[4], oc[4];
+        for (int a = 0; a < 4; ++a) ot[a] = V.take(sizeof(double) * n);
+        for (int a = 0; a < 4; ++a) oc[a] = W.take(sizeof(double) * n);
+        char *set = NULL, *canon = NULL;
+        int st = C->rj ? KMM_OK : kmm_dalloc(ctx, (void **)&C->rj, sizeof(double) * 3 * ctx->nyp);
+        if (st == KMM_OK && !C->n) st = fill_rj(ctx, C->rj, blocked);
+        if (st == KMM_OK) st = kmm_dalloc(ctx, (void **)&set, V.end);
+        if (st == KMM_OK && blocked) st = kmm_dalloc(ctx, (void **)&canon, W.end);
         if (st == KMM_OK) {
-            k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(cn[0], cn[1], cn[2], cn[3], tab[4], want, ctx->d_wavx,
-                                                                      ctx->d_wavz, ncols, ctx->nz, ctx->nyp, ctx->dyde);
+            double *tab[4], *cn[4];
+            for (int a = 0; a < 4; ++a) {
+                tab[a] = reinterpret_cast<double *>(set + ot[a]);
+                cn[a] = blocked ? reinterpret_cast<double *>(canon + oc[a]) : tab[a];
+                C->tabs[s][a] = tab[a];
+            }
+            C->tabs[s][4] = reinterpret_cast<double *>(set + of);
+            TabJobs J;
+            memset(&J, 0, sizeof(J));
+            J.td[0] = cn[0]; J.te[0] = cn[1]; J.tb1[0] = cn[2]; J.tb2[0] = cn[3]; J.tf[0] = C->tabs[s][4];
+            J.cfg[0] = want;
+            J.nc[0] = ncols;
+            k_tau_tables<<<(ncols + 127) / 128, 128, 0, ctx->stream>>>(J, ctx->d_wavx, ctx->d_wavz, ctx->nz, ctx->nyp, ctx->dyde);
             CKL();
             if (blocked) {
-                const double *src[4] = {canon[0], canon[1], canon[2], canon[3]};
+                const double *src[4] = {cn[0], cn[1], cn[2], cn[3]};
                 st = block_tables(ctx, src, tab, ncols);
                 CK(cudaStreamSynchronize(ctx->stream));   // once per configuration, before the canonical copies go
             } else {
@@ -350,12 +395,9 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
                 CKL();
             }
         }
-        for (int a = 0; a < 4; ++a) cudaFree(canon[a]);
+        cudaFree(canon);
         if (st != KMM_OK) {   // no room for tables: the caller keeps the table-free kernels
-            for (int a = 0; a < 5; ++a) {
-                cudaFree(tab[a]);
-                tab[a] = NULL;
-            }
+            cudaFree(set);
             return st == KMM_ERR_NOMEM ? KMM_ERR_UNSUPPORTED : st;
         }
         C->cfg[s] = want;
@@ -383,8 +425,7 @@ void kmm_tau_release(kmm_ctx *ctx) {
     }
     TauCache *C = (TauCache *)ctx->tauc;
     if (!C) return;
-    for (int i = 0; i < C->n; ++i)
-        for (int a = 0; a < 5; ++a) cudaFree(C->tabs[i][a]);
+    for (int i = 0; i < C->n; ++i) cudaFree(C->tabs[i][4]);   // a set's allocation starts with tf
     cudaFree(C->rj);
     free(C);
     ctx->tauc = NULL;

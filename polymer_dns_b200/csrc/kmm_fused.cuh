@@ -21,9 +21,10 @@ template <typename C>
 __host__ __device__ __forceinline__ int col_ld(int nyp) { return sizeof(C) == 8 ? ((nyp + 1) & ~1) : nyp; }
 
 struct KmmFused {
+    char *block;   // the one allocation of the members below (the FP32 twiddles excepted)
     FusedTabs tabs;
     // the same tables and rj rows in the lane-blocked order of the blocked column kernels
-    // (kmm_colblk.cuh), td there holding 1 / d; built where ny is a multiple of 16
+    // (kmm_colblk.cuh), td there holding 1 / d; built for the ny of kmm_blocked_ny
     FusedTabs btabs;
     double2 *yp, *q, *r, *yo;
     double *acc;   // the step's own accumulators: cfl[nyp], umax[nyp], the status word; zero between steps
