@@ -196,7 +196,11 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
         __syncthreads();
         if (threadIdx.x == 0) tma_store4(&tout, 2 * kx0, 0, y0, g, stage);
     }
-    if (threadIdx.x == 0) tma_store_wait_read();   // shared memory must outlive the last store's read
+    if (threadIdx.x == 0) {
+        tma_store_wait_read();   // shared memory must outlive the last store's read
+        // after a timeout, wait (again with the limit) for the tile loads still in flight before the CTA exits
+        for (int q = 0; !ok && q < nslot; ++q) mbar_wait(&bar[q], 0);
+    }
     if (!ok && lane == 0) atomicMax(status, KMM_ERR_TIMEOUT);
 }
 
@@ -226,10 +230,11 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    unsigned issued = 0, ready = 0;
+    unsigned issued = 0;
+    bool ok = true;
     const int o0 = blockIdx.z * nper;
     auto load = [&](int o) {
-        if (o >= nper) return;
+        if (o >= nper || !ok) return;   // nothing is loaded over a tile that did not arrive
         mbar_expect_tx(&bar[o], (unsigned)(TIN * sizeof(C)));
         tma_load4(tiles + (size_t)(o % ZF_SLOTS) * TIN, &tin, 2 * kx0, 0, y0, o0 + o, &bar[o]);
         issued |= 1u << o;
@@ -241,10 +246,8 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
     const T rs = (T)(1.0 / scale);
     const C zc = kct::mk<C>((T)0, (T)0);
     C *a = scr + (size_t)warp * flen<C>(MZ);
-    bool ok = true;
     for (int o = 0; o < nper; ++o) {
         ok = mbar_wait(&bar[o], 0) && ok;
-        ready |= 1u << o;
         const C *t = tiles + (size_t)(o % ZF_SLOTS) * TIN;
         auto ld = [&](int z) { return ok ? t[tile_idx<C, KX>(y * MZ + z, kl)] : zc; };
         auto before = [&] {
@@ -267,9 +270,8 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
     }
     if (threadIdx.x == 0) {
         tma_store_wait_read();
-        if (!ok)
-            for (int o = 0; o < nper; ++o)
-                if (((issued >> o) & 1u) && !((ready >> o) & 1u)) mbar_wait(&bar[o], 0);
+        for (int o = 0; !ok && o < nper; ++o)   // as above
+            if ((issued >> o) & 1u) mbar_wait(&bar[o], 0);
     }
     if (!ok && lane == 0) *status = KMM_ERR_TIMEOUT;
 }
