@@ -317,6 +317,7 @@ int kmm_fused_select(kmm_ctx *ctx, bool *fused) {
 // polymer components)
 #define KMM_TAU_SETS 12
 #define KMM_TAU_AFTER 3
+#define KMM_TAU_KEEP (2u << 20)   // a small grid's setup would spend 0.35 ms a set on this scratch's release
 struct TauCache {
     int n;
     TabCfg seen[KMM_TAU_SETS];       // ny without blocked kernels: the last configurations asked for, and how often
@@ -324,6 +325,7 @@ struct TauCache {
     TabCfg cfg[KMM_TAU_SETS];
     double *tabs[KMM_TAU_SETS][5];   // td (as 1 / d), te, tb1, tb2 (lane-blocked for the blocked ny); tf
     double *rj;                      // rj rows in the same order
+    char *canon;                     // the blocked ny's canonical arrays, kept where small (KMM_TAU_KEEP)
 };
 
 static bool same_cfg(const TabCfg &a, const TabCfg &b) {
@@ -369,16 +371,16 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
         size_t ot[4], oc[4];
         for (int a = 0; a < 4; ++a) ot[a] = V.take(sizeof(double) * n);
         for (int a = 0; a < 4; ++a) oc[a] = W.take(sizeof(double) * n);
-        char *set = NULL, *canon = NULL;
+        char *set = NULL;
         int st = C->rj ? KMM_OK : kmm_dalloc(ctx, (void **)&C->rj, sizeof(double) * 3 * ctx->nyp);
         if (st == KMM_OK && !C->n) st = fill_rj(ctx, C->rj, blocked);
         if (st == KMM_OK) st = kmm_dalloc(ctx, (void **)&set, V.end);
-        if (st == KMM_OK && blocked) st = kmm_dalloc(ctx, (void **)&canon, W.end);
+        if (st == KMM_OK && blocked && !C->canon) st = kmm_dalloc(ctx, (void **)&C->canon, W.end);
         if (st == KMM_OK) {
             double *tab[4], *cn[4];
             for (int a = 0; a < 4; ++a) {
                 tab[a] = reinterpret_cast<double *>(set + ot[a]);
-                cn[a] = blocked ? reinterpret_cast<double *>(canon + oc[a]) : tab[a];
+                cn[a] = blocked ? reinterpret_cast<double *>(C->canon + oc[a]) : tab[a];
                 C->tabs[s][a] = tab[a];
             }
             C->tabs[s][4] = reinterpret_cast<double *>(set + of);
@@ -398,7 +400,10 @@ int kmm_tau_tabset(kmm_ctx *ctx, double g, int robin, double at, double bt, doub
                 CKL();
             }
         }
-        cudaFree(canon);
+        if (W.end > KMM_TAU_KEEP) {
+            cudaFree(C->canon);
+            C->canon = NULL;
+        }
         if (st != KMM_OK) {   // no room for tables: the caller keeps the table-free kernels
             cudaFree(set);
             return st == KMM_ERR_NOMEM ? KMM_ERR_UNSUPPORTED : st;
@@ -430,6 +435,7 @@ void kmm_tau_release(kmm_ctx *ctx) {
     if (!C) return;
     for (int i = 0; i < C->n; ++i) cudaFree(C->tabs[i][4]);   // a set's allocation starts with tf
     cudaFree(C->rj);
+    cudaFree(C->canon);
     free(C);
     ctx->tauc = NULL;
 }
