@@ -20,6 +20,8 @@
 #include <math.h>
 
 #include <atomic>
+#include <chrono>
+#include <thread>
 
 #include "kmm_fft.cuh"
 #include "kmm_fused.cuh"
@@ -1694,19 +1696,49 @@ int kmm_fused_finish(kmm_ctx *ctx) {
     return report_status(ctx);
 }
 
+// The host's wait between two looks at the report: for the first 20 us none (a small grid's step takes 40), then
+// what the device's scheduling flag asks for: a sleep under cudaDeviceScheduleBlockingSync (the step's last kernels,
+// behind its report, cover the wake-up of a larger grid), else a yield, so that a host with more run threads than
+// cores, or other work on them, is not held up by the polling.
+namespace {
+struct HostWait {
+    typedef std::chrono::steady_clock Clock;
+    Clock::time_point t0 = Clock::now(), asked = t0;
+    int mode = -1;
+    void pause() {
+        if (mode < 0) {
+            for (int k = 0; k < 64; ++k) std::atomic_signal_fence(std::memory_order_seq_cst);
+            if (Clock::now() - t0 < std::chrono::microseconds(20)) return;
+            unsigned f = 0;
+            if (cudaGetDeviceFlags(&f) != cudaSuccess) cudaGetLastError();
+            mode = (f & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
+        }
+        if (mode == 1) std::this_thread::sleep_for(std::chrono::microseconds(20));
+        else std::this_thread::yield();
+    }
+    // every 200 us: time to ask the stream for an error
+    bool due() {
+        if (mode < 0) return false;
+        const Clock::time_point t = Clock::now();
+        if (t - asked < std::chrono::microseconds(200)) return false;
+        asked = t;
+        return true;
+    }
+};
+}  // namespace
+
 int kmm_fused_report(kmm_ctx *ctx) {
     // the report is the last store of a kernel already enqueued; the stream is asked now and then, so
     // that a launch or device error ends the wait
-    for (unsigned k = 1; !ctx->rep->flag; ++k) {
-        if ((k & 0xfff) == 0) {
-            const cudaError_t e = cudaStreamQuery(ctx->stream);
-            if (e != cudaErrorNotReady) {
-                CK(e);
-                CK(cudaStreamSynchronize(ctx->stream));
-                if (!ctx->rep->flag) {
-                    kmm_set_error(ctx, "the step ended without its report");
-                    return KMM_ERR_CUDA;
-                }
+    for (HostWait w; !ctx->rep->flag; w.pause()) {
+        if (!w.due()) continue;
+        const cudaError_t e = cudaStreamQuery(ctx->stream);
+        if (e != cudaErrorNotReady) {
+            CK(e);
+            CK(cudaStreamSynchronize(ctx->stream));
+            if (!ctx->rep->flag) {
+                kmm_set_error(ctx, "the step ended without its report");
+                return KMM_ERR_CUDA;
             }
         }
     }
