@@ -252,9 +252,7 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
         auto ld = [&](int z) { return ok ? t[tile_idx<C, KX>(y * MZ + z, kl)] : zc; };
         auto before = [&] {
             if (threadIdx.x == 0) tma_store_wait_read();   // the previous field's store has read the stage
-            fence_async_smem();   // orders this field's tile reads before the TMA load that refills the slot
             __syncthreads();
-            if (threadIdx.x == 0) load(o + ZF_SLOTS);   // every warp has read this field's tile
         };
         auto out = [&](int z, C v) {
             if (z < NZH || z >= MZ - NZH) {
@@ -264,9 +262,12 @@ __global__ void __launch_bounds__(KX * YT * 32, MINB)
             }
         };
         z_column<MZ, C, -1>(ld, out, before, a, tw);
-        fence_async_smem();
+        fence_async_smem();   // also orders this field's tile reads before the TMA load that refills the slot
         __syncthreads();
-        if (threadIdx.x == 0) tma_store4(&tout, 2 * y0, 0, kx0, o0 + o, stage);
+        if (threadIdx.x == 0) {
+            tma_store4(&tout, 2 * y0, 0, kx0, o0 + o, stage);
+            load(o + ZF_SLOTS);
+        }
     }
     if (threadIdx.x == 0) {
         tma_store_wait_read();
