@@ -376,8 +376,11 @@ int  kmm_wait_selftest(kmm_ctx *ctx, double limit_ms);
  * allocation from now on among those made on first use by the fused step (tables, buffers) and by
  * kmm_solve / kmm_penta / kmm_phirhs (tables) reports out of memory, as if the device were full
  * (0: none).  Those paths then run their forms that need no such memory: the routine step (until
- * KMM_OPT_FUSED is set again or kmm_initial is called) and the table-free solves.            */
-enum kmm_injection { KMM_INJECT_NOMEM = 1 };
+ * KMM_OPT_FUSED is set again or kmm_initial is called) and the table-free solves.
+ * KMM_INJECT_LATE: the `value`-th time from now that the host looks for a wait that ran out after a
+ * fused step's report (each step's report, and the end of a run), it finds one: the call returns
+ * KMM_ERR_TIMEOUT, the next is not affected (0: none).                                       */
+enum kmm_injection { KMM_INJECT_NOMEM = 1, KMM_INJECT_LATE = 2 };
 int  kmm_inject(kmm_ctx *ctx, int what, int value);
 
 /* ---- transform without device allocation --------------------------------------

@@ -14,7 +14,7 @@ OPT_FUSED, OPT_COLUMN_BLOCKED, OPT_GRAPH, OPT_ZTMA, OPT_WAIT_LIMIT_MS, OPT_XBIG,
     1, 2, 3, 4, 5, 6, 7, 8)
 
 # failures injected on the host (enum kmm_injection)
-INJECT_NOMEM = 1
+INJECT_NOMEM, INJECT_LATE = 1, 2
 
 # status codes (enum kmm_status)
 OK, ERR_ARG, ERR_CUDA, ERR_CFL, ERR_NAN, ERR_INTERP, ERR_TIMEOUT, ERR_NOMEM, ERR_UNSUPPORTED, ERR_PCFL = range(10)

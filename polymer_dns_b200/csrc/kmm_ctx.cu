@@ -65,8 +65,8 @@ int kmm_dalloc(kmm_ctx *ctx, void **p, size_t bytes) {
 }
 
 extern "C" int kmm_inject(kmm_ctx *ctx, int what, int value) {
-    if (!ctx || what != KMM_INJECT_NOMEM || value < 0) return KMM_ERR_ARG;
-    ctx->inject_nomem = value;
+    if (!ctx || value < 0 || (what != KMM_INJECT_NOMEM && what != KMM_INJECT_LATE)) return KMM_ERR_ARG;
+    (what == KMM_INJECT_NOMEM ? ctx->inject_nomem : ctx->inject_late) = value;
     return KMM_OK;
 }
 

@@ -1670,11 +1670,17 @@ static int fused_launch(kmm_ctx *ctx) {
     return KMM_OK;
 }
 
+// a wait of a z forward transform that ran out after its step's report
+static bool late(kmm_ctx *ctx) {
+    if (ctx->inject_late > 0 && --ctx->inject_late == 0) ctx->rep->late = KMM_ERR_TIMEOUT;
+    return ctx->rep->late != 0;
+}
+
 // the status of an enqueued step from its report (solvers.f90:3497-3514)
 static int report_status(kmm_ctx *ctx) {
     const KmmReport *R = ctx->rep;
     int st = KMM_OK;
-    if (R->late || R->status == KMM_ERR_TIMEOUT) {
+    if (late(ctx) || R->status == KMM_ERR_TIMEOUT) {
         ctx->rep->late = 0;
         kmm_set_error(ctx, "a device-side wait ran out");
         st = KMM_ERR_TIMEOUT;
@@ -1748,7 +1754,7 @@ int kmm_fused_report(kmm_ctx *ctx) {
 
 int kmm_fused_drain(kmm_ctx *ctx, int st) {
     CK(cudaStreamSynchronize(ctx->stream));
-    if (ctx->rep->late) {
+    if (late(ctx)) {
         ctx->rep->late = 0;
         kmm_set_error(ctx, "a device-side wait ran out");
         ctx->stats.status = KMM_ERR_TIMEOUT;

@@ -140,6 +140,7 @@ struct kmm_ctx {
     int frate_ready;
     int fused_ran;            // a fused step has run since its kernels were chosen (attributes and fields are set: capturable)
     int fused_nomem;          // the fused step's tables or buffers did not fit: the routine step runs
+    int inject_late;          // KMM_INJECT_LATE: the look at rep->late that is to find a timeout (counted down)
     int inject_nomem;         // KMM_INJECT_NOMEM: the allocation that is to fail (counted down), 0: none
     void *hoststate;  // host arrays bound by kmm_bind_host, their copy streams and events (kmm_hoststate.cu)
 };
