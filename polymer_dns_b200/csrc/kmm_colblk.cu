@@ -281,7 +281,6 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::v) k_bcol_v(ColFw
     char *wreg = reinterpret_cast<char *>(sm) + (size_t)(threadIdx.x >> 5) * CbSmem<K, C>::warp_bytes;
     C *fa = reinterpret_cast<C *>(wreg), *fb = reinterpret_cast<C *>(wreg + CbSmem<K, C>::a_bytes);
     double2 *wsm = reinterpret_cast<double2 *>(wreg);   // bload_s / bstore_s scratch (fa's space)
-    const int lane = threadIdx.x & 31, h = lane >> 4;
     BPair P;
     if (!bpair<K>(P, A.nz, A.nzh, A.nxh, A.wavx, A.wavz)) return;
     const size_t fstride = (size_t)A.nz * A.nxh * col_ld<C>(NYP), yoff = (size_t)P.col * col_ld<C>(NYP);
@@ -556,7 +555,6 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::bwd) k_bcol_bwd(C
         for (int m = 0; m <= K; ++m) h2.v[m] = make_double2(w2 * h2.v[m].x - d.v[m].x, w2 * h2.v[m].y - d.v[m].y);
         bstore_s<K>(A.fn + off, h2, wsm);
     }
-    (void)h;
 }
 
 // K = ny / 16 where blocked kernels are compiled: the fused column kernels for ny = 32 .. 128 (K <=

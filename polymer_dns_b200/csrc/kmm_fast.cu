@@ -339,9 +339,9 @@ __global__ void __launch_bounds__(FX_WARPS * 32, Fx2MinB<C>::v) k_fx2(const C *_
 // in a shared buffer of MX complex values, transforms it in place (the last stage through registers) and
 // leaves the two physical rows there; the block forms the pointwise terms of k_fx2, holding its points'
 // results in registers, and puts (h1, h2) and (h3, scalar term) into the first two buffers, which two warps
-// transform back.  The buffers are the only copy of a row: 46 KB a block, so three blocks of five warps share an SM.
+// transform back.  The buffers are the only copy of a row: 52 KB a block, so three blocks of five warps share an SM.
 // It reads q and writes r once; the passes through HBM buffers of the physical inputs and outputs that it
-// replaces (k_xinv_big2, k_xpoint, k_xfwd2) took 8.1 ms at 384 x 257 x 384 with a scalar, this takes 4.8.
+// replaces (k_xinv_big2, k_xpoint, k_xfwd2) took 8.1 ms at 384 x 257 x 384 with a scalar, this takes 4.1.
 template <int MX, int NP>
 __global__ void __launch_bounds__(NP * 32, NP == 5 ? 3 : 5)
     k_fx_row(const double2 *__restrict__ q, double2 *__restrict__ r, double *__restrict__ up3, double *__restrict__ vp3,

@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         }
         // ---- influence matrix (main_dns.f90:426-466)
         {
-            double2 wb, wt, tmp;
+            double2 wb, wt;
             if (A.nb == 1 && A.nt == 1) {
                 col_wall1<E>(v, nyp, A.dyde, wb, wt);
             } else {
@@ -810,7 +810,6 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
                 col_wall1<E>(v, nyp, A.dyde, wb, wt);
                 if (A.nb == 2) wb = b2;
                 if (A.nt == 2) wt = t2;
-                (void)tmp;
             }
             const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[col]), cmul(wt, A.dnv2b[col])), A.denom[col]);
             const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[col]), cmul(wb, A.dnv1t[col])), A.denom[col]);
@@ -913,12 +912,10 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
 #define ZT_WARPS (ZT_KX * ZT_Y)
 
 // Q[g][y][z][kx], g = u v w wx wy wz [cx cy cz], from the y-physical base fields
-// MZ > 0: compile-time z length (specialised FFT); MZ = 0: runtime plan
-template <int MZ>
+// (run-time z length; the compiled ones are k_zb_tma's and k_zb2's)
 __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb(const double2 *__restrict__ yp, double2 *__restrict__ q,
                                                       const double *__restrict__ wavx, const double *__restrict__ wavz,
-                                                      const __grid_constant__ DevPlan P, int nout, int nyp, int nz, int nxh, int mz_rt) {
-    const int mz = MZ > 0 ? MZ : mz_rt;
+                                                      const __grid_constant__ DevPlan P, int nout, int nyp, int nz, int nxh, int mz) {
     extern __shared__ double2 sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kl = warp % ZT_KX, yl = warp / ZT_KX;
@@ -929,10 +926,9 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb(const double2 *__restrict_
     double2 *a = sm + (size_t)warp * 2 * mz, *b = a + mz;
     double2 *stage = sm + (size_t)ZT_WARPS * 2 * mz;   // [y][z][kx] tile for the store
     const double kxv = act ? wavx[kx] : 0.0;
-    auto SW = [](int x) { return MZ > 0 ? swz<double2>(x) : x; };
     for (int g = blockIdx.z; g < nout; g += gridDim.z) {
         if (act) {
-            for (int z = lane; z < mz; z += 32) a[SW(z)] = make_double2(0.0, 0.0);
+            for (int z = lane; z < mz; z += 32) a[z] = make_double2(0.0, 0.0);
             __syncwarp();
             for (int kz = lane; kz < nz; kz += 32) {
                 const size_t o = ((size_t)kx * nz + kz) * nyp + y;
@@ -955,13 +951,12 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb(const double2 *__restrict_
                 default: val = __ldg(yp + (size_t)g * ncols * nyp + o); break;   // u v w
                 }
                 const int jj = kz < nzh ? kz : (mz - nz) + kz;
-                a[SW(jj)] = val;
+                a[jj] = val;
             }
             __syncwarp();
             const double2 *r;
-            if constexpr (MZ > 0) r = fft_warp_ct<double2, MZ, +1, 1, true>(a, b, P.tw);
-            else r = fft_warp(P, a, b, +1);
-            for (int z = lane; z < mz; z += 32) stage[((size_t)yl * mz + z) * ZT_KX + kl] = r[SW(z)];
+            r = fft_warp(P, a, b, +1);
+            for (int z = lane; z < mz; z += 32) stage[((size_t)yl * mz + z) * ZT_KX + kl] = r[z];
         }
         __syncthreads();
         // store rows of ZT_KX consecutive kx
@@ -977,10 +972,8 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zb(const double2 *__restrict_
 }
 
 // y-physical outputs [o][ncols][nyp] from R[o][y][z][kx]
-template <int MZ>
 __global__ void __launch_bounds__(ZT_WARPS * 32) k_zf(const double2 *__restrict__ r, double2 *__restrict__ yo, const __grid_constant__ DevPlan P,
-                                                      int nout, int nyp, int nz, int nxh, int mz_rt, double scale) {
-    const int mz = MZ > 0 ? MZ : mz_rt;
+                                                      int nout, int nyp, int nz, int nxh, int mz, double scale) {
     extern __shared__ double2 sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kl = warp % ZT_KX, yl = warp / ZT_KX;
@@ -990,17 +983,15 @@ __global__ void __launch_bounds__(ZT_WARPS * 32) k_zf(const double2 *__restrict_
     const int nzh = nz / 2;
     double2 *a = sm + (size_t)warp * 2 * mz, *b = a + mz;
     double2 *stage = sm + (size_t)ZT_WARPS * 2 * mz;   // [kx][kz][y] tile for the store
-    auto SW = [](int x) { return MZ > 0 ? swz<double2>(x) : x; };
     for (int o = blockIdx.z; o < nout; o += gridDim.z) {
         if (act) {
-            for (int z = lane; z < mz; z += 32) a[SW(z)] = __ldg(r + (((size_t)o * nyp + y) * mz + z) * nxh + kx);
+            for (int z = lane; z < mz; z += 32) a[z] = __ldg(r + (((size_t)o * nyp + y) * mz + z) * nxh + kx);
             __syncwarp();
             const double2 *res;
-            if constexpr (MZ > 0) res = fft_warp_ct<double2, MZ, -1, 1, true>(a, b, P.tw);
-            else res = fft_warp(P, a, b, -1);
+            res = fft_warp(P, a, b, -1);
             for (int kz = lane; kz < nz; kz += 32) {
                 const int jj = kz < nzh ? kz : (mz - nz) + kz;
-                const double2 v = res[SW(jj)];
+                const double2 v = res[jj];
                 stage[((size_t)kl * nz + kz) * ZT_Y + yl] = make_double2(v.x / scale, v.y / scale);
             }
         }
@@ -1245,11 +1236,12 @@ int kmm_fast_x2(kmm_ctx *ctx, const void *q, void *r, const void *tw, bool fp32,
 int kmm_tracers(kmm_ctx *ctx);
 
 // the fused path applies when: no polymer, no immersed boundary, Dirichlet-type velocity walls
-// (nb = nt = 1 or 2), nyp in the compiled register layouts, and the x transform instance exists
+// (nb = nt = 1 or 2), nyp up to 192 or 257 .. 288 and mx up to 288 or 353 .. 384 (the kernels' registers), mz up to 300 (their
+// shared memory), and the tables and buffers fitted in memory (kmm_fused_select)
 bool kmm_fused_applicable(const kmm_ctx *ctx) {
     if (ctx->p.polymer_on || ctx->f[KMM_IMATRIX] != NULL || ctx->fused_nomem) return false;
-    // the flow-rate correction sits between the v and the u, w column kernels, which only the
-    // blocked kernels (ny = 32, 64, 96, 128) launch separately
+    // the flow-rate correction of u0 follows the mean modes on their stream, ahead of the u, w kernel: only the blocked
+    // kernels (ny = 32, 64, 96, 128) have the mean modes in a launch of their own before it
     const bool blocked = ctx->use_colblk && (ctx->ny == 32 || ctx->ny == 64 || ctx->ny == 96 || ctx->ny == 128);
     if (ctx->p.flow_rate > 0.0 && !blocked) return false;
     if (ctx->p.scalar_on && ctx->p.scl_flag >= 2) return false;
@@ -1442,10 +1434,9 @@ static int fused_launch(kmm_ctx *ctx) {
     const int nyp = ctx->nyp, nz = ctx->nz, nxh = ctx->nxh, mz = ctx->mz;
     const size_t ncols = (size_t)nz * nxh;
     const int scalar = ctx->p.scalar_on ? 1 : 0;
-    const int nbase = scalar ? 8 : 6, nq = scalar ? 9 : 6, nout = scalar ? 4 : 3;
+    const int nq = scalar ? 9 : 6, nout = scalar ? 4 : 3;
     KmmFused *FU = ctx->fused;
     double2 *g_yp = FU->yp, *g_q = FU->q, *g_r = FU->r, *g_yo = FU->yo;
-    (void)nbase;
     // the mixed-precision form (FP32 transforms and products, FP64 solves) has compiled kernels
     // for ny, nx, nz in {32, 64, 96, 128} (nx, nz: the 3/2 lengths 48 .. 192)
     const bool f32 = ctx->p.precision == 1;
@@ -1554,8 +1545,8 @@ static int fused_launch(kmm_ctx *ctx) {
         case 144: ZB2(144, double2); break;
         case 192: ZB2(192, double2); break;
         default:
-            RET(kmm_smem_attr(ctx, (const void *)k_zb<0>, smz));
-            k_zb<0><<<dim3(gz.x, gz.y, nq), ZT_WARPS * 32, smz, ctx->stream>>>(g_yp, g_q, ctx->d_wavx, ctx->d_wavz, ctx->wmz, nq, nyp, nz,
+            RET(kmm_smem_attr(ctx, (const void *)k_zb, smz));
+            k_zb<<<dim3(gz.x, gz.y, nq), ZT_WARPS * 32, smz, ctx->stream>>>(g_yp, g_q, ctx->d_wavx, ctx->d_wavz, ctx->wmz, nq, nyp, nz,
                                                            nxh, mz);
             break;
         }
@@ -1613,8 +1604,8 @@ static int fused_launch(kmm_ctx *ctx) {
         case 144: ZF2(144, double2); break;
         case 192: ZF2(192, double2); break;
         default:
-            RET(kmm_smem_attr(ctx, (const void *)k_zf<0>, smzf));
-            k_zf<0><<<dim3(gz.x, gz.y, nout), ZT_WARPS * 32, smzf, ctx->stream>>>(g_r, g_yo, ctx->wmz, nout, nyp, nz, nxh, mz,
+            RET(kmm_smem_attr(ctx, (const void *)k_zf, smzf));
+            k_zf<<<dim3(gz.x, gz.y, nout), ZT_WARPS * 32, smzf, ctx->stream>>>(g_r, g_yo, ctx->wmz, nout, nyp, nz, nxh, mz,
                                                             (double)ctx->mx * (double)mz);
             break;
         }

@@ -88,7 +88,7 @@ struct kmm_ctx {
     double *d_umax;              // scratch for |u| max (per plane)
     double *d_scratch;           // 9*KMM_MAX_NYP doubles for the (0,0)-mode solver
     KmmReport *rep;              // the fused step's report (pinned host)
-    double *h_pin;               // pinned host: cfl[KMM_MAX_NYP], umax[KMM_MAX_NYP], status (step read-backs)
+    double *h_pin;               // pinned host words: status, flow-rate correction, tensor-core status
     double *scsource;            // the KMM_SCSOURCE field's storage (scl_flag = 2, 4, 5)
     // targeted sources (scl_flag = 4, 5): -Q on the 3/2 grid, the candidate list and its count,
     // the placed targets' centres, reduction scratch; the host copy of the last targets
@@ -203,11 +203,11 @@ int kmm_field_info(const kmm_ctx *ctx, int field, size_t *nelem, int *eb);
 void *kmm_field_ptr(kmm_ctx *ctx, int field);   // allocates (zeroed) on first use, NULL on failure
 static inline double2 *SPEC(kmm_ctx *ctx, int f) { return (double2 *)kmm_field_ptr(ctx, f); }
 static inline double *REAL(kmm_ctx *ctx, int f) { return (double *)kmm_field_ptr(ctx, f); }
-// the pinned status word after the cfl and umax rows of h_pin, and the flow-rate correction after it
-static inline int *kmm_h_pin_status(kmm_ctx *ctx) { return (int *)(ctx->h_pin + 2 * KMM_MAX_NYP); }
-static inline double *kmm_h_pin_delta(kmm_ctx *ctx) { return ctx->h_pin + 2 * KMM_MAX_NYP + 1; }
-static inline int *kmm_h_pin_tcstat(kmm_ctx *ctx) { return (int *)(ctx->h_pin + 2 * KMM_MAX_NYP + 2); }
-#define KMM_H_PIN_DOUBLES (2 * KMM_MAX_NYP + 3)
+// the pinned words of h_pin
+static inline int *kmm_h_pin_status(kmm_ctx *ctx) { return (int *)ctx->h_pin; }
+static inline double *kmm_h_pin_delta(kmm_ctx *ctx) { return ctx->h_pin + 1; }
+static inline int *kmm_h_pin_tcstat(kmm_ctx *ctx) { return (int *)(ctx->h_pin + 2); }
+#define KMM_H_PIN_DOUBLES 3
 
 // internal entry points shared between translation units
 int kmm_internal_cderiv(kmm_ctx *ctx, const double2 *f, double2 *df);

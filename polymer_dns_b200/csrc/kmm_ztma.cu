@@ -12,8 +12,8 @@
 // own mbarrier.  Each warp's FFT (the warp-private compile-time FFT of kmm_fft.cuh) forms the field's
 // z-spectral values from the tiles in its first stage, runs in place in one buffer, and leaves its
 // result in a [y][z][kx] staging tile, which a tiled TMA store (box: KX kx x mz z x YT y) writes out
-// while the next field is transformed.  49 KB of shared memory per CTA at mz = 192 in FP64.  Both
-// kinds of tile are swizzled by the length of their rows.
+// while the next field is transformed.  52 KB of shared memory per CTA for the inverse and 48 KB for the
+// forward transform at mz = 192 in FP64.  Both kinds of tile are swizzled by the length of their rows.
 //
 // Every wait on an mbarrier is bounded (KMM_OPT_WAIT_LIMIT_MS, default 2 s of %globaltimer); a wait
 // that runs out records KMM_ERR_TIMEOUT in the step's status word (the forward transform, which runs
