@@ -319,7 +319,11 @@ __global__ void __launch_bounds__(CB_WARPS * 32, CbMinB<K, C>::v) k_bcol_v(ColFw
         }
         const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[P.col]), cmul(wt, A.dnv2b[P.col])), A.denom[P.col]);
         const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[P.col]), cmul(wb, A.dnv1t[P.col])), A.denom[P.col]);
-        if (KEEP && bl_t() == 0) { A.kc1[P.col] = c1; A.kc2[P.col] = c2; }
+        if (KEEP && bl_t() == 0) {
+            A.kc1[P.col] = c1;
+            A.kc2[P.col] = c2;
+            A.kbt[P.col] = A.kbb[P.col] = zero;
+        }
         BCol<K> gfa;
         bload_s<K>(gfa, A.gf1 + P.off, wsm);
 #pragma unroll

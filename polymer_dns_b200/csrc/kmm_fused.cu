@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
         }
 #pragma unroll
         for (int e = 0; e < E; ++e) v.v[e] = om.v[e] = make_double2(0.0, 0.0);
-        if (A.kc1 && lane == 0) A.kc1[col] = A.kc2[col] = make_double2(0.0, 0.0);
+        if (A.kc1 && lane == 0) A.kc1[col] = A.kc2[col] = A.kbt[col] = A.kbb[col] = make_double2(0.0, 0.0);
         __syncthreads();   // warp 0 reads w0 below
     } else {
         // ---- wall-normal velocity: phi, phirhs, Helmholtz + Poisson (main_dns.f90:363-407)
@@ -813,7 +813,11 @@ __global__ void __launch_bounds__(64) k_col_fwd(ColFwdArgs A, FusedTabs T, const
             }
             const double2 c1 = cdiv(csub(cmul(wb, A.dnv2t[col]), cmul(wt, A.dnv2b[col])), A.denom[col]);
             const double2 c2 = cdiv(csub(cmul(wt, A.dnv1b[col]), cmul(wb, A.dnv1t[col])), A.denom[col]);
-            if (A.kc1 && lane == 0) { A.kc1[col] = c1; A.kc2[col] = c2; }
+            if (A.kc1 && lane == 0) {
+                A.kc1[col] = c1;
+                A.kc2[col] = c2;
+                A.kbt[col] = A.kbb[col] = make_double2(0.0, 0.0);
+            }
             Col<E> gfa;
             col_load<E>(gfa, A.gf1 + off, nyp);
 #pragma unroll
@@ -1465,9 +1469,9 @@ static int fused_launch(kmm_ctx *ctx) {
     F.h3n = REAL(ctx, KMM_H3N); F.h3nm1 = REAL(ctx, KMM_H3NM1);
     if (kmm_keeps_mirrors(ctx)) {
         F.ku = SPEC(ctx, KMM_U); F.kw = SPEC(ctx, KMM_W); F.komx = SPEC(ctx, KMM_OMX);
-        F.kc1 = SPEC(ctx, KMM_C1); F.kc2 = SPEC(ctx, KMM_C2);
+        F.kc1 = SPEC(ctx, KMM_C1); F.kc2 = SPEC(ctx, KMM_C2); F.kbt = SPEC(ctx, KMM_BCTOP); F.kbb = SPEC(ctx, KMM_BCBOT);
         F.kscly = scalar ? SPEC(ctx, KMM_SCLY) : NULL;
-        if (!F.ku || !F.kw || !F.komx || !F.kc1 || !F.kc2 || (scalar && !F.kscly)) return KMM_ERR_NOMEM;
+        if (!F.ku || !F.kw || !F.komx || !F.kc1 || !F.kc2 || !F.kbt || !F.kbb || (scalar && !F.kscly)) return KMM_ERR_NOMEM;
     }
     F.yp = g_yp; F.wavx = ctx->d_wavx; F.wavz = ctx->d_wavz;
     F.nz = nz; F.nxh = nxh; F.nyp = nyp; F.nzh = ctx->nzh; F.scalar = scalar; F.nb = ctx->nb; F.nt = ctx->nt;

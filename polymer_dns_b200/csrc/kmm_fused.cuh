@@ -48,8 +48,9 @@ struct ColFwdArgs {
     const double2 *gf1, *gf2, *dnv1b, *dnv1t, *dnv2b, *dnv2t, *denom;
     double *u0, *w0, *h1n, *h1nm1, *h3n, *h3nm1;
     double2 *yp;      // y-physical outputs [8][ncols][nyp]
-    // mirrors the step also leaves current (kmm_keeps_mirrors; all NULL elsewhere): u, w, omega_x, dc/dy, c1, c2
-    double2 *ku, *kw, *komx, *kscly, *kc1, *kc2;
+    // mirrors the step also leaves current (kmm_keeps_mirrors; all NULL elsewhere): u, w, omega_x, dc/dy, c1, c2 and
+    // the wall rows, zero as phirhs leaves them
+    double2 *ku, *kw, *komx, *kscly, *kc1, *kc2, *kbt, *kbb;
     const double *wavx, *wavz;
     int nz, nxh, nyp, nzh, scalar, nb, nt;
     double re, dt, th, dyde, diff, c0;

@@ -32,3 +32,16 @@ def test_mirrors_after_a_run(grid, scalar):
         assert np.abs(got[1][k]).max() > 0.0, k
         # two steps of FP64 rounding; c1 and c2 divide by the wall derivatives' determinant
         assert rel_err(got[0][k], got[1][k]) < 1e-9, k
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+def test_wall_rows_are_zero_after_a_step(grid):
+    p = cfg_small(*grid, dt=0.002)
+    with runtime.KmmContext(p) as c:
+        load_initial(c, p, initial_fields(p, kmax=3))
+        c.initial()
+        for k in ("BCTOP", "BCBOT"):
+            c.upload(k, np.ones_like(c.download(k)))
+        c.run(1)
+        for k in ("BCTOP", "BCBOT"):
+            assert not c.download(k).any(), k
