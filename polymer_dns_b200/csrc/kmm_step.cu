@@ -335,6 +335,28 @@ static int swap_fields(kmm_ctx *ctx, int nm1, int n) {
     return KMM_OK;
 }
 
+// work on the two side streams that the context's stream has to wait for, also when the step returns early: what the
+// caller does next (a download of u0, another step) is ordered on the context's stream alone
+namespace {
+struct SideJoin {
+    kmm_ctx *ctx;
+    bool open = true;
+    explicit SideJoin(kmm_ctx *c) : ctx(c) {}
+    int join() {
+        open = false;
+        const cudaStream_t s[2] = {ctx->side, ctx->side2};
+        for (int e = 0; e < 2; ++e) {
+            CK(cudaEventRecord(ctx->cjoin_ev[e], s[e]));
+            CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[e], 0));
+        }
+        return KMM_OK;
+    }
+    ~SideJoin() {
+        if (open) join();
+    }
+};
+}  // namespace
+
 // ---------------------------------------------------------------------------
 // one iteration of the time loop, main_dns.f90:198-811
 // ---------------------------------------------------------------------------
@@ -411,10 +433,9 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
     CK(cudaStreamWaitEvent(ctx->side, ctx->fork_ev, 0));
     CK(cudaStreamWaitEvent(ctx->side2, ctx->fork_ev, 0));
+    SideJoin side_solves(ctx);
     RET(kmm_internal_uzero(ctx, 3, ctx->side));
     RET(kmm_internal_uzero(ctx, 1, ctx->side2));
-    CK(cudaEventRecord(ctx->cjoin_ev[0], ctx->side));
-    CK(cudaEventRecord(ctx->cjoin_ev[1], ctx->side2));
     // phirhs and its solves in one blocked kernel per field where compiled (every boundary value
     // is zero: phirhs zeroes bctop / bcbot, main_dns.f90:39, solvers.f90:670-671), else routine by
     // routine
@@ -465,7 +486,7 @@ extern "C" int kmm_step(kmm_ctx *ctx) {
     }
     RET(kmm_zero(ctx, KMM_BCTOP));   // as phirhs leaves them
     RET(kmm_zero(ctx, KMM_BCBOT));
-    for (int e = 0; e < 2; ++e) CK(cudaStreamWaitEvent(ctx->stream, ctx->cjoin_ev[e], 0));   // u0, w0
+    RET(side_solves.join());   // u0, w0
     RET(kmm_flowrate_apply(ctx, ctx->stream));
     k_zero_mean<<<1, 256, 0, ctx->stream>>>(SPEC(ctx, KMM_OMY), ctx->nyp);
     CKL();
