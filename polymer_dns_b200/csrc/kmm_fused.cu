@@ -1428,6 +1428,8 @@ int kmm_fused_launch(kmm_ctx *ctx) {
     ctx->d_umax = ctx->d_cfl + ctx->nyp;
     ctx->d_status = (int *)(ctx->d_umax + ctx->nyp);
     const int st = fused_launch(ctx);
+    if (st != KMM_OK)   // a step cut short has no report to leave the words zero
+        cudaMemsetAsync(ctx->fused->acc, 0, sizeof(double) * (2 * (size_t)ctx->nyp + 1), ctx->stream);
     ctx->d_cfl = cfl;
     ctx->d_umax = um;
     ctx->d_status = status;
