@@ -258,7 +258,9 @@ int  kmm_filter(kmm_ctx *ctx);
 int  kmm_initial(kmm_ctx *ctx);
 /* one iteration of the time loop body, main_dns.f90:198-811, fused */
 int  kmm_step(kmm_ctx *ctx);
-/* `n` iterations (stops early with the status of a failing step) */
+/* `n` iterations (stops early with the status of a failing step).  While it waits for a step the
+ * calling thread polls for 20 us, then yields, or sleeps where the device was set to
+ * cudaDeviceScheduleBlockingSync. */
 int  kmm_run(kmm_ctx *ctx, int n);
 
 /* ---- state held in host arrays ---------------------------------------------
@@ -326,7 +328,12 @@ int  kmm_ensemble_run(kmm_ctx **ctxs, int n, int nsteps, int *status);
 /* ---- options --------------------------------------------------------------- */
 enum kmm_option {
     KMM_OPT_FUSED = 1,  /* 1 (default): kmm_step runs the fused kernels when the run has no polymer and no
-                           immersed boundary; 0: kmm_step runs the routine-by-routine kernels   */
+                           immersed boundary, the grid fits them and so do their tables and buffers in
+                           device memory; 0: kmm_step runs the routine-by-routine kernels.  After a
+                           fused step with nx, ny in {32, 64, 96, 128} the mirrors of u, w, omega_x, dc/dy,
+                           c1, c2, the wall rows and (npart = 0) UP3D .. WP3D are not current
+                           (kmm_veloc, kmm_vort, kmm_gradscl form them); on every other grid they are,
+                           as after a routine step                                              */
     KMM_OPT_COLUMN_BLOCKED = 2, /* 1 (default): the fused step's column kernels hold a column on 16
                            lanes in blocks of ny/16 coefficients (ny = 32, 64, 96, 128);
                            0: one warp per column, coefficient i on lane i mod 32           */
