@@ -16,7 +16,9 @@
 // at ny = 128 (two 628 us, three 617, four 629, where they spill) and four at the smaller ny (96: 344 us against
 // 363 with two); the back kernel two, at ny = 96 four (post stage 43 us against 48).  FP32: four (v at
 // three made a 128 x 129 x 128 mixed step 498 us, four 487; at ny = 96 it stays at three, where the budget of four
-// is compiled to another last bit of v and mixed runs would not repeat earlier ones), the back kernel three.
+// is compiled to another last bit of v than the FP64 form's, and mixed runs would not repeat earlier ones), the back
+// kernel three.  The compiler chooses which product of a two-product FP64 expression stays unrounded; the instances of
+// both precisions agree at these budgets (compared bit for bit in tests/test_gpu_mixed_bits.py).
 template <int K, typename C> struct CbMinB {
     static constexpr bool f64 = sizeof(C) == 16;
     static constexpr int fwd = f64 && K == 8 ? 3 : 4;   // k_bcol_scl, k_bcol_uw

@@ -69,3 +69,23 @@ def test_routines_are_the_general_sequences(grid):
         w2 = kx * kx + kz * kz
         phi = (d2.real - w2 * f["V"].real) + 1j * (d2.imag - w2 * f["V"].imag)
         assert np.array_equal(c.download("V"), phi)
+
+
+@pytest.mark.parametrize("ny", [32, 64, 96, 128])
+def test_column_solves_do_not_depend_on_the_precision(ny):
+    """The fused column kernels solve in FP64 in both precisions: one step from one state leaves the same bits, whatever
+    register budget each instance is compiled for."""
+    out = []
+    for precision in (0, 1):
+        p = kc.cfg_small(32, ny, 32, dt=0.001, precision=precision, scalar_on=1, diff=1.0, scalar_bc=1)
+        rng = np.random.default_rng(5)
+        with runtime.KmmContext(p) as c:
+            fields = kc.initial_fields(p)
+            kc.load_initial(c, p, fields, 0.1 * fields[0])
+            c.initial()
+            for k in ("V", "OMY", "FN", "FNM1", "GN", "GNM1", "SCALAR", "SCN", "SCNM1"):
+                c.upload(k, kc.random_spectral(rng, p))
+            c.call("step", allow=(abi.ERR_CFL,))
+            out.append({k: c.download(k) for k in ("V", "OMY", "SCALAR")})
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
