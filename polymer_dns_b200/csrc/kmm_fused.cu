@@ -233,8 +233,9 @@ static int fill_tables(kmm_ctx *ctx, KmmFused *F) {
     if (blocked)
         for (int a = 0; a < 4; ++a) ob[a] = V.take(sizeof(double) * nall);
     const size_t obrj = blocked ? V.take(sizeof(double) * 3 * nyp) : 0;
-    // the buffers start on 2 MB pages like allocations of their own: packed behind one another they made the FP32 z
-    // inverse 77 us at 128 x 129 x 128 instead of 72
+    // the buffers start on 2 MB pages like allocations of their own.  (The FP32 z inverse, which stores 16-byte pieces of
+    // rows, takes 68 to 90 us at 128 x 129 x 128 by where q lies in memory, in steps of 2 MB as of 32, with one allocation
+    // as with four: no offset is good at every placement.)
     const size_t big = ncp * 8 < 65536 ? 256 : 2u << 20;
     const size_t oyp = V.take(sizeof(double2) * ncp * 8, big), oq = V.take(sizeof(double2) * nq * 10, big);
     const size_t orr = V.take(sizeof(double2) * nq * 4, big), oyo = V.take(sizeof(double2) * ncp * 4, big);
