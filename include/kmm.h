@@ -330,10 +330,10 @@ enum kmm_option {
     KMM_OPT_FUSED = 1,  /* 1 (default): kmm_step runs the fused kernels when the run has no polymer and no
                            immersed boundary, the grid fits them and so do their tables and buffers in
                            device memory; 0: kmm_step runs the routine-by-routine kernels.  After a
-                           fused step with nx, ny in {32, 64, 96, 128} the mirrors of u, w, omega_x, dc/dy,
-                           c1, c2, the wall rows and (npart = 0) UP3D .. WP3D are not current
-                           (kmm_veloc, kmm_vort, kmm_gradscl form them); on every other grid they are,
-                           as after a routine step                                              */
+                           fused step with nx and ny in {32, 64, 96, 128} the mirrors of u, w, omega_x,
+                           dc/dy, c1, c2 and the wall rows are not current (kmm_veloc, kmm_vort,
+                           kmm_gradscl form them); on every other grid they are, as after a routine
+                           step.  UP3D .. WP3D are current with npart > 0 or nx outside that set.   */
     KMM_OPT_COLUMN_BLOCKED = 2, /* 1 (default): the fused step's column kernels hold a column on 16
                            lanes in blocks of ny/16 coefficients (ny = 32, 64, 96, 128);
                            0: one warp per column, coefficient i on lane i mod 32           */

@@ -174,9 +174,10 @@ void kmm_fused_replayed(kmm_ctx *ctx, int parity);
 int kmm_fused_enqueue(kmm_ctx *ctx);
 void kmm_graph_release(kmm_ctx *ctx);
 bool kmm_fused_applicable(const kmm_ctx *ctx);
-// The grids on which the fused step leaves u, w, omega_x, dc/dy, c1, c2 and the 3/2-grid velocities in their
-// mirrors as the routine step does: those with a run-time length in y or x.  At the compiled lengths of both
-// it writes only what the next step reads (the mirrors would be 2 % of a step's traffic there).
+// The grids on which the fused step leaves u, w, omega_x, dc/dy, c1, c2, the wall rows and (a run-time length in x) the
+// 3/2-grid velocities in their mirrors as the routine step does: those with a run-time length in y or x.  At the
+// compiled lengths of both it writes only what the next step reads.  The stores take 3 us of a step of 310 at
+// 80 x 61 x 60.
 static inline bool kmm_compiled_mx(const kmm_ctx *ctx) {
     return ctx->mx == 48 || ctx->mx == 96 || ctx->mx == 144 || ctx->mx == 192;
 }
